@@ -178,7 +178,7 @@ extern "C" int posit_batch_gemm_plan_create(const posit_batch_gemm *probs, int n
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    p->ctas = sms * 2;
+    p->ctas = sms * pg::BATCH_GEMM_CTAS_PER_SM;
     const size_t nt = tiles.size() > 0 ? tiles.size() : 1;
     cudaError_t e = cudaMalloc(&p->d_probs, sizeof(pg::BatchGemmDesc) * desc.size());
     if (e == cudaSuccess)

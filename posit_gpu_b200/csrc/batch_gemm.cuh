@@ -29,6 +29,8 @@ constexpr int BATCH_TILE_CONFIGS = 3;
 __host__ __device__ inline int batch_tile_rows(int cfg) { return cfg == 0 ? 64 : 32; }
 __host__ __device__ inline int batch_tile_cols(int cfg) { return cfg == 2 ? 64 : 32; }
 
+constexpr int BATCH_GEMM_CTAS_PER_SM = 3;
+
 size_t batch_gemm_smem_bytes();
 cudaError_t batch_gemm_launch(const BatchGemmDesc *probs, const BatchTile *tiles, int ntiles, int *next, int ctas,
                               cudaStream_t st);

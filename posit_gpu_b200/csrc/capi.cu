@@ -106,13 +106,15 @@ int rgemm_device(bool nota, bool notb, int m, int n, int k, uint32_t alpha, cons
     }
     size_t need = pg::gemm_workspace_bytes(m, n, k);
     bool own = false;
-    if (ws == nullptr) {
+    if (ws == nullptr && pg::gemm_route(nota, notb, m, n, k, A, lda, B, ldb, C, ldc, false) != pg::GEMM_STAGED) {
+        need = 0; // the fused route uses none
+    } else if (ws == nullptr) {
         PG_TRY(cudaMallocAsync(&ws, need, st));
         own = true;
     } else if (ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15u)) {
         return POSIT_E_WORKSPACE;
     }
-    cudaError_t e = pg::gemm_launch(nota, notb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, ws, st);
+    cudaError_t e = pg::gemm_launch(nota, notb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, ws, st, false);
     if (own)
         cudaFreeAsync(ws, st);
     if (e != cudaSuccess)

@@ -8,23 +8,17 @@
 //            then c <- alpha*t (beta == 0) or alpha*t + beta*c.
 // Both are one chain of "acc <- acc + x_l*y_l" per output; they differ only in the
 // operand prescale (alpha*B for NN/NT), the accumulator's start value and the
-// epilogue.  So one main kernel serves all four transpose cases:
+// epilogue.  Two routes, the same k-step (gemm_tile.cuh) and the same bits:
 //
-//  1. decode pre-pass: op(A) and op(B) (times alpha for NN/NT, rounded exactly as the
-//     reference rounds alpha*b_lj) are converted ONCE per element to FP64 (posit32
-//     values are exact there), stored tile-contiguously in a workspace: A as
-//     [m-tile][k-tile][l][i], B as [n-tile][k-tile][l][j], plus a NaR flag per row and
-//     column.  Transposition is absorbed here, so the main kernel never sees lda/ldb.
-//  2. main kernel: one CTA per 64x32 tile of C, 256 threads, 4x2 outputs per thread held
-//     in FP64 across the whole k loop (two sets taking turns, gemm_tile.cuh), 3 CTAs per
-//     SM.  Each 16-deep k tile of A and B
-//     (8 KB + 4 KB) is brought into shared memory by the bulk-copy (TMA) engine
-//     (cp.async.bulk + mbarrier transaction counts, 3 stages, every wait bounded).  The
-//     inner step is the FP64 form of p32_mul + p32_add (posit32.cuh, f64_posit_mac) with
-//     the rounding constants in a shared-memory table, written into the other accumulator
-//     set without a select; the rare step it flags (an inexact FP64 sum, a result outside
-//     the fast window) is redone exactly from the set it read, in order, right after its
-//     k step.
+//  * staged (large products): a pre-pass converts op(A) and op(B) (times alpha for NN/NT,
+//    rounded exactly as the reference rounds alpha*b_lj) ONCE per element to FP64 (posit32
+//    values are exact there) into a workspace of 32 x 16 blocks, [block][k-tile][l][32],
+//    plus a NaR flag per row and column; transposition is absorbed here.  The main kernel,
+//    one CTA of 256 threads per 64x64 tile of C, 2 CTAs per SM, brings each k tile's four
+//    4 KB blocks into shared memory by the bulk-copy (TMA) engine (cp.async.bulk + mbarrier
+//    transaction counts, 3 stages, every wait bounded);
+//  * fused (small products): one launch, no workspace; a CTA reads the patterns of its own
+//    operand blocks and converts them itself (gemm_tile.cuh, fused_tile).
 #include "gemm.cuh"
 #include "gemm_tile.cuh"
 #include "posit32.cuh"
@@ -96,12 +90,14 @@ GemmPlan gemm_plan(int m, int n, int k)
     p.m = m;
     p.n = n;
     p.k = k;
-    p.mt = (m + BM - 1) / BM;
-    p.nt = (n + BN - 1) / BN;
+    p.mb = (m + BLK - 1) / BLK;
+    p.nb = (n + BLK - 1) / BLK;
     p.kt = (k + BK - 1) / BK;
-    p.a_bytes = (size_t)p.mt * p.kt * BK * BM * sizeof(double);
-    p.b_bytes = (size_t)p.nt * p.kt * BK * BN * sizeof(double);
-    p.flag_bytes = (size_t)(p.mt * BM + p.nt * BN);
+    // op(A)'s blocks are padded to pairs, so that a workspace of the size the callers are
+    // told holds any tile shape's operands
+    p.a_bytes = (size_t)((p.mb + 1) / 2 * 2) * p.kt * BK * BLK * sizeof(double);
+    p.b_bytes = (size_t)p.nb * p.kt * BK * BLK * sizeof(double);
+    p.flag_bytes = (size_t)((p.mb + 1) / 2 * 2 + p.nb) * BLK;
     return p;
 }
 
@@ -112,79 +108,61 @@ size_t gemm_workspace_bytes(int m, int n, int k)
 }
 
 // ---------------------------------------------------------------------------
-// Decode pre-pass
+// Staged route: the conversion pre-pass
 // ---------------------------------------------------------------------------
-// op(A) (m x k) -> Ad[mt][kt][l][i].  Rows/columns beyond the matrix hold 1.0 so that
-// padded lanes stay on the fast path; their results are never stored.
-// A NaR operand makes every output of its row NaR (p32_mul and p32_add propagate NaR,
-// kernel_entry.cl:385-390, 414-417); that is recorded in row_nar[] and the operand is
-// decoded as 1.0 so the row's arithmetic stays on the fast path.
-__global__ void decode_a_kernel(bool nota, int m, int k, const uint32_t *__restrict__ A, size_t lda,
-                                int KT, size_t total, double *__restrict__ Ad, unsigned char *__restrict__ row_nar)
+// op(A) (m x k) -> Ad[block][kt][l][i], op(B) (k x n) -> Td[block][kt][l][j], the latter
+// times alpha when `scale`, in one launch (indexes below `na` are A's).  Rows and columns
+// beyond the matrix hold 1.0 so that padded lanes stay on the fast path (their results are
+// never stored), steps past k hold 0.  A NaR operand makes every output of its row (column) NaR (p32_mul and
+// p32_add propagate NaR, kernel_entry.cl:385-390, 414-417); that is recorded in the flags
+// and the operand is decoded as 1.0 so the row's arithmetic stays on the fast path.
+__global__ void decode_kernel(bool nota, bool notb, int m, int n, int k, const uint32_t *__restrict__ A, size_t lda,
+                              const uint32_t *__restrict__ B, size_t ldb, bool scale, uint32_t alpha, int KT,
+                              size_t na, size_t total, double *__restrict__ Ad, double *__restrict__ Td,
+                              unsigned char *__restrict__ row_nar, unsigned char *__restrict__ col_nar)
 {
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(idx % BM);
-        size_t r = idx / BM;
-        int l = (int)(r % BK);
-        r /= BK;
-        int kt = (int)(r % KT);
-        int mt = (int)(r / KT);
-        int row = mt * BM + i, kk = kt * BK + l;
-        uint32_t u = P32_ONE;
-        if (row < m && kk < k)
-            u = nota ? A[(size_t)row + (size_t)kk * lda] : A[(size_t)kk + (size_t)row * lda];
-        if (u == P32_NAR) {
-            row_nar[row] = 1;
-            u = P32_ONE;
+    for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (size_t)gridDim.x * blockDim.x) {
+        const bool is_a = g < na;
+        const size_t idx = is_a ? g : g - na;
+        const int i = (int)(idx % BLK);
+        size_t q = idx / BLK;
+        const int l = (int)(q % BK);
+        q /= BK;
+        const int kt = (int)(q % KT);
+        const int row = (int)(q / KT) * BLK + i, kk = kt * BK + l;
+        const bool rows_contiguous = is_a ? nota : !notb;
+        const uint32_t *X = is_a ? A : B;
+        const size_t ld = is_a ? lda : ldb;
+        double v = kk < k ? 1.0 : 0.0;
+        if (row < (is_a ? m : n) && kk < k) {
+            v = p32_to_double(rows_contiguous ? X[(size_t)row + (size_t)kk * ld] : X[(size_t)kk + (size_t)row * ld]);
+            if (!is_a && scale)
+                v = scale_operand(v, alpha);
         }
-        Ad[idx] = p32_to_double(u);
-    }
-}
-
-// op(B) (k x n) -> Td[nt][kt][l][j], times alpha (exactly rounded) when `scale`.
-__global__ void decode_b_kernel(bool notb, int k, int n, const uint32_t *__restrict__ B, size_t ldb,
-                                bool scale, uint32_t alpha, int KT, size_t total, double *__restrict__ Td,
-                                unsigned char *__restrict__ col_nar)
-{
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        int j = (int)(idx % BN);
-        size_t r = idx / BN;
-        int l = (int)(r % BK);
-        r /= BK;
-        int kt = (int)(r % KT);
-        int nt = (int)(r / KT);
-        int col = nt * BN + j, kk = kt * BK + l;
-        uint32_t u = P32_ONE;
-        if (col < n && kk < k) {
-            u = notb ? B[(size_t)kk + (size_t)col * ldb] : B[(size_t)col + (size_t)kk * ldb];
-            if (scale)
-                u = pmul(alpha, u); // Rgemm.cpp:180 / 222: temp = alpha*b
+        if (v != v) {
+            (is_a ? row_nar : col_nar)[row] = 1;
+            v = 1.0;
         }
-        if (u == P32_NAR) {
-            col_nar[col] = 1;
-            u = P32_ONE;
-        }
-        Td[idx] = p32_to_double(u);
+        (is_a ? Ad : Td)[idx] = v;
     }
 }
 
 // ---------------------------------------------------------------------------
-// Main kernel
+// Staged route: the main kernel
 // ---------------------------------------------------------------------------
 // TRI selects the entries written: TRI_FULL all of C; TRI_LOWER only row >= column (the
 // symmetric trailing update of a lower Cholesky factorization); TRI_UPPER only row <=
 // column (Rsyrk('U', 'T') of an upper one).  Tiles wholly outside the triangle exit at once.
 // `stop`, if given, is a device flag (a factorization's info) that turns the call into a
 // no-op when it is nonzero.
-template <bool DOT, int TRI>
-__global__ void __launch_bounds__(NTHREADS, MIN_CTAS_PER_SM)
-    gemm_main_kernel(int m, int n, int k, int KT, uint32_t alpha, uint32_t beta,
+template <int TRI>
+__global__ void __launch_bounds__(TILE_THREADS, MIN_CTAS_PER_SM)
+    gemm_main_kernel(bool dot, int m, int n, int k, int KT, int mb, int nb, uint32_t alpha, uint32_t beta,
                      const double *__restrict__ Ad, const double *__restrict__ Td, uint32_t *__restrict__ C,
                      size_t ldc, const unsigned char *__restrict__ row_nar,
                      const unsigned char *__restrict__ col_nar, const int *__restrict__ stop)
 {
+    constexpr int BM = 16 * TM, BN = 16 * TN;
     if (stop && *stop != 0)
         return;
     if (TRI == TRI_LOWER && (int)(blockIdx.x * BM + BM - 1) < (int)(blockIdx.y * BN))
@@ -192,83 +170,68 @@ __global__ void __launch_bounds__(NTHREADS, MIN_CTAS_PER_SM)
     if (TRI == TRI_UPPER && (int)(blockIdx.x * BM) > (int)(blockIdx.y * BN + BN - 1))
         return; // every row of the tile is below its last column
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    double *As = reinterpret_cast<double *>(smem_raw);
-    double *Ts = As + STAGES * BK * BM;
-    double *ctab = Ts + STAGES * BK * BN; // rounding constants (F64ConstTable8)
+    unsigned char *tab = smem_raw;
+    constexpr int NBLK = TM / 2 + TN / 2;   // operand blocks of a stage
+    constexpr int BLK_DBL = BK * BLK;       // doubles of a block
+    double *stages = reinterpret_cast<double *>(smem_raw + STEP_TAB_BYTES);
     __shared__ __align__(8) uint64_t full[STAGES];
 
     const int tid = threadIdx.x;
     const int tx = tid % 16, ty = tid / 16;
     const int mt = blockIdx.x, nt = blockIdx.y;
-    const double *Ablk = Ad + (size_t)mt * KT * BK * BM;
-    const double *Tblk = Td + (size_t)nt * KT * BK * BN;
-    constexpr uint32_t kATileBytes = BK * BM * sizeof(double);
-    constexpr uint32_t kBTileBytes = BK * BN * sizeof(double);
+    constexpr uint32_t kBlkBytes = BLK_DBL * sizeof(double);
+    // the tile's blocks that exist (the last tile of an odd count has one block less)
+    const int na = min(TM / 2, mb - mt * (TM / 2)), nbk = min(TN / 2, nb - nt * (TN / 2));
+    auto fetch = [&](int kt, int s) {
+        mbar_arrive_expect_tx(&full[s], (uint32_t)(na + nbk) * kBlkBytes);
+        double *dst = stages + (size_t)s * NBLK * BLK_DBL;
+        for (int q = 0; q < na; ++q)
+            bulk_g2s(dst + q * BLK_DBL, Ad + ((size_t)(mt * (TM / 2) + q) * KT + kt) * BLK_DBL, kBlkBytes, &full[s]);
+        for (int q = 0; q < nbk; ++q)
+            bulk_g2s(dst + (TM / 2 + q) * BLK_DBL, Td + ((size_t)(nt * (TN / 2) + q) * KT + kt) * BLK_DBL, kBlkBytes,
+                     &full[s]);
+    };
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s)
             mbar_init(&full[s], 1);
         mbar_fence_init();
     }
-    for (int i = tid; i < F64_CONST_ENTRIES; i += NTHREADS)
-        ctab[i] = f64_from_hi(f64_round_const_top(i));
+    step_tables_fill(tab, tid, TILE_THREADS);
+    // blocks that do not exist hold 1.0 throughout: their lanes stay on the fast path
+    if (na < TM / 2 || nbk < TN / 2)
+        for (int e = tid; e < STAGES * NBLK * BLK_DBL; e += TILE_THREADS) {
+            const int q = e / BLK_DBL % NBLK;
+            if (q < TM / 2 ? q >= na : q - TM / 2 >= nbk)
+                stages[e] = 1.0;
+        }
     __syncthreads();
-    if (tid == 0) {
-        for (int s = 0; s < STAGES && s < KT; ++s) {
-            mbar_arrive_expect_tx(&full[s], kATileBytes + kBTileBytes);
-            bulk_g2s(As + s * BK * BM, Ablk + (size_t)s * BK * BM, kATileBytes, &full[s]);
-            bulk_g2s(Ts + s * BK * BN, Tblk + (size_t)s * BK * BN, kBTileBytes, &full[s]);
-        }
-    }
+    if (tid == 0)
+        for (int s = 0; s < STAGES && s < KT; ++s)
+            fetch(s, s);
 
-    // Accumulators: NN/NT start from beta*C, TN/TT from zero.  A NaR start value is
-    // remembered in nar_bits (the output stays NaR whatever follows) and replaced by 1.0.
     double acc[TM][TN];
-    uint32_t nar_bits = 0;
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int row = mt * BM + own_off(tx, i), col = nt * BN + own_off(ty, j);
-            uint32_t u = 0;
-            if (!DOT) {
-                u = P32_ONE;
-                if (row < m && col < n) {
-                    u = C[(size_t)row + (size_t)col * ldc];
-                    if (beta == 0)
-                        u = 0; // Rgemm.cpp:170-173: C is not read
-                    else if (beta != P32_ONE)
-                        u = pmul(beta, u);
-                }
-                if (u == P32_NAR) {
-                    nar_bits |= 1u << (i * TN + j);
-                    u = P32_ONE;
-                }
-            }
-            acc[i][j] = p32_to_double(u);
-        }
-    }
+    uint32_t nar_bits;
+    tile_start<TM, TN>(dot, acc, nar_bits, mt * BM, nt * BN, m, n, beta, C, ldc, tx, ty);
 
-    bool bad = false;
-    int kt_stop = 0;
+    bool bad = false, slow = false;
+    int kt_stop = 0, s = 0;
+    uint32_t parity = 0;
+#pragma unroll 1
     for (int kt = 0; kt < KT; ++kt) {
         kt_stop = kt;
-        const int s = kt % STAGES;
-        const uint32_t parity = (uint32_t)(kt / STAGES) & 1u;
         const bool arrived = mbar_wait_bounded(&full[s], parity);
-        const double *as = As + s * BK * BM;
-        const double *ts = Ts + s * BK * BN;
-        const int lmax = min(BK, k - kt * BK);
-        tile_steps_f64<TM, TN>(acc, as, ts, lmax, ctab, tx, ty);
+        const double *as = stages + (size_t)s * NBLK * BLK_DBL;
+        tile_steps<TM, TN, BLK, 8>(acc, as, as + (TM / 2) * BLK_DBL, tile_step_count<8>(k - kt * BK), tab, tx, ty, slow);
         // every thread is done with stage s before it is refilled
         bad = __syncthreads_or(!arrived) != 0;
         if (bad)
             break;
-        if (tid == 0 && kt + STAGES < KT) {
-            const int nk = kt + STAGES;
-            mbar_arrive_expect_tx(&full[s], kATileBytes + kBTileBytes);
-            bulk_g2s(As + s * BK * BM, Ablk + (size_t)nk * BK * BM, kATileBytes, &full[s]);
-            bulk_g2s(Ts + s * BK * BN, Tblk + (size_t)nk * BK * BN, kBTileBytes, &full[s]);
+        if (tid == 0 && kt + STAGES < KT)
+            fetch(kt + STAGES, s);
+        if (++s == STAGES) {
+            s = 0;
+            parity ^= 1u;
         }
     }
 
@@ -281,24 +244,27 @@ __global__ void __launch_bounds__(NTHREADS, MIN_CTAS_PER_SM)
         }
         return;
     }
+    tile_finish<TRI, TM, TN>(dot, acc, nar_bits, mt * BM, nt * BN, m, n, alpha, beta, C, ldc, tx, ty,
+                             [&](int i, int j) { return (row_nar[mt * BM + i] | col_nar[nt * BN + j]) != 0; });
+}
 
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int row = mt * BM + own_off(tx, i), col = nt * BN + own_off(ty, j);
-            if (row < m && col < n && (TRI != TRI_LOWER || row >= col) && (TRI != TRI_UPPER || row <= col)) {
-                uint32_t *cp = C + (size_t)row + (size_t)col * ldc;
-                const bool nar = ((nar_bits >> (i * TN + j)) & 1u) || row_nar[row] || col_nar[col];
-                uint32_t v = nar ? P32_NAR : p32_from_double(acc[i][j]);
-                if (DOT) { // Rgemm.cpp:197-201
-                    uint32_t at = pmul(alpha, v);
-                    v = (beta == 0) ? at : padd(at, pmul(beta, *cp));
-                }
-                *cp = v;
-            }
-        }
-    }
+// ---------------------------------------------------------------------------
+// Fused route
+// ---------------------------------------------------------------------------
+template <int TRI, int TM_, int TN_>
+__global__ void __launch_bounds__(TILE_THREADS, TM_ * TN_ >= 16 ? 2 : (TM_ * TN_ >= 8 ? 3 : 4))
+    gemm_fused_kernel(const __grid_constant__ TileArgs P, const int *__restrict__ stop)
+{
+    constexpr int BM = 16 * TM_, BN = 16 * TN_;
+    if (stop && *stop != 0)
+        return;
+    if (TRI == TRI_LOWER && (int)(blockIdx.x * BM + BM - 1) < (int)(blockIdx.y * BN))
+        return;
+    if (TRI == TRI_UPPER && (int)(blockIdx.x * BM) > (int)(blockIdx.y * BN + BN - 1))
+        return;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    step_tables_fill(smem_raw, threadIdx.x, TILE_THREADS);
+    fused_tile<TRI, TM_, TN_>(P, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 // C <- 0 or beta*C (alpha == 0, Rgemm.cpp:142-156; NN/NT with k == 0, Rgemm.cpp:169-177), or,
@@ -403,55 +369,112 @@ static int grid_for(size_t total, int threads)
     return (int)(b < cap ? (b ? b : 1) : cap);
 }
 
-template <int TRI>
-static cudaError_t gemm_launch_impl(bool nota, bool notb, int m, int n, int k, uint32_t alpha, const uint32_t *A,
-                                    int lda, const uint32_t *B, int ldb, uint32_t beta, uint32_t *C, int ldc,
-                                    void *workspace, cudaStream_t stream, const int *stop)
+static bool spans_overlap(const void *x, size_t xn, const void *y, size_t yn)
 {
-    GemmPlan p = gemm_plan(m, n, k);
-    double *Ad = reinterpret_cast<double *>(workspace);
-    double *Td = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(workspace) + p.a_bytes);
-    unsigned char *row_nar = reinterpret_cast<unsigned char *>(workspace) + p.a_bytes + p.b_bytes;
-    unsigned char *col_nar = row_nar + (size_t)p.mt * BM;
-    const bool dot = !nota; // TN / TT use the dot-then-combine order
-    size_t na = p.a_bytes / sizeof(double), nb = p.b_bytes / sizeof(double);
+    const uintptr_t a = (uintptr_t)x, b = (uintptr_t)y;
+    return a < b + yn * 4 && b < a + xn * 4;
+}
+
+// Entries from the first to the last of a rows x cols matrix.
+static size_t span(int rows, int cols, int ld) { return (size_t)(cols - 1) * ld + rows; }
+
+static long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
+
+GemmRoute gemm_route(bool nota, bool notb, int m, int n, int k, const uint32_t *A, int lda, const uint32_t *B,
+                     int ldb, const uint32_t *C, int ldc, bool disjoint)
+{
+    if (!disjoint &&
+        (spans_overlap(C, span(m, n, ldc), A, nota ? span(m, k, lda) : span(k, m, lda)) ||
+         spans_overlap(C, span(m, n, ldc), B, notb ? span(k, n, ldb) : span(n, k, ldb))))
+        return GEMM_STAGED;
+    const long long t44 = ceil_div(m, 64) * ceil_div(n, 64), t42 = ceil_div(m, 64) * ceil_div(n, 32);
+    if (t44 >= 2 * SM_COUNT && (double)m * n * k >= GEMM_STAGED_MIN_MADS)
+        return GEMM_STAGED;
+    return t44 >= 2 * SM_COUNT ? GEMM_FUSED_64x64 : (t42 >= SM_COUNT ? GEMM_FUSED_64x32 : GEMM_FUSED_32x32);
+}
+
+template <class Kernel>
+static cudaError_t allow_smem(Kernel fn, size_t smem)
+{
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+template <int TRI, int TM_, int TN_>
+static cudaError_t fused_launch(const TileArgs &P, cudaStream_t stream, const int *stop)
+{
+    const size_t smem = tile_smem_bytes(TM_, TN_);
+    cudaError_t e = allow_smem(gemm_fused_kernel<TRI, TM_, TN_>, smem);
+    if (e != cudaSuccess)
+        return e;
+    const dim3 grid((unsigned)ceil_div(P.m, 16 * TM_), (unsigned)ceil_div(P.n, 16 * TN_));
+    gemm_fused_kernel<TRI, TM_, TN_><<<grid, TILE_THREADS, smem, stream>>>(P, stop);
+    return cudaGetLastError();
+}
+
+template <int TRI>
+static cudaError_t staged_launch(const TileArgs &P, void *workspace, cudaStream_t stream, const int *stop,
+                                 cudaEvent_t *start)
+{
+    const GemmPlan p = gemm_plan(P.m, P.n, P.k);
+    unsigned char *ws = reinterpret_cast<unsigned char *>(workspace);
+    double *Ad = reinterpret_cast<double *>(ws);
+    double *Td = reinterpret_cast<double *>(ws + p.a_bytes);
+    unsigned char *row_nar = ws + p.a_bytes + p.b_bytes;
+    unsigned char *col_nar = row_nar + (size_t)((p.mb + 1) / 2 * 2) * BLK;
+    const size_t na = (size_t)p.mb * p.kt * BK * BLK, nb = (size_t)p.nb * p.kt * BK * BLK;
     cudaError_t e = cudaMemsetAsync(row_nar, 0, p.flag_bytes, stream);
     if (e != cudaSuccess)
         return e;
-    decode_a_kernel<<<grid_for(na, 256), 256, 0, stream>>>(nota, m, k, A, (size_t)lda, p.kt, na, Ad, row_nar);
-    decode_b_kernel<<<grid_for(nb, 256), 256, 0, stream>>>(notb, k, n, B, (size_t)ldb, !dot, alpha, p.kt, nb,
-                                                           Td, col_nar);
-    const size_t smem = (size_t)STAGES * BK * (BM + BN) * sizeof(double) + (size_t)F64_CONST_ENTRIES * sizeof(double);
-    dim3 grid(p.mt, p.nt);
-    e = dot ? cudaFuncSetAttribute(gemm_main_kernel<true, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem)
-            : cudaFuncSetAttribute(gemm_main_kernel<false, TRI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem);
+    decode_kernel<<<grid_for(na + nb, 256), 256, 0, stream>>>(P.nota, P.notb, P.m, P.n, P.k, P.A, P.lda, P.B, P.ldb,
+                                                              P.nota, P.alpha, p.kt, na, na + nb, Ad, Td, row_nar,
+                                                              col_nar);
+    const size_t smem = STEP_TAB_BYTES + (size_t)STAGES * (TM / 2 + TN / 2) * BK * BLK * sizeof(double);
+    e = allow_smem(gemm_main_kernel<TRI>, smem);
     if (e != cudaSuccess)
         return e;
+    if (start)
+        *start = prof_mark(stream); // the main kernel alone is timed
+    const dim3 grid((unsigned)ceil_div(P.m, 16 * TM), (unsigned)ceil_div(P.n, 16 * TN));
+    gemm_main_kernel<TRI><<<grid, TILE_THREADS, smem, stream>>>(!P.nota, P.m, P.n, P.k, p.kt, p.mb, p.nb, P.alpha,
+                                                                P.beta, Ad, Td, P.C, P.ldc, row_nar, col_nar, stop);
+    return cudaGetLastError();
+}
+
+template <int TRI>
+static cudaError_t gemm_launch_route(GemmRoute route, const TileArgs &P, void *workspace, cudaStream_t stream,
+                                     const int *stop)
+{
     const bool prof = g_prof_on;
-    cudaEvent_t e0 = prof ? prof_mark(stream) : nullptr;
-    if (dot)
-        gemm_main_kernel<true, TRI><<<grid, NTHREADS, smem, stream>>>(m, n, k, p.kt, alpha, beta, Ad, Td, C,
-                                                                        (size_t)ldc, row_nar, col_nar, stop);
-    else
-        gemm_main_kernel<false, TRI><<<grid, NTHREADS, smem, stream>>>(m, n, k, p.kt, alpha, beta, Ad, Td, C,
-                                                                         (size_t)ldc, row_nar, col_nar, stop);
+    cudaEvent_t e0 = prof && route != GEMM_STAGED ? prof_mark(stream) : nullptr;
+    const cudaError_t e = route == GEMM_STAGED ? staged_launch<TRI>(P, workspace, stream, stop, prof ? &e0 : nullptr)
+                        : route == GEMM_FUSED_64x64 ? fused_launch<TRI, 4, 4>(P, stream, stop)
+                        : route == GEMM_FUSED_64x32 ? fused_launch<TRI, 4, 2>(P, stream, stop)
+                                                    : fused_launch<TRI, 2, 2>(P, stream, stop);
     if (prof) {
         cudaEvent_t e1 = prof_mark(stream);
         std::lock_guard<std::mutex> lk(g_prof_mu);
         g_prof_events.emplace_back(e0, e1);
     }
-    prof_count(3);
-    return cudaGetLastError();
+    prof_count(route == GEMM_STAGED ? 2 : 1);
+    return e;
+}
+
+template <int TRI>
+static cudaError_t gemm_launch_impl(bool nota, bool notb, int m, int n, int k, uint32_t alpha, const uint32_t *A,
+                                    int lda, const uint32_t *B, int ldb, uint32_t beta, uint32_t *C, int ldc,
+                                    void *workspace, cudaStream_t stream, const int *stop, bool disjoint)
+{
+    const GemmRoute route = gemm_route(nota, notb, m, n, k, A, lda, B, ldb, C, ldc, disjoint);
+    const TileArgs P{nota, notb, m, n, k, alpha, beta, A, (size_t)lda, B, (size_t)ldb, C, (size_t)ldc};
+    return gemm_launch_route<TRI>(route, P, workspace, stream, stop);
 }
 
 cudaError_t gemm_launch(bool nota, bool notb, int m, int n, int k, uint32_t alpha, const uint32_t *A, int lda,
                         const uint32_t *B, int ldb, uint32_t beta, uint32_t *C, int ldc, void *workspace,
-                        cudaStream_t stream)
+                        cudaStream_t stream, bool disjoint)
 {
     return gemm_launch_impl<TRI_FULL>(nota, notb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, workspace, stream,
-                                      nullptr);
+                                      nullptr, disjoint);
 }
 
 cudaError_t gemm_launch_tri(int tri, bool nota, bool notb, int m, int n, int k, uint32_t alpha, const uint32_t *A,
@@ -460,20 +483,12 @@ cudaError_t gemm_launch_tri(int tri, bool nota, bool notb, int m, int n, int k, 
 {
     if (tri == TRI_LOWER)
         return gemm_launch_impl<TRI_LOWER>(nota, notb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, workspace,
-                                           stream, stop);
+                                           stream, stop, true);
     if (tri == TRI_UPPER)
         return gemm_launch_impl<TRI_UPPER>(nota, notb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, workspace,
-                                           stream, stop);
+                                           stream, stop, true);
     return gemm_launch_impl<TRI_FULL>(nota, notb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, workspace, stream,
-                                      stop);
-}
-
-cudaError_t gemm_launch_lower(bool nota, bool notb, int m, int n, int k, uint32_t alpha, const uint32_t *A, int lda,
-                              const uint32_t *B, int ldb, uint32_t beta, uint32_t *C, int ldc, void *workspace,
-                              cudaStream_t stream, const int *stop)
-{
-    return gemm_launch_impl<TRI_LOWER>(nota, notb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, workspace,
-                                       stream, stop);
+                                      stop, true);
 }
 
 cudaError_t scale_launch(int m, int n, bool dot, uint32_t alpha, uint32_t beta, uint32_t *C, int ldc,

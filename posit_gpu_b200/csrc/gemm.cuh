@@ -4,31 +4,29 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "gemm_tile.cuh"
+
 namespace pg {
 
-// Output tile of one CTA and the k-depth of one staged tile.  A thread owns TM x TN
-// outputs; 16 x 16 threads; rows and columns are owned in pairs 32 apart (own_off).
+// The staged route's output tile: 16*TM x 16*TN outputs per CTA of 256 threads, TM x TN per
+// thread (gemm_tile.cuh).  4x4 at 2 CTAs per SM (up to 128 registers: the accumulators, their
+// values at the k tile's start and the operands of a step).
 constexpr int TM = 4; // rows per thread
-constexpr int TN = 2; // columns per thread
-constexpr int BM = 16 * TM;
-constexpr int BN = 16 * TN;
-constexpr int BK = 16;
-constexpr int NTHREADS = 256;
+constexpr int TN = 4; // columns per thread
 constexpr int STAGES = 3;
-constexpr int MIN_CTAS_PER_SM = 3;
-static_assert(TM % 2 == 0 && TN % 2 == 0, "operands are loaded in pairs");
+constexpr int MIN_CTAS_PER_SM = 2;
+constexpr int SM_COUNT = 148;
 
-// Which entries of C a launch writes (gemm_launch_tri).
-constexpr int TRI_FULL = 0;
-constexpr int TRI_LOWER = 1; // row >= column
-constexpr int TRI_UPPER = 2; // row <= column
+// How a product is computed (gemm_route); the bits are the same.
+enum GemmRoute { GEMM_STAGED, GEMM_FUSED_64x64, GEMM_FUSED_64x32, GEMM_FUSED_32x32 };
+constexpr double GEMM_STAGED_MIN_MADS = 536870912.0; // 2^29 multiply-adds
 
 // Error flags a kernel can raise (read back with posit_get_device_error).
 constexpr int DEV_ERR_WAIT_TIMEOUT = 1;
 
 struct GemmPlan {
     int m, n, k;
-    int mt, nt, kt; // tile counts
+    int mb, nb, kt; // 32-row blocks of op(A), 32-column blocks of op(B), k tiles
     size_t a_bytes, b_bytes, flag_bytes;
 };
 
@@ -39,20 +37,20 @@ GemmPlan gemm_plan(int m, int n, int k);
 int rgemm_check_args(char ta, char tb, int m, int n, int k, int lda, int ldb, int ldc, bool &nota, bool &notb);
 size_t gemm_workspace_bytes(int m, int n, int k);
 
-// Decode op(A) and alpha*op(B) (or op(B) for the dot-then-combine order) into the
-// workspace, then run the main kernel.  Device pointers; stream-ordered.
+// The route of one product.  `disjoint`: the caller knows that no entry of C is one of A or
+// B; otherwise a C whose address range meets A's or B's takes the staged route, which has
+// read both before it writes C.
+GemmRoute gemm_route(bool nota, bool notb, int m, int n, int k, const uint32_t *A, int lda, const uint32_t *B,
+                     int ldb, const uint32_t *C, int ldc, bool disjoint);
+
+// C <- alpha*op(A)*op(B) + beta*C.  Device pointers; stream-ordered.  The workspace
+// (gemm_workspace_bytes) is used by the staged route only.
 cudaError_t gemm_launch(bool nota, bool notb, int m, int n, int k, uint32_t alpha,
                         const uint32_t *A, int lda, const uint32_t *B, int ldb, uint32_t beta,
-                        uint32_t *C, int ldc, void *workspace, cudaStream_t stream);
+                        uint32_t *C, int ldc, void *workspace, cudaStream_t stream, bool disjoint);
 
-// Same, writing only the entries on or below the diagonal of C (row >= column), and
+// Same, on disjoint operands, writing all of C, its lower or its upper triangle (TRI_*), and
 // doing nothing when *stop != 0 (stop may be null).
-cudaError_t gemm_launch_lower(bool nota, bool notb, int m, int n, int k, uint32_t alpha,
-                              const uint32_t *A, int lda, const uint32_t *B, int ldb, uint32_t beta,
-                              uint32_t *C, int ldc, void *workspace, cudaStream_t stream, const int *stop);
-
-// Any of the three: all of C, its lower or its upper triangle (TRI_*), doing nothing when
-// *stop != 0 (stop may be null).
 cudaError_t gemm_launch_tri(int tri, bool nota, bool notb, int m, int n, int k, uint32_t alpha,
                             const uint32_t *A, int lda, const uint32_t *B, int ldb, uint32_t beta,
                             uint32_t *C, int ldc, void *workspace, cudaStream_t stream, const int *stop);

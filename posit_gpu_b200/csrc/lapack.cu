@@ -1414,7 +1414,7 @@ cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb,
             if (j + jb < m) {
                 e = gemm_launch(true, true, m - j - jb, nr, jb, 0xC0000000u /* -1 */,
                                             A + (j + jb) + (size_t)j * L, lda, A12, lda, P32_ONE,
-                                            A + (j + jb) + (size_t)(j + jb) * L, lda, gws, st);
+                                            A + (j + jb) + (size_t)(j + jb) * L, lda, gws, st, true);
                 if (e != cudaSuccess)
                     return e;
             }
@@ -1461,7 +1461,7 @@ cudaError_t rpotrf_lower_launch(int n, uint32_t *A, int lda, int nb, int *info, 
         if (j + jb < n) {
             const int nr = n - j - jb;
             const uint32_t *L21 = A + (j + jb) + (size_t)j * L;
-            cudaError_t e = gemm_launch_lower(true, false, nr, nr, jb, 0xC0000000u /* -1 */, L21, lda, L21,
+            cudaError_t e = gemm_launch_tri(TRI_LOWER, true, false, nr, nr, jb, 0xC0000000u /* -1 */, L21, lda, L21,
                                               lda, P32_ONE, A + (j + jb) + (size_t)(j + jb) * L, lda, gws, st, info);
             if (e != cudaSuccess)
                 return e;

@@ -634,10 +634,10 @@ PG_HD double f64_from_hi(uint32_t h)
 #endif
 }
 
-// The rounding constant's high word for an FP64 value whose top 12 bits (sign and
-// exponent field) are `top`: C = 1.5 * 2^(e + 52 - fb), the same for either sign.  A binade
-// outside the fast window gets a NaN instead, so that a product or sum falling there comes
-// out NaN and is redone exactly.  Binade 0 holds zero (a zero product or an exactly
+// The rounding constant's high word for an FP64 value whose exponent field is the low 11
+// bits of `top`: C = 1.5 * 2^(e + 52 - fb), the same for either sign.  A binade outside the
+// fast window gets a NaN instead, so that a product or sum falling there comes out NaN and
+// is redone by f64_posit_mac_exact.  Binade 0 holds zero (a zero product or an exactly
 // cancelling sum): in the window.
 PG_HD uint32_t f64_round_const_top(uint32_t top)
 {
@@ -646,18 +646,14 @@ PG_HD uint32_t f64_round_const_top(uint32_t top)
         return 0x7FF80000u;
     return f64_round_const_hi(eb);
 }
-// The table the GEMM kernels keep in shared memory: f64_round_const_top for every top
-// 12 bits, so that a lookup is one shift of the value's high word.
-constexpr int F64_CONST_ENTRIES = 4096;
+// The table the kernels keep in shared memory: f64_round_const_top for every exponent
+// field.  The sign bit is masked off, so that two lanes whose values differ only in sign
+// read the same word instead of two words 8 KB apart, i.e. in the same bank.
+constexpr int F64_CONST_ENTRIES = 2048;
 struct F64ConstTable {
     const uint32_t *tab;
-    PG_HD_MEMBER uint32_t hi(double x) const { return tab[f64_hi(x) >> 20]; }
+    PG_HD_MEMBER uint32_t hi(double x) const { return tab[(f64_hi(x) >> 20) & 0x7FF]; }
     PG_HD_MEMBER double operator()(double x) const { return f64_from_hi(hi(x)); }
-};
-struct F64ConstTable8 {
-    const double *tab;
-    PG_HD_MEMBER uint32_t hi(double x) const { return f64_hi(tab[f64_hi(x) >> 20]); }
-    PG_HD_MEMBER double operator()(double x) const { return tab[f64_hi(x) >> 20]; }
 };
 struct F64ConstComputed {
     PG_HD_MEMBER uint32_t hi(double x) const { return f64_round_const_top(f64_hi(x) >> 20); }
@@ -669,37 +665,86 @@ struct F64ConstComputed {
 //   q = fma(t, a, Cp) - Cp    the exact product rounded once to the posit grid of its
 //                             binade (taken from fl(t*a); where that rounds up to a power
 //                             of two both give that power);
-//   s = c + q                 the FP64 sum, tested for exactness: s - c == q and s - q == c
-//                             (Fast2Sum on the larger operand makes an inexact s fail it);
-//   r = (s + Cs) - Cs         the exact sum rounded to the posit grid of its binade.
-// `fail` is set when the step must be done exactly instead: an inexact FP64 sum (a
-// product outside the fast window has a NaN constant, so q and s are NaN and fail the
-// test), or a sum outside the fast window (its table entry is the NaN marker).
-// Flagging every inexact sum is conservative: beyond 30 binades the rounded sum would be
-// right anyway, but that case is rare on the data the GEMM sees.
+//   s = c + q                 the FP64 sum, rounded to 53 bits;
+//   r = (s + Cs) - Cs         s rounded to the posit grid of its binade.
+// The second rounding of the sum is harmless although s may be inexact.  r differs from
+// the exact sum rounded once only if s is inexact and lies exactly half way between two
+// posits, s = (N + 1/2) u with u = 2^(e_s - fb_s) the grid there.  Call the operand of
+// larger magnitude X, the other Y.  X is a multiple of its own grid, and no step of that
+// grid is finer than u unless the sum carried into the next binade, so reaching a half
+// step takes |Y| >= u/2 less a rounding, i.e. e_Y >= e_s - fb_s - 2; and s can only be
+// inexact through Y's last bit, e_Y - fb_Y <= e_s - 53.  Together fb_s + fb_Y >= 51, that
+// is, regime runs with run_s + run_Y <= 5, which puts e_s and e_Y at most 4*5 - 1 = 19
+// binades apart, while the second condition wants e_s - e_Y >= 53 - fb_Y >= 26.  So it
+// cannot happen.  (The earlier form tested s - c == q and s - q == c on every step: four
+// of its ten FP64 instructions.)  The reference's own truncating alignment agrees with
+// the exact sum rounded once, see dadd_core.
+// `fail` is set when the step must be done by f64_posit_mac_exact instead: a product or a
+// sum outside the fast window (its constant is NaN, and so is r) or a NaN operand.
 template <class ConstOf>
 PG_HD double f64_posit_mac(double c, double t, double a, ConstOf const_of, bool &fail)
 {
-    const double p = f64_mul(t, a);
-    const double Cp = const_of(p);
+    const double Cp = const_of(f64_mul(t, a));
     const double q = f64_add(f64_fma(t, a, Cp), -Cp);
     const double s = f64_add(c, q);
-    // s is exact iff s - c == q and s - q == c: with the operands ordered by exponent,
-    // s - larger is exact (Dekker's Fast2Sum), so an inexact s leaves that difference
-    // unequal to the smaller operand
-    const bool inexact = (f64_add(s, -c) != q) | (f64_add(s, -q) != c);
     const uint32_t cs_hi = const_of.hi(s);
     const double Cs = f64_from_hi(cs_hi);
     const double r = f64_add(f64_add(s, Cs), -Cs);
-    fail = inexact | (cs_hi == 0x7FF80000u); // the sum's binade is outside the fast window
+    fail = cs_hi == 0x7FF80000u; // s NaN, or its binade outside the fast window
     return r;
 }
 
-// The same step on patterns (the exact path).  Inlined: a called function in the GEMM
-// kernels' inner loop made them fault and crawl on inputs that take this path often.
+// x rounded to posit32 where its binade e lies outside the fast window (regime runs of 28
+// to 30, where the pattern has no fraction and 2, 1 or 0 exponent bits left, and beyond,
+// where the reference saturates; kernel_entry.cl:184-213, 504-533): the result is a power
+// of two, the exponent with its `drop` lowest bits rounded off, the guard bit being the
+// highest bit dropped and, for run 30, the lower exponent bit in neither the guard nor the
+// sticky bits.  x is exact there: a product of two posits has at most 30 significant bits
+// that far out, a sum of posits lies on a grid of powers of two.  From the binade and the 52
+// fraction bits of |x|, the result's exponent.
+PG_HD constexpr int32_t outside_exponent(int32_t e, uint64_t frac)
+{
+    if (e >= 120)
+        return 120; // maxpos
+    if (e < -120)
+        return -120; // minpos
+    const int32_t k = e >> 2, run = (k ^ (k >> 31)) + 1, drop = run - 28;
+    const uint32_t guard = drop == 0 ? (uint32_t)(frac >> 51) : ((uint32_t)e >> (drop - 1)) & 1u;
+    const bool sticky = (drop == 0 ? frac << 13 : frac) != 0;
+    const uint32_t lsb = drop == 2 ? (k < 0 ? 1u : 0u) : ((uint32_t)e >> drop) & 1u;
+    const int32_t r = e & ~((1 << drop) - 1);
+    return guard && (sticky || lsb) ? r + (1 << drop) : r;
+}
+// NaN stays NaN.
+PG_HD double f64_round_outside(double x)
+{
+    if (x != x)
+        return x;
+    const uint64_t b = f64_bits(x);
+    const int32_t r = outside_exponent((int32_t)((b >> 52) & 0x7FF) - 1023, b & 0xFFFFFFFFFFFFFull);
+    return f64_from_bits((b & 0x8000000000000000ull) | ((uint64_t)(uint32_t)(r + 1023) << 52));
+}
+
+// The FP64 value x (exact, or a sum as in f64_posit_mac) rounded to posit32, any binade.
+PG_HD double f64_round_any(double x)
+{
+    const uint32_t ch = f64_round_const_top(f64_hi(x) >> 20);
+    if (ch == 0x7FF80000u)
+        return f64_round_outside(x);
+    const double C = f64_from_hi(ch);
+    return f64_add(f64_add(x, C), -C);
+}
+
+// The same step for any operands: a product or a sum outside the fast window is rounded by
+// f64_round_outside.  Inlined: a called function in the GEMM kernels' inner loop made them
+// fault and crawl on inputs that take this path often.
 PG_HD double f64_posit_mac_exact(double c, double t, double a)
 {
-    return p32_to_double(padd(p32_from_double(c), pmul(p32_from_double(t), p32_from_double(a))));
+    const double p = f64_mul(t, a);
+    const uint32_t ch = f64_round_const_top(f64_hi(p) >> 20);
+    const double Cp = f64_from_hi(ch);
+    const double q = ch == 0x7FF80000u ? f64_round_outside(p) : f64_add(f64_fma(t, a, Cp), -Cp);
+    return f64_round_any(f64_add(c, q));
 }
 
 // c + t*a with the exact path taken where the FP64 step is flagged.
@@ -722,13 +767,13 @@ PG_HD double f64_posit_mac_checked(double c, double t, double a, ConstOf const_o
 // x*y rounded as p32_mul (kernel_entry.cl:399-538) rounds it, both posit32 values held in
 // FP64: the exact product rounded once onto the posit grid of its binade, fma(x, y, Cp) - Cp
 // (the product step of f64_posit_mac).  A product outside the fast window (its constant is
-// NaN) and NaR operands (NaN) go through the pattern routine.
+// NaN) is rounded by f64_round_outside, and NaR operands (NaN) stay NaN.
 template <class ConstOf>
 PG_HD double f64_posit_mul_checked(double x, double y, ConstOf const_of)
 {
     const double Cp = const_of(f64_mul(x, y));
     const double q = f64_add(f64_fma(x, y, Cp), -Cp);
-    return q == q ? q : p32_to_double(pmul(p32_from_double(x), p32_from_double(y)));
+    return q == q ? q : f64_round_outside(f64_mul(x, y));
 }
 
 // FP64 -> posit32 for a value that IS a posit32 value (an output of the FP64 steps or of
