@@ -739,7 +739,7 @@ static cudaError_t launch_lun(int nrhs, int threads, const uint32_t *U, size_t l
 // Lower, transposed (Rtrsm.cpp:175-186): one block per right-hand side; the column is
 // staged in shared memory (when it fits) and one thread runs the whole dependent chain
 // (trsm_chain.cuh).
-constexpr int LLT_SMEM_MAX = 227 * 1024;
+constexpr int LLT_SMEM_MAX = 227 * 1024 - 128; // dynamic, beside a row's scalars
 
 __global__ void __launch_bounds__(32) trsm_llt_kernel(const uint32_t *__restrict__ L, size_t ldl,
                                                       uint32_t *__restrict__ B, size_t ldb, int m, bool staged,
@@ -764,236 +764,164 @@ __global__ void __launch_bounds__(32) trsm_llt_kernel(const uint32_t *__restrict
         bcol[i] = s_col[i];
 }
 
-// The dot-form solves split over warps (below): the scan form's window parameters.
-constexpr int LLT_SCAN_E = 4;
-constexpr int LLT_SHORT_WINDOW = 64; // a window that ends sooner ...
-constexpr int LLT_SEQ_STEPS = 32;    // ... is followed by this many sequential steps
-
-// Term storage: FP64, or (for long columns) the posit32 patterns of the products.
-template <class T>
-struct LltTerms;
-template <>
-struct LltTerms<double> {
-    using View = TermsF64;
-    __device__ static double store(uint32_t p) { return p32_to_double(p); }
-};
-template <>
-struct LltTerms<uint32_t> {
-    using View = TermsP32;
-    __device__ static uint32_t store(uint32_t p) { return p; }
-};
-
 // ---------------------------------------------------------------------------
-// The dot-form solve with the row's windows spread over a group of warps.
+// The dot-form solves, one block per right-hand side.
 // ---------------------------------------------------------------------------
 // Rtrsm('L', 'L', 'T'), Rtrsm.cpp:175-186: for i = m-1 down to 0, t = b_i, t = t - a_ki*b_k
 // for k = i+1 .. m-1 in order, b_i = t / a_ii (UPPER: Rtrsm('L', 'U', 'T'),
-// Rtrsm.cpp:160-173, rows in increasing order, terms k = 0 .. i-1; the warps scan the terms
-// k <= i-2, computed while row i-1 ran, then add the last one from the value just
-// finished).  One block of 2 * LLT_GROUP_WARPS warps per right-hand side: the first
-// LLT_GROUP_WARPS warps (the consumer group) sum each row in windows of
-// LLT_GROUP_WARPS * 32 * LLT_SCAN_E terms in the scan form (trsm_chain.cuh) -- the first term
-// (the b just finished) by one exact step -- while the others compute the next row's terms
-// -a_k * b_k (all whose b_k are final) into the other half of a double buffer.  A
-// window is the warp scan of step maps in every consumer warp, then each warp's composed map
-// goes to shared memory, a named barrier (the consumer group only), each warp composes the
-// maps of the warps before it with its own exclusive prefix and walks its addends, each warp
-// reports its first step the scan form does not cover, a named barrier, and every consumer
-// thread takes the first such step of the window (or the window's end value).  Every
-// consumer thread then holds the same running value; the exact steps and the sequential
-// runs after a window cut short run in every consumer thread alike (no broadcast needed).
-constexpr int LLT_GROUP_WARPS = 4;
-constexpr int LLT_GROUP_THREADS = 2 * LLT_GROUP_WARPS * 32;
+// Rtrsm.cpp:160-173, rows in increasing order, terms k = 0 .. i-1).  A right-hand side is one
+// chain of m(m-1)/2 dependent additions, so the warp that adds (warp 0) bounds the solve;
+// the other three compute the next row's terms -a_k * b_k (all whose b_k are final) into the
+// other half of a double buffer, and its diagonal's reciprocal, meanwhile.  Warp 0 sums a row
+// with warp_chain (trsm_chain.cuh); the term of the b just finished (the first one, UPPER:
+// the last) it forms itself.  Four warps: one per sub-partition of the SM, so nothing else
+// issues where the chain runs.
+// NaR travels as NaN; a NaR term sets its row's flag and is replaced by 0.
+constexpr int LTX_THREADS = 128;
 
-// One window's exchange between the consumer warps; two of them, used by turns, so that a
-// window's results may be read while the next window's are written.
-struct __align__(16) GroupScan {
-    SegFn wt[LLT_GROUP_WARPS];     // each consumer warp's composed map
-    int jbad[LLT_GROUP_WARPS];     // each warp's first uncovered step (-1: none)
-    int32_t Mbad[LLT_GROUP_WARPS]; // M before that step
-    int32_t Mend;                  // M after the window's last addend
+// The solution column in shared memory: FP64, or patterns where the columns are long.
+struct LtxCol64 {
+    double *b;
+    static constexpr size_t BYTES = 8;
+    __device__ double get(int k) const { return b[k]; }
+    __device__ void set(int k, double v) const { b[k] = v; }
 };
-static_assert(LLT_GROUP_WARPS == 4, "the window's results are read as int4 vectors");
-
-__device__ __forceinline__ void group_bar() { asm volatile("bar.sync 1, %0;" ::"r"(LLT_GROUP_WARPS * 32) : "memory"); }
-
-template <int E, class Q>
-__device__ double group_chain_scan(double t, Q q, int pos, int end, GroupScan *gsb, int &turn)
+struct LtxCol32 {
+    uint32_t *b;
+    static constexpr size_t BYTES = 4;
+    __device__ double get(int k) const { return p32_to_double(b[k]); }
+    __device__ void set(int k, double v) const { b[k] = p32_from_double_exact(v); }
+};
+template <class Terms>
+struct LtxColOf;
+template <>
+struct LtxColOf<ChainTerms64> {
+    using Col = LtxCol64;
+};
+template <>
+struct LtxColOf<ChainTerms32> {
+    using Col = LtxCol32;
+};
+template <class Terms>
+static size_t ltx_smem_bytes(int m)
 {
-    constexpr unsigned FULL = 0xFFFFFFFFu;
-    const int ct = threadIdx.x, lane = ct & 31, w = ct >> 5;
-    while (pos < end) {
-        GroupScan *gs = gsb + turn;
-        SegParams sp;
-        if (!seg_begin(t, sp)) { // zero, or outside the fast window: one exact step
-            t = chain_add_one(t, q[pos]);
-            ++pos;
-            continue;
-        }
-        const int wend = min(end, pos + LLT_GROUP_WARPS * 32 * E);
-        const int j0 = pos + ct * E;
-        SegFn fe[E];
-        int32_t K[E];
-        bool rk[E];
-        SegFn f = {0, 0};
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const double qv = j0 + e < wend ? q[j0 + e] : 0.0; // 0 is the identity map
-            fe[e] = seg_fn(qv, sp, K[e], rk[e]);
-            f = seg_then(f, fe[e]);
-        }
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            SegFn o;
-            o.c0 = __shfl_up_sync(FULL, f.c0, off);
-            o.c1 = __shfl_up_sync(FULL, f.c1, off);
-            if (lane >= off)
-                f = seg_then(o, f);
-        }
-        SegFn ex;
-        ex.c0 = __shfl_up_sync(FULL, f.c0, 1);
-        ex.c1 = __shfl_up_sync(FULL, f.c1, 1);
-        if (lane == 0)
-            ex = SegFn{0, 0};
-        if (lane == 31)
-            gs->wt[w] = f;
-        group_bar();
-        const int4 wt01 = *reinterpret_cast<const int4 *>(&gs->wt[0]);
-        const int4 wt23 = *reinterpret_cast<const int4 *>(&gs->wt[2]);
-        SegFn pre = {0, 0};
-        if (w > 0)
-            pre = SegFn{wt01.x, wt01.y};
-        if (w > 1)
-            pre = seg_then(pre, SegFn{wt01.z, wt01.w});
-        if (w > 2)
-            pre = seg_then(pre, SegFn{wt23.x, wt23.y});
-        int32_t M = seg_apply(seg_then(pre, ex), sp.M0);
-        int jbad = -1;
-        int32_t Mbad = 0;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const bool live = (jbad < 0) & (j0 + e < wend);
-            const bool ok = seg_valid(M, K[e], rk[e], sp);
-            if (live & !ok) {
-                jbad = j0 + e;
-                Mbad = M;
-            }
-            if (live & ok)
-                M = seg_apply(fe[e], M);
-        }
-        const unsigned bal = __ballot_sync(FULL, jbad >= 0);
-        if (bal == 0) {
-            if (lane == 0)
-                gs->jbad[w] = -1;
-        } else if (lane == __ffs(bal) - 1) {
-            gs->jbad[w] = jbad;
-            gs->Mbad[w] = Mbad;
-        }
-        if (ct == (wend - 1 - pos) / E) // the thread holding the window's last addend
-            gs->Mend = M;
-        group_bar();
-        // the first warp's first uncovered step (warps hold increasing positions)
-        const int4 jb4 = *reinterpret_cast<const int4 *>(gs->jbad);
-        const int4 mb4 = *reinterpret_cast<const int4 *>(gs->Mbad);
-        const int32_t Me = gs->Mend;
-        int js = jb4.w;
-        int32_t Ms = mb4.w;
-        if (jb4.z >= 0) { js = jb4.z; Ms = mb4.z; }
-        if (jb4.y >= 0) { js = jb4.y; Ms = mb4.y; }
-        if (jb4.x >= 0) { js = jb4.x; Ms = mb4.x; }
-        // The next window writes the other exchange; this one is written again only after
-        // the next window's first group barrier, which every consumer reaches after the
-        // reads above.
-        turn ^= 1;
-        if (js < 0) {
-            t = sp.us * (double)Me;
-            pos = wend;
-        } else {
-            t = chain_add_one(sp.us * (double)Ms, q[js]);
-            const bool cut_short = js - pos < LLT_SHORT_WINDOW;
-            pos = js + 1;
-            if (cut_short) {
-                const int cnt = min(LLT_SEQ_STEPS, end - pos);
-                t = chain_add_run_reg(t, q + pos, cnt);
-                pos += cnt;
-            }
-        }
-    }
-    return t;
+    return 2 * Terms::bytes(m) + (size_t)m * LtxColOf<Terms>::Col::BYTES;
 }
 
-template <class T, bool UPPER = false>
-__global__ void __launch_bounds__(LLT_GROUP_THREADS) trsm_ltx_group_kernel(const uint32_t *__restrict__ L,
-                                                                           size_t ldl, uint32_t *__restrict__ B,
-                                                                           size_t ldb, int m, bool unit,
-                                                                           const int *__restrict__ info)
+// What warp 0 needs of a row besides its terms.
+struct LtxRow {
+    double diag, recip; // a_ii and fl(1/a_ii)
+    double near;        // the coefficient of the b finished last
+    int nar;            // a term was NaR
+};
+
+template <class Terms, bool UPPER>
+__global__ void __launch_bounds__(LTX_THREADS) trsm_ltx_kernel(const uint32_t *__restrict__ L, size_t ldl,
+                                                               uint32_t *__restrict__ B, size_t ldb, int m, bool unit,
+                                                               const int *__restrict__ info)
 {
-    extern __shared__ __align__(16) unsigned char smem_pc[];
-    T *s_q = reinterpret_cast<T *>(smem_pc); // [2][m]: terms
-    uint32_t *s_b = reinterpret_cast<uint32_t *>(s_q + 2 * (size_t)m);
-    __shared__ uint32_t s_nar[2];
-    __shared__ GroupScan s_gs[2];
+    extern __shared__ __align__(16) unsigned char smem_ltx[];
+    __shared__ LtxRow s_row[2];
+    using Col = typename LtxColOf<Terms>::Col;
     if (info && *info != 0) // a factorization stopped before this solve
         return;
+    auto terms = [&](int half) {
+        Terms q;
+        q.q = reinterpret_cast<decltype(q.q)>(smem_ltx + half * Terms::bytes(m));
+        return q;
+    };
+    Col s_b;
+    s_b.b = reinterpret_cast<decltype(s_b.b)>(smem_ltx + 2 * Terms::bytes(m));
     uint32_t *bcol = B + (size_t)blockIdx.x * ldb;
     const int tid = threadIdx.x;
-    constexpr int NC = LLT_GROUP_WARPS * 32; // consumer threads
-    for (int k = tid; k < m; k += LLT_GROUP_THREADS)
-        s_b[k] = bcol[k];
+    for (int k = tid; k < m; k += LTX_THREADS)
+        s_b.set(k, p32_to_double(bcol[k]));
+    // Terms outside a row's range are zero for warp_chain: rows grow, so what no earlier row
+    // wrote is still this.
+    for (int k = tid; k < (int)(2 * Terms::bytes(m) / sizeof(typename Terms::Word)); k += LTX_THREADS)
+        reinterpret_cast<typename Terms::Word *>(smem_ltx)[k] = 0;
+    auto row_of = [&](int step) { return UPPER ? step : m - 1 - step; };
+    // the row's diagonal and nearest coefficient
+    auto head = [&](int step) {
+        const int i = row_of(step);
+        const uint32_t *li = L + (size_t)i * ldl;
+        LtxRow &r = s_row[step & 1];
+        r.diag = unit ? 1.0 : p32_to_double(li[i]);
+        r.recip = 1.0 / r.diag;
+        r.near = step > 0 ? p32_to_double(li[UPPER ? i - 1 : i + 1]) : 0.0;
+    };
     if (tid < 2)
-        s_nar[tid] = 0;
+        s_row[tid].nar = 0;
+    if (tid == 32)
+        head(0);
     __syncthreads();
-    uint32_t xprev = 0; // the row finished last, b_{i+1} (lower) or b_{i-1} (upper) (consumers)
-    int turn = 0;       // which of s_gs the next window uses (consumers)
+    double x = 0.0; // the b finished last (warp 0)
     for (int step = 0; step < m; ++step) {
-        const int i = UPPER ? step : m - 1 - step;
-        const int cur = step & 1;
-        if (tid < NC) {
-            const uint32_t *li = L + (size_t)i * ldl;
-            const uint32_t bi = s_b[i];
-            uint32_t nar = (bi == P32_NAR) | s_nar[cur];
-            double c = p32_to_double(bi == P32_NAR ? 0u : bi);
-            const typename LltTerms<T>::View q{s_q + (size_t)cur * m};
-            if (!UPPER && i + 1 < m) {
-                c = chain_add_one(c, llt_term(li[i + 1], xprev, &nar));
-                c = group_chain_scan<LLT_SCAN_E>(c, q, i + 2, m, s_gs, turn);
+        const int i = row_of(step), cur = step & 1;
+        if (tid < 32) {
+            const LtxRow r = s_row[cur];
+            double t = s_b.get(i);
+            bool nar = t != t || r.nar;
+            double near = 0.0; // -a*b of the b just finished
+            if (step > 0) {
+                near = f64_posit_mul_checked(-x, r.near, F64ConstComputed{});
+                if (near != near) {
+                    nar = true;
+                    near = 0.0;
+                }
             }
-            if (UPPER && i >= 1) {
-                c = group_chain_scan<LLT_SCAN_E>(c, q, 0, i - 1, s_gs, turn);
-                c = chain_add_one(c, llt_term(li[i - 1], xprev, &nar));
+            if (nar)
+                t = 0.0;
+            if (!UPPER && step > 0) {
+                t = f64_round_any(f64_add(t, near));
+                t = warp_chain(t, terms(cur), i + 2, m);
             }
-            uint32_t t = nar ? P32_NAR : p32_from_double(c);
+            if (UPPER && step > 0) {
+                t = warp_chain(t, terms(cur), 0, i - 1);
+                t = f64_round_any(f64_add(t, near));
+            }
+            x = nar ? p32_to_double(P32_NAR) : t;
             if (!unit)
-                t = pdiv_est(t, li[i]);
-            xprev = t;
-            group_bar(); // every consumer has read s_nar[cur]
+                x = f64_posit_div(x, r.diag, r.recip);
+            __syncwarp(); // every lane has read the row
             if (tid == 0) {
-                s_b[i] = t;
-                s_nar[cur] = 0;
+                s_b.set(i, x);
+                s_row[cur].nar = 0;
             }
         } else if (step + 1 < m) {
             // the terms of the next row whose b_k are final: k = i+1 .. m-1 of row i-1
             // (lower), k = 0 .. i-1 of row i+1 (upper)
-            const int nxt = UPPER ? i + 1 : i - 1;
             const int kbeg = UPPER ? 0 : i + 1, kend = UPPER ? i : m;
-            const uint32_t *lp = L + (size_t)nxt * ldl;
-            T *qn = s_q + (size_t)(cur ^ 1) * m;
-            uint32_t nar = 0;
-            for (int k = kbeg + (tid - NC); k < kend; k += LLT_GROUP_THREADS - NC) {
-                const uint32_t p = pmul(0u - s_b[k], lp[k]); // (-b)*a == -(a*b) bit for bit
-                nar |= p == P32_NAR;
-                qn[k] = LltTerms<T>::store(p == P32_NAR ? 0u : p);
+            const uint32_t *lp = L + (size_t)row_of(step + 1) * ldl;
+            if (tid == 32)
+                head(step + 1);
+            const Terms q = terms(cur ^ 1);
+            int nar = 0;
+            constexpr int P = LTX_THREADS - 32, U = 8; // U loads in flight per thread
+            for (int k = kbeg + (tid - 32); k < kend; k += U * P) {
+                uint32_t l[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    l[u] = k + u * P < kend ? lp[k + u * P] : 0u;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (k + u * P < kend) {
+                        double v = f64_posit_mul_checked(-s_b.get(k + u * P), p32_to_double(l[u]), F64ConstComputed{});
+                        if (v != v) {
+                            nar = 1;
+                            v = 0.0;
+                        }
+                        q.set(k + u * P, v);
+                    }
             }
             if (nar)
-                s_nar[cur ^ 1] = 1;
+                s_row[cur ^ 1].nar = 1;
         }
         __syncthreads();
     }
-    for (int k = tid; k < m; k += LLT_GROUP_THREADS)
-        bcol[k] = s_b[k];
+    for (int k = tid; k < m; k += LTX_THREADS)
+        bcol[k] = p32_from_double_exact(s_b.get(k));
 }
-
-size_t llt_pc_smem_bytes(int m, size_t term_bytes) { return (size_t)m * (2 * term_bytes + 4); }
 
 // ---------------------------------------------------------------------------
 // Cholesky panel (lower)
@@ -1572,34 +1500,25 @@ cudaError_t rgetrs_launch(int n, int nrhs, const uint32_t *A, int lda, const int
 
 // The dot-form solves with the triangle transposed: L^-T B (Rtrsm('L', 'L', 'T'),
 // Rtrsm.cpp:175-186) or, with `upper`, U^-T B (Rtrsm('L', 'U', 'T'), Rtrsm.cpp:160-173).
-// One block per right-hand side: the scan-form kernel where its terms fit in shared
-// memory (FP64 where 20n bytes fit, patterns where 12n do), else one thread's chain.
+// One block per right-hand side: trsm_ltx_kernel where its terms fit in shared memory
+// (FP64 where 26n bytes do, patterns where 12n do), else one thread's chain.
 // A nonzero *info (when given) turns the solve into a no-op.
 static cudaError_t launch_ltx(bool upper, bool unit, int n, int nrhs, const uint32_t *A, int lda, uint32_t *B,
                               int ldb, const int *info, cudaStream_t st)
 {
     cudaError_t e = cudaSuccess;
-    const size_t pc8 = llt_pc_smem_bytes(n, sizeof(double)), pc4 = llt_pc_smem_bytes(n, sizeof(uint32_t));
-    if (pc8 <= (size_t)LLT_SMEM_MAX || pc4 <= (size_t)LLT_SMEM_MAX) {
-        const bool f64 = pc8 <= (size_t)LLT_SMEM_MAX;
-        const size_t pc = f64 ? pc8 : pc4;
-        const void *fn = f64 ? (upper ? (const void *)trsm_ltx_group_kernel<double, true>
-                                      : (const void *)trsm_ltx_group_kernel<double, false>)
-                             : (upper ? (const void *)trsm_ltx_group_kernel<uint32_t, true>
-                                      : (const void *)trsm_ltx_group_kernel<uint32_t, false>);
-        if (pc > 48 * 1024) {
-            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pc);
+    const size_t b64 = ltx_smem_bytes<ChainTerms64>(n), b32 = ltx_smem_bytes<ChainTerms32>(n);
+    if (b64 <= (size_t)LLT_SMEM_MAX || b32 <= (size_t)LLT_SMEM_MAX) {
+        const bool f64 = b64 <= (size_t)LLT_SMEM_MAX;
+        const size_t bytes = f64 ? b64 : b32;
+        auto *fn = f64 ? (upper ? trsm_ltx_kernel<ChainTerms64, true> : trsm_ltx_kernel<ChainTerms64, false>)
+                       : (upper ? trsm_ltx_kernel<ChainTerms32, true> : trsm_ltx_kernel<ChainTerms32, false>);
+        if (bytes > 48 * 1024) {
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
             if (e != cudaSuccess)
                 return e;
         }
-        if (f64 && upper)
-            trsm_ltx_group_kernel<double, true><<<nrhs, LLT_GROUP_THREADS, pc, st>>>(A, lda, B, ldb, n, unit, info);
-        else if (f64)
-            trsm_ltx_group_kernel<double, false><<<nrhs, LLT_GROUP_THREADS, pc, st>>>(A, lda, B, ldb, n, unit, info);
-        else if (upper)
-            trsm_ltx_group_kernel<uint32_t, true><<<nrhs, LLT_GROUP_THREADS, pc, st>>>(A, lda, B, ldb, n, unit, info);
-        else
-            trsm_ltx_group_kernel<uint32_t, false><<<nrhs, LLT_GROUP_THREADS, pc, st>>>(A, lda, B, ldb, n, unit, info);
+        fn<<<nrhs, LTX_THREADS, bytes, st>>>(A, lda, B, ldb, n, unit, info);
         return cudaGetLastError();
     }
     const size_t col = (size_t)n * 4;

@@ -83,4 +83,25 @@ PG_HD uint32_t psqrt_est(uint32_t a)
     return pack_exact(0, (d.s - odd) / 2, r << 31, rem != 0);
 }
 
+// t / a rounded, both posit32 values held in FP64 (NaN for NaR), given rc = fl(1/a): the
+// quotient to within an ulp by one correction step (Markstein: q0 = t rc, r = t - q0 a
+// exactly by FMA, q = q0 + r rc), rounded onto the posit grid of its binade.  That is the
+// rounded quotient unless q is so near half way between two posits that its last bits
+// decide (within 2^-50 of its size; the exact ties are among these), or the quotient is
+// outside the fast window, or an operand is zero or NaN: those take the integer quotient.
+// A dependent chain of about 110 cycles on B200 against 490 for pdiv_est.
+PG_HD double f64_posit_div(double t, double a, double rc)
+{
+    const double q0 = f64_mul(t, rc);
+    const double q = f64_fma(f64_fma(-q0, a, t), rc, q0);
+    const uint32_t ch = f64_round_const_top(f64_hi(q) >> 20);
+    const double C = f64_from_hi(ch);
+    const double z = f64_add(f64_add(q, C), -C);
+    const double half = f64_from_hi((ch & 0x7FF00000u) - (53u << 20)); // half the grid's spacing
+    const double d = fabs(f64_add(q, -z)), off = fabs(f64_add(d, -half));
+    if (off > f64_mul(fabs(q), 8.8817841970012523e-16 /* 2^-50 */) && q != 0.0)
+        return z;
+    return p32_to_double(pdiv_est(p32_from_double_exact(t), p32_from_double_exact(a)));
+}
+
 } // namespace pg

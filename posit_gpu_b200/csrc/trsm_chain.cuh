@@ -8,9 +8,13 @@
 //   * llt_chain: one thread runs a right-hand side's whole chain with the accumulator
 //     held in the decoded integer form (the batched kernel; very long columns);
 //   * chain_add_run / chain_add_run_reg: one thread's chain of additions in FP64, the
-//     products computed elsewhere;
-//   * the scan form (below): a warp sums a row's additions as a parallel prefix of step
-//     maps on the posit grid (lapack.cu's transposed-solve kernel).
+//     products computed elsewhere (chain_add_run is the sequence the tests hold the others
+//     to);
+//   * warp_chain (end of this file): a warp sums a row's additions with the running value
+//     biased onto its binade's grid, one FP64 addition per step, and where the value is calm
+//     as a parallel prefix of step maps (lapack.cu's transposed-solve kernel and the
+//     batched kernel).  The scan form it grew from, one map per addend, stays written out
+//     for the host.
 //
 // For the one-thread chains latency is everything.  Only the addition depends on the previous step: loads,
 // decoding and the product of step k+1 can overlap the addition of step k, but not across
@@ -107,19 +111,16 @@ PG_HD void llt_chain(const uint32_t *__restrict__ L, size_t ldl, uint32_t *b, in
 // ---------------------------------------------------------------------------
 // A posit32 value is exact in FP64 (at most 28 significant bits, scale within +-120).
 // One step t + q of the chain is then:
-//   s = fl64(t + q)        exact whenever the operands' binades are at most 24 apart
-//                          (the sum needs at most 29 + 24 bits);
+//   s = fl64(t + q);
 //   r = (s + C) - C        C = 1.5 * 2^(e + 52 - fb), e the binade of s and fb the posit's
 //                          fraction width there: round to nearest even at the posit's last
 //                          fraction bit (ties to the even pattern, whose parity is the
 //                          fraction's).
-// The reference's p32_add is that rounding of the exact sum (within its 64-bit frame; an
-// addend more than 30 binades down contributes nothing, which is also what rounding the
-// exact sum gives).  More than 30 binades apart, fl64(t + q) may be inexact but lies far
-// from every rounding boundary, so r is still right.  A step is handed to the exact path
-// when the operands are 25..30 binades apart (the FP64 rounding could meet a posit tie),
-// or when the sum's scale is outside the fast window (regime longer than 27 bits, fewer
-// than one fraction bit; this includes an exactly cancelling sum, whose FP64 value is 0).
+// Where s is inexact it never lies half way between two posits (posit32.cuh,
+// f64_posit_mac), so r is the exact sum rounded once, which is the reference's p32_add.  A
+// step is handed to the exact path when the sum's scale is outside the fast window (regime
+// longer than 27 bits, fewer than one fraction bit; this includes an exactly cancelling
+// sum, whose FP64 value is 0).
 // The dependent path per step: three FP64 additions and a handful of integer operations
 // that build C from the exponent of s.
 // t + q rounded to posit32, both posit values held in FP64; bit 30 of `bad` is set when
@@ -128,17 +129,9 @@ PG_HD double f64_posit_add(double t, double q, uint32_t &bad)
 {
     const double s = f64_add(t, q);
     const int32_t eb = (int32_t)((f64_bits(s) >> 52) & 0x7FF); // biased binade of s
-    const int32_t k = (eb - 1023) >> 2;                         // regime value
-    const int32_t run = (k ^ (k >> 31)) + 1;                     // regime run; fb = 28 - run
-    const uint32_t hc = ((uint32_t)(eb + 24 + run) << 20) | 0x00080000u; // 1.5 * 2^(e - fb + 52)
-    const double C = f64_from_bits((uint64_t)hc << 32);
+    const double C = f64_from_hi(f64_round_const_hi(eb));
     const double r = f64_add(f64_add(s, C), -C);
-    // off the dependent path: is this step one the FP64 form does exactly?
-    const int32_t et = (int32_t)((f64_bits(t) >> 52) & 0x7FF), eq = (int32_t)((f64_bits(q) >> 52) & 0x7FF);
-    const int32_t gap = et > eq ? et - eq : eq - et;
-    const bool risky = (et != 0) & (eq != 0) & (gap > 24) & (gap <= 30);
-    const bool outside = (uint32_t)(eb - 1023 - FAST_LO) > (uint32_t)(FAST_HI - FAST_LO);
-    bad |= (risky | outside) ? 0x40000000u : 0u;
+    bad |= f64_outside_fast(eb) ? 0x40000000u : 0u;
     return r;
 }
 
@@ -326,8 +319,7 @@ PG_HD double chain_add_one(double t, double q)
 // dependent path.  The fraction width is that of the value a block of steps starts at; it
 // is the same in regimes k and -k-1 (both have a run of the same length), so the scales
 // [2^-4, 2^4) around 1 form one such range of 8 binades, and the other ranges are single
-// regimes.  A step whose sum lands at another fraction width (or is zero, or is risky as in
-// f64_posit_add) is flagged, and the caller redoes the block with chain_add_one.
+// regimes.  A step whose sum lands at another fraction width (or is zero) is flagged, and the caller redoes the block with chain_add_one.
 PG_HD int32_t f64_regime(double x) { return ((int32_t)((f64_bits(x) >> 52) & 0x7FF) - 1023) >> 2; }
 
 // The regime run length of the scale of FP64 pattern sb (fb = 28 - run).
@@ -345,12 +337,7 @@ PG_HD double f64_posit_add_split(double t, double q, double C, int32_t run, uint
     const double s = f64_add(t, q);
     const double g = f64_mul(C, s);
     const double r = f64_add(g, f64_add(s, -g));
-    // off the dependent path
-    const uint64_t sb = f64_bits(s);
-    const int32_t et = (int32_t)((f64_bits(t) >> 52) & 0x7FF), eq = (int32_t)((f64_bits(q) >> 52) & 0x7FF);
-    const int32_t gap = et > eq ? et - eq : eq - et;
-    const bool risky = (eq != 0) & (gap > 24) & (gap <= 30);
-    bad |= (risky | (f64_bits_run(sb) != run)) ? 0x40000000u : 0u;
+    bad |= f64_bits_run(f64_bits(s)) != run ? 0x40000000u : 0u; // off the dependent path
     return r;
 }
 
@@ -397,5 +384,233 @@ PG_HD double chain_add_run_reg(double t, Q q, int count)
         t = chain_add_one(t, q[k]);
     return t;
 }
+
+// ---------------------------------------------------------------------------
+// A warp's chain of additions on the biased running value.
+// ---------------------------------------------------------------------------
+// While t stays in one binade, t = M u with the grid's spacing u = 2^(e - fb) and
+// 2^fb <= |M| < 2^(fb+1).  Hold it as w = C + t, C = sign(t) 1.5 * 2^52 u: w is exact, its
+// spacing as an FP64 number is u, and C/u is even, so the FP64 addition w + q, rounded to
+// nearest even, IS the posit addition: one FP64 addition per step instead of the sum, its
+// exponent, a constant and two more additions.  And |M| is w's low word: the step was inside
+// the binade iff w's high word is C's and the low word in (2^fb, 2^(fb+1)) -- 2^fb itself is
+// given up, since the exact sum may have been below it, where the grid is finer.
+//
+//   runs     8 steps are run, then tested at once; where one left the binade they are done
+//            again by the fixed-width step or, across a change of fraction width, by
+//            f64_posit_add.
+//   windows  512 addends at once, 16 per lane.  A step moves M by an amount that depends on
+//            M's parity alone (ties), so a lane's 16 steps are two displacements, found by
+//            running them from an even and from an odd M; a warp scan composes them
+//            (mod 2^32: past the first step that left the binade nothing is used), and each
+//            lane runs its steps again from its true start, tested at once.  The window
+//            ends where the first lane with a step outside starts.
+//
+// After a cut window the value is near a power of two and often crosses it again soon:
+// runs follow until CHAIN_CALM of them in a row stayed inside.
+//
+// What bounds it: latency.  A dependent FP64 addition takes 8.1 cycles, a run of 8 with its
+// test 98 at best, a window of 512 about 900, a repeated run 500; in a Cholesky solve of
+// order 2048 a row of 1024 addends meets 3.7 windows (2 of them cut), 13 clean runs and 9
+// repeated ones: 13,500 cycles, half of them around the places where the value crosses a
+// power of two several times.  Rpotrs, one right-hand side: n = 1024 10.5 -> 6.5 ms, 4096
+// 92 -> 61, 8192 325 -> 196, against a scan of one step map per addend over four warps with
+// fixed-width steps between its windows.
+#if defined(__CUDACC__)
+constexpr int CHAIN_CALM = 4;        // clean runs before the next window
+constexpr int CHAIN_WINDOW_MIN = 64; // addends left for a window to pay
+
+// A row's addends in shared memory, in groups of 16.  FP64: a group every 18 doubles, so that
+// the lanes of a warp reading a group each spread over the banks.  Patterns (columns too
+// long for that): packed.
+struct ChainTerms64 {
+    double *q;
+    static __host__ __device__ size_t bytes(int n) { return (size_t)((n + 15) / 16) * 18 * sizeof(double); }
+    using Word = double;
+    __device__ static int at(int k) { return k + (k >> 4) * 2; }
+    __device__ void set(int k, double v) const { q[at(k)] = v; }
+    __device__ double get(int k) const { return q[at(k)]; }
+    template <int N> // N addends from k, a multiple of N, N <= 16 a power of two
+    __device__ void load(int k, double (&v)[N]) const
+    {
+        const double2 *p = reinterpret_cast<const double2 *>(q + at(k));
+#pragma unroll
+        for (int j = 0; j < N / 2; ++j) {
+            const double2 x = p[j];
+            v[2 * j] = x.x;
+            v[2 * j + 1] = x.y;
+        }
+    }
+};
+struct ChainTerms32 {
+    uint32_t *q;
+    static __host__ __device__ size_t bytes(int n) { return (size_t)((n + 15) / 16) * 16 * sizeof(uint32_t); }
+    using Word = uint32_t;
+    __device__ void set(int k, double v) const { q[k] = p32_from_double_exact(v); }
+    __device__ double get(int k) const { return p32_to_double(q[k]); }
+    template <int N>
+    __device__ void load(int k, double (&v)[N]) const
+    {
+        const uint4 *p = reinterpret_cast<const uint4 *>(q + k);
+#pragma unroll
+        for (int j = 0; j < N / 4; ++j) {
+            const uint4 x = p[j];
+            v[4 * j] = p32_to_double(x.x);
+            v[4 * j + 1] = p32_to_double(x.y);
+            v[4 * j + 2] = p32_to_double(x.z);
+            v[4 * j + 3] = p32_to_double(x.w);
+        }
+    }
+};
+
+// t + q[pos] + ... + q[end-1], every addition rounded, in that order; t and the q are posit32
+// values, none NaR.  In the groups that hold q[pos] and q[end-1], every other addend is zero
+// (so nothing is masked).  Every lane of a full warp calls it with the same arguments and
+// returns the same value.
+template <class Q>
+__device__ double warp_chain(double t, Q q, int pos, int end)
+{
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    bool calm = true;
+    int clean = 0;
+    pos &= ~7; // from here on a multiple of 8: adding a zero changes nothing
+    while (pos < end) {
+        const uint32_t th = f64_hi(t);
+        const int32_t eb = (int32_t)((th >> 20) & 0x7FF);
+        if (f64_outside_fast(eb)) { // zero among them: no grid to sit on, step by step
+            for (int k = 0; k < 8; ++k)
+                t = f64_round_any(f64_add(t, q.get(pos + k)));
+            pos += 8;
+            continue;
+        }
+        const uint32_t chi = f64_round_const_hi(eb) | (th & 0x80000000u);
+        const double C = f64_from_hi(chi);
+        const int32_t run = (int32_t)((chi >> 20) & 0x7FF) - eb - 24;
+        const uint32_t lim = 1u << (28 - run); // 2^fb
+        double w = f64_add(C, t);
+        for (;;) { // in this binade
+            if (calm && end - pos >= CHAIN_WINDOW_MIN) {
+                const int g0 = pos >> 4, k0 = (g0 + lane) * 16;
+                const int wend = min(end, (g0 + 32) * 16);
+                double v[16];
+                if (k0 < end) {
+                    q.load(k0, v);
+                    if (k0 < pos) { // the group's first half is done
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            v[e] = 0.0;
+                    }
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 16; ++e)
+                        v[e] = 0.0;
+                }
+                // the lane's displacements: of an even M, and by how much an odd one's differs
+                constexpr uint32_t M0 = 1u << 28;
+                double w0 = __hiloint2double((int)chi, (int)M0), w1 = __hiloint2double((int)chi, (int)(M0 + 1));
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    w0 = f64_add(w0, v[e]);
+                    w1 = f64_add(w1, v[e]);
+                }
+                uint32_t c0 = (uint32_t)__double2loint(w0) - M0, d = (uint32_t)__double2loint(w1) - 1 - M0 - c0;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const uint32_t o0 = __shfl_up_sync(FULL, c0, off), od = __shfl_up_sync(FULL, d, off);
+                    // this lane's steps after the earlier ones': M moves by o0 (+ od), then by
+                    // c0, and by d more where M is odd then
+                    const uint32_t p0 = o0 & 1, p1 = (o0 + od + 1) & 1;
+                    const uint32_t n0 = o0 + c0 + p0 * d, nd = od + (p1 - p0) * d;
+                    c0 = lane >= off ? n0 : c0;
+                    d = lane >= off ? nd : d;
+                }
+                uint32_t x0 = __shfl_up_sync(FULL, c0, 1), xd = __shfl_up_sync(FULL, d, 1);
+                if (lane == 0)
+                    x0 = xd = 0;
+                uint32_t M = (uint32_t)__double2loint(w);
+                M += x0 + (M & 1) * xd;
+                double y = __hiloint2double((int)chi, (int)M);
+                uint32_t bad = 0, mn = 0xFFFFFFFFu, mx = 0;
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    y = f64_add(y, v[e]);
+                    const uint32_t lo = (uint32_t)__double2loint(y);
+                    bad |= (uint32_t)__double2hiint(y) ^ chi;
+                    mn = min(mn, lo);
+                    mx = max(mx, lo);
+                }
+                const unsigned bal = __ballot_sync(FULL, bad != 0 || mn <= lim || mx >= 2 * lim);
+                const uint32_t Mend = __shfl_sync(FULL, (uint32_t)__double2loint(y), 31);
+                if (bal == 0) {
+                    w = __hiloint2double((int)chi, (int)Mend);
+                    pos = wend;
+                    if (pos < end)
+                        continue;
+                    return f64_add(w, -C);
+                }
+                const int src = __ffs(bal) - 1;
+                w = __hiloint2double((int)chi, (int)__shfl_sync(FULL, M, src));
+                pos = max(pos, (g0 + src) * 16);
+                calm = false;
+                clean = 0;
+            }
+            // runs of 8
+            double v[8], wb;
+            q.load(pos, v);
+            bool left;
+            for (;;) {
+                wb = w;
+                uint32_t bad = 0, mn = 0xFFFFFFFFu, mx = 0;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    w = f64_add(w, v[e]);
+                    const uint32_t lo = (uint32_t)__double2loint(w);
+                    bad |= (uint32_t)__double2hiint(w) ^ chi;
+                    mn = min(mn, lo);
+                    mx = max(mx, lo);
+                }
+                left = bad != 0 || mn <= lim || mx >= 2 * lim;
+                if (left)
+                    break;
+                pos += 8;
+                if (pos >= end || ++clean >= CHAIN_CALM)
+                    break;
+                q.load(pos, v);
+            }
+            if (!left) {
+                calm = end - pos >= CHAIN_WINDOW_MIN;
+                if (pos < end)
+                    continue;
+                return f64_add(w, -C);
+            }
+            // the run again: the fixed-width step, or f64_posit_add
+            clean = 0;
+            calm = false;
+            const double t0 = f64_add(wb, -C), Cs = f64_split_const(run);
+            uint32_t flag = 0;
+            t = t0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                t = f64_posit_add_split(t, v[e], Cs, run, flag);
+            if (flag & 0x40000000u) {
+                t = t0;
+                flag = 0;
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    t = f64_posit_add(t, v[e], flag);
+                if (flag & 0x40000000u) {
+                    t = t0;
+                    for (int e = 0; e < 8; ++e)
+                        t = f64_round_any(f64_add(t, q.get(pos + e)));
+                }
+            }
+            pos += 8;
+            break;
+        }
+    }
+    return t;
+}
+#endif
 
 } // namespace pg
