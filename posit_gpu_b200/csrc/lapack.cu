@@ -16,7 +16,7 @@
 //                        (Cholesky: square root) step of one CTA, then the scaling of
 //                        the column and the rank-1 update of the rest of the panel over
 //                        all rows in parallel;
-//   U block row          Rtrsm("L","L","N","U") as one CTA per column;
+//   U block row          Rtrsm("L","L","N","U"), a warp or a CTA per column;
 //   row interchanges     Rlaswp on the columns outside the panel;
 //   trailing update      the posit32 GEMM of gemm.cu (NN for LU; NT restricted to the
 //                        lower triangle for Cholesky).
@@ -502,238 +502,259 @@ __global__ void laswp_kernel(uint32_t *__restrict__ A, size_t lda, int ncols, in
     }
 }
 
-// ---------------------------------------------------------------------------
-// Triangular solves with many right-hand sides: one CTA per column of B, one thread per
-// row (strided), the column in shared memory.  Loop orders and zero skips as in
-// Rtrsm.cpp:115-156 (side = L, trans = N).
-// ---------------------------------------------------------------------------
-// lower, unit or non-unit diagonal: forward substitution (Rtrsm.cpp:139-154).  The column
-// is held in shared memory as FP64 (posit32 values are exact there) and every update
-// b_i - b_k*a_ik is the FP64 multiply-add step of the GEMM (posit32.cuh, f64_posit_mac),
-// its rare flagged steps redone on patterns.  NaR travels as NaN (every step that meets
-// it is flagged and redone on patterns, which give NaR).
-PG_HD double trsm_update(double c, double t, double a) { return f64_posit_mac_checked(c, t, a); }
+// The same on a few columns of B, all n interchanges of a solve: one CTA per column, the
+// column and a stretch of ipiv in shared memory, one thread doing the swaps there (about 60
+// cycles each, against an L2 round trip each for laswp_kernel).
+constexpr int LASWP_COL_THREADS = 256;
+constexpr int LASWP_COL_MAX = 48 * 1024; // rows: 4 bytes each, beside the stretch
+constexpr int LASWP_STRETCH = 1024;
 
-// The column: staged in shared memory as FP64, or (too long for that) left in place as
-// patterns and converted at every access.
-template <bool STAGED>
-struct SolveCol {
-    double *s;
-    uint32_t *g;
-    __device__ double get(int i) const { return STAGED ? s[i] : p32_to_double(g[i]); }
-    __device__ void set(int i, double v) const
-    {
-        if (STAGED)
-            s[i] = v;
-        else
-            g[i] = p32_from_double(v);
-    }
-};
-
-template <bool STAGED>
-__global__ void trsm_lln_kernel(const uint32_t *__restrict__ L, size_t ldl, uint32_t *__restrict__ B, size_t ldb,
-                                int m, bool unit, const int *__restrict__ info)
+__global__ void __launch_bounds__(LASWP_COL_THREADS) laswp_col_kernel(uint32_t *__restrict__ B, size_t ldb, int n,
+                                                                      const int *__restrict__ ipiv, bool forward)
 {
-    extern __shared__ double s_x[];
-    if (info && *info < 0)
-        return;
-    uint32_t *bcol = B + (size_t)blockIdx.x * ldb;
-    const SolveCol<STAGED> x{s_x, bcol};
-    if (STAGED)
-        for (int i = threadIdx.x; i < m; i += blockDim.x)
-            s_x[i] = p32_to_double(bcol[i]);
-    __syncthreads();
-    for (int k = 0; k < m; ++k) {
-        double bk = x.get(k);
-        if (bk != 0.0) {
-            if (!unit) {
-                bk = p32_to_double(pdiv_est(p32_from_double(bk), L[k + (size_t)k * ldl]));
-                __syncthreads();
-                if (threadIdx.x == 0)
-                    x.set(k, bk);
-            }
-            const double nb = -bk;
-            const uint32_t *lk = L + (size_t)k * ldl;
-            for (int i = k + 1 + threadIdx.x; i < m; i += blockDim.x)
-                x.set(i, trsm_update(x.get(i), nb, p32_to_double(lk[i])));
-        }
+    extern __shared__ uint32_t s_c[]; // [n]
+    __shared__ int s_p[LASWP_STRETCH];
+    uint32_t *col = B + (size_t)blockIdx.x * ldb;
+    for (int i = threadIdx.x; i < n; i += LASWP_COL_THREADS)
+        s_c[i] = col[i];
+    for (int d0 = 0; d0 < n; d0 += LASWP_STRETCH) {
+        const int cnt = min(LASWP_STRETCH, n - d0);
+        __syncthreads(); // the column is staged; the last stretch is done with
+        for (int d = threadIdx.x; d < cnt; d += LASWP_COL_THREADS)
+            s_p[d] = ipiv[forward ? d0 + d : n - 1 - d0 - d] - 1;
         __syncthreads();
+        if (threadIdx.x == 0)
+            for (int d = 0; d < cnt; ++d) {
+                const int i = forward ? d0 + d : n - 1 - d0 - d, p = s_p[d];
+                const uint32_t x = s_c[i];
+                s_c[i] = s_c[p];
+                s_c[p] = x;
+            }
     }
-    if (STAGED)
-        for (int i = threadIdx.x; i < m; i += blockDim.x)
-            bcol[i] = p32_from_double(s_x[i]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += LASWP_COL_THREADS)
+        col[i] = s_c[i];
 }
 
-// upper, non-unit diagonal: backward substitution (Rtrsm.cpp:121-136), as above
-template <bool STAGED>
-__global__ void trsm_lun_kernel(const uint32_t *__restrict__ U, size_t ldu, uint32_t *__restrict__ B, size_t ldb,
-                                int m, bool unit, const int *__restrict__ info)
+// Rlaswp of a solve's right-hand sides (Rgetrs.cpp:84-114).
+static cudaError_t launch_laswp_rhs(uint32_t *B, int ldb, int nrhs, int n, const int *ipiv, bool forward,
+                                    cudaStream_t st)
 {
-    extern __shared__ double s_x[];
-    if (info && *info < 0)
-        return;
-    uint32_t *bcol = B + (size_t)blockIdx.x * ldb;
-    const SolveCol<STAGED> x{s_x, bcol};
-    if (STAGED)
-        for (int i = threadIdx.x; i < m; i += blockDim.x)
-            s_x[i] = p32_to_double(bcol[i]);
-    __syncthreads();
-    for (int k = m - 1; k >= 0; --k) {
-        double bk = x.get(k);
-        if (bk != 0.0) {
-            if (!unit) {
-                bk = p32_to_double(pdiv_est(p32_from_double(bk), U[k + (size_t)k * ldu]));
-                __syncthreads();
-                if (threadIdx.x == 0)
-                    x.set(k, bk);
-            }
-            const double nb = -bk;
-            const uint32_t *uk = U + (size_t)k * ldu;
-            for (int i = threadIdx.x; i < k; i += blockDim.x)
-                x.set(i, trsm_update(x.get(i), nb, p32_to_double(uk[i])));
+    if (n <= LASWP_COL_MAX) {
+        const size_t bytes = (size_t)n * 4;
+        if (bytes > 40 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(laswp_col_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)bytes);
+            if (e != cudaSuccess)
+                return e;
         }
-        __syncthreads();
+        laswp_col_kernel<<<nrhs, LASWP_COL_THREADS, bytes, st>>>(B, ldb, n, ipiv, forward);
+    } else {
+        laswp_kernel<<<(nrhs + 127) / 128, 128, 0, st>>>(B, ldb, nrhs, 1, n, ipiv, forward ? 1 : -1, nullptr);
     }
-    if (STAGED)
-        for (int i = threadIdx.x; i < m; i += blockDim.x)
-            bcol[i] = p32_from_double(s_x[i]);
+    return cudaGetLastError();
 }
 
-// The same two solves with the column staged in shared memory and each thread's rows of
-// the triangle's next column loaded into registers while the current step runs, so no step
-// waits for memory: rows tid + j*T (j < J) belong to thread tid.  The thread that holds the
-// next step's row divides it by its diagonal right after that row's last update, before the
-// step's barrier, so every thread reads b_k already divided: one division per step instead
-// of one per thread, and one barrier per step.
-template <bool UPPER, int J>
-__global__ void __launch_bounds__(1024) trsm_col_kernel(const uint32_t *__restrict__ A, size_t lda,
-                                                        uint32_t *__restrict__ B, size_t ldb, int m, bool unit,
-                                                        const int *__restrict__ info)
+// ---------------------------------------------------------------------------
+// The axpy-form solves: lower forwards (Rtrsm.cpp:139-154) and upper backwards
+// (Rtrsm.cpp:121-136), side = L, trans = N.
+// ---------------------------------------------------------------------------
+// Each b_i takes its updates b_i - b_k*a_ik in the order of k, then (non-unit) one division;
+// a zero b_k is skipped.  Which other rows are updated when does not matter, so the column
+// is cut into blocks of 32 rows: a warp solves the next block's 32 rows by itself, a lane
+// each, b_k by shuffle, publishes them, and every warp then runs its own rows through those
+// 32 columns.  One thread-block cluster of up to 8 CTAs of 16 warps per right-hand side, the
+// blocks dealt out CTA by CTA, then warp by warp; a published block goes to every CTA's
+// shared memory, double-buffered, with one cluster barrier (one CTA: a block barrier) per
+// block.  The owner of the block after the published one updates that first and solves it
+// while the others update the rest.
+// What bounds it: the chain of one row after the other, about 70 cycles for an update whose
+// multiplier is there and 150 for one whose b_k was the last step's (260 with the division),
+// i.e. 230 (340) cycles per row and no more barriers than blocks.  A column per step of one
+// CTA of 1024 threads, with a barrier each, took 1.9 us per row at n = 4096.  Rgetrs, one
+// right-hand side: n = 1024 1.84 -> 0.79 ms, 4096 15.4 -> 3.1 ms, 8192 48.8 -> 8.4 ms.
+// Updates and solves run in step_one (gemm_tile.cuh): a value outside the fast window or a
+// NaR turns into NaN, is noticed at the end of the block and done again step by step.
+constexpr int COL_BLK = 32;
+constexpr int COL_WARPS = 16;
+constexpr int COL_MAX_CTAS = 8;
+constexpr size_t COL_SMEM_MAX = 227 * 1024 - 1024;
+
+// Shared memory of a CTA: tables, a diagonal block's patterns per warp, the CTA's rows.
+static size_t col_smem_bytes(int nb, int ncta, int warps)
 {
-    extern __shared__ double s_x[];
-    if (info && *info < 0)
+    const int per = (nb + ncta - 1) / ncta;
+    return STEP_TAB_BYTES + (size_t)warps * COL_BLK * COL_BLK * 4 + (size_t)per * COL_BLK * 8;
+}
+
+template <bool UPPER, bool UNIT>
+__global__ void __launch_bounds__(COL_WARPS * 32, 1) trsm_block_kernel(const uint32_t *__restrict__ A, size_t lda,
+                                                                       uint32_t *__restrict__ B, size_t ldb, int m,
+                                                                       const int *__restrict__ info)
+{
+    namespace cgs = cooperative_groups;
+    cgs::cluster_group cluster = cgs::this_cluster();
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    extern __shared__ __align__(128) unsigned char smem_col[];
+    __shared__ double s_sol[2][COL_BLK]; // the published block, by step parity
+    if (info && *info < 0) // written by earlier launches: the same in every CTA
         return;
-    uint32_t *bcol = B + (size_t)blockIdx.x * ldb;
-    const int T = (int)blockDim.x, tid = threadIdx.x;
-    for (int i = tid; i < m; i += T)
-        s_x[i] = p32_to_double(bcol[i]);
-    auto step_col = [&](int st) { return UPPER ? m - 1 - st : st; };
-    uint32_t lc[J], ln[J]; // this thread's rows of the current / next column
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-        const int i = tid + j * T;
-        lc[j] = i < m ? A[i + (size_t)step_col(0) * lda] : 0u;
-    }
-    // b_i / a_ii by the thread holding row i (Rtrsm.cpp:127, 145; b_i = 0 is left alone, as
-    // the reference skips it)
-    auto finish = [&](int i, uint32_t d) {
-        const double v = s_x[i];
-        if (!unit && v != 0.0)
-            s_x[i] = p32_to_double(pdiv_est(p32_from_double_exact(v), d));
+    const int rank = (int)cluster.block_rank(), ncta = (int)cluster.num_blocks();
+    const int nw = (int)blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nb = (m + COL_BLK - 1) / COL_BLK;
+    const unsigned char *tab = smem_col;
+    uint32_t *tile = reinterpret_cast<uint32_t *>(smem_col + STEP_TAB_BYTES) + warp * COL_BLK * COL_BLK;
+    double *s_x = reinterpret_cast<double *>(smem_col + STEP_TAB_BYTES + (size_t)nw * COL_BLK * COL_BLK * 4);
+    uint32_t *bcol = B + (size_t)(blockIdx.x / ncta) * ldb;
+    step_tables_fill(smem_col, threadIdx.x, blockDim.x);
+
+    // block j is this warp's when mine(j); the warp's blocks in the order they are solved
+    auto mine = [&](int j) { return j % ncta == rank && (j / ncta) % nw == warp; };
+    auto block_of = [&](int step) { return UPPER ? nb - 1 - step : step; };
+    const int first = rank + ncta * warp, stride = ncta * nw;
+    const int count = first < nb ? (nb - 1 - first) / stride + 1 : 0;
+    auto own = [&](int s) { return first + stride * (UPPER ? count - 1 - s : s); };
+    auto xrow = [&](int j) -> double & { return s_x[(j / ncta) * COL_BLK + lane]; };
+    auto load_tile = [&](int j) { // the diagonal block: lane's row, all columns
+        const int i = j * COL_BLK + lane;
+        for (int k = 0; k < COL_BLK; ++k) {
+            const int c = j * COL_BLK + k;
+            tile[k * COL_BLK + lane] = (i < m && c < m) ? A[i + (size_t)c * lda] : 0u;
+        }
     };
-    uint32_t dn = unit ? 0u : A[step_col(0) + (size_t)step_col(0) * lda];
-    __syncthreads(); // the column is staged
-    if (tid == step_col(0) % T)
-        finish(step_col(0), dn);
-    __syncthreads();
-    for (int st = 0; st < m; ++st) {
-        const int k = step_col(st), kn = step_col(st + 1);
-        if (st + 1 < m) {
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                const int i = tid + j * T;
-                ln[j] = i < m ? A[i + (size_t)kn * lda] : 0u;
+    // Solves block j (its tile loaded, its updates done) and publishes it into `buf`.
+    auto solve = [&](int j, int buf) {
+        const double x0 = xrow(j);
+        const bool live = j * COL_BLK + lane < m;
+        double x = x0, d = 1.0, rc = 1.0;
+        if (!UNIT && live) {
+            d = p32_to_double(tile[lane * COL_BLK + lane]);
+            rc = 1.0 / d;
+        }
+#pragma unroll 4
+        for (int q = 0; q < COL_BLK; ++q) {
+            const int k = UPPER ? COL_BLK - 1 - q : q;
+            if (!UNIT && lane == k && x != 0.0)
+                x = f64_posit_div(x, d, rc);
+            const double xk = __shfl_sync(FULL, x, k);
+            const double r = step_one(x, -xk, p32_to_double(tile[k * COL_BLK + lane]), tab);
+            if (UPPER ? lane < k : lane > k)
+                x = r;
+        }
+        if (__any_sync(FULL, live && x != x)) { // step by step, as the reference skips and rounds
+            x = x0;
+#pragma unroll 1
+            for (int q = 0; q < COL_BLK; ++q) {
+                const int k = UPPER ? COL_BLK - 1 - q : q;
+                if (!UNIT && lane == k && x != 0.0)
+                    x = f64_posit_div(x, d, rc);
+                const double xk = __shfl_sync(FULL, x, k);
+                if (xk != 0.0 && (UPPER ? lane < k : lane > k))
+                    x = f64_posit_mac_checked(x, -xk, p32_to_double(tile[k * COL_BLK + lane]));
             }
-            if (!unit)
-                dn = A[kn + (size_t)kn * lda];
         }
-        const double bk = s_x[k]; // final: divided by its row's thread at the end of the last step
-        if (bk != 0.0) {          // zero multipliers skipped (Rtrsm.cpp:125-126, 143-144)
-            const double nb = -bk;
+        if (!live)
+            x = 0.0;
+        xrow(j) = x;
+        for (int r = 0; r < ncta; ++r)
+            *cluster.map_shared_rank(&s_sol[buf][lane], r) = x;
+    };
+    // Block j's coefficients of the columns of block c, a row per lane.
+    auto load_coef = [&](int j, int c, uint32_t (&l)[COL_BLK]) {
+        const int i = j * COL_BLK + lane;
+        const uint32_t *p = A + i + (size_t)c * COL_BLK * lda;
 #pragma unroll
-            for (int j = 0; j < J; ++j) {
-                const int i = tid + j * T;
-                if (UPPER ? i < k : (i > k && i < m))
-                    s_x[i] = trsm_update(s_x[i], nb, p32_to_double(lc[j]));
+        for (int k = 0; k < COL_BLK; ++k)
+            l[k] = (i < m && c * COL_BLK + k < m) ? p[(size_t)k * lda] : 0u;
+    };
+    for (int s = 0; s < count; ++s) {
+        const int j = own(s), i = j * COL_BLK + lane;
+        xrow(j) = i < m ? p32_to_double(bcol[i]) : 0.0;
+    }
+    if (count > 0)
+        load_tile(own(0));
+    panel_sync(cluster, ncta); // the tables are filled; every CTA has started
+    int done = 0; // the warp's blocks solved so far
+    if (mine(block_of(0))) {
+        solve(block_of(0), 0);
+        if (++done < count)
+            load_tile(own(done));
+    }
+    for (int step = 0; step + 1 < nb; ++step) {
+        const int c = block_of(step);
+        uint32_t l[COL_BLK];
+        if (done < count)
+            load_coef(own(done), c, l); // in flight across the barrier
+        panel_sync(cluster, ncta); // block c is published
+        const double *sol = s_sol[step & 1];
+        for (int s = done; s < count; ++s) {
+            const int j = own(s);
+            if (s > done)
+                load_coef(j, c, l);
+            const double x0 = xrow(j);
+            double x = x0;
+#pragma unroll
+            for (int q = 0; q < COL_BLK; ++q) {
+                const int k = UPPER ? COL_BLK - 1 - q : q;
+                x = step_one(x, -sol[k], p32_to_double(l[k]), tab);
             }
+            if (x != x) {
+                x = x0;
+                const int i = j * COL_BLK + lane;
+#pragma unroll 1
+                for (int q = 0; q < COL_BLK; ++q) {
+                    const int k = UPPER ? COL_BLK - 1 - q : q;
+                    const double xk = sol[k];
+                    if (xk != 0.0 && i < m)
+                        x = f64_posit_mac_checked(x, -xk, p32_to_double(A[i + (size_t)(c * COL_BLK + k) * lda]));
+                }
+            }
+            xrow(j) = x;
+            __syncwarp();
+            if (s == done && j == block_of(step + 1))
+                solve(j, (step + 1) & 1);
         }
-        // the next step's row has had its last update: its thread divides it now
-        if (st + 1 < m && tid == kn % T)
-            finish(kn, dn);
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < J; ++j)
-            lc[j] = ln[j];
+        if (done < count && own(done) == block_of(step + 1))
+            if (++done < count)
+                load_tile(own(done));
     }
-    for (int i = tid; i < m; i += T)
-        bcol[i] = p32_from_double_exact(s_x[i]);
+    panel_sync(cluster, ncta); // no CTA leaves while another may still write its shared memory
+    for (int s = 0; s < count; ++s) {
+        const int j = own(s), i = j * COL_BLK + lane;
+        if (i < m)
+            bcol[i] = p32_from_double_exact(xrow(j));
+    }
 }
 
-template <bool UPPER>
-static cudaError_t launch_col(int J, int nrhs, int threads, const uint32_t *A, size_t lda, uint32_t *B, size_t ldb,
-                              int m, bool unit, const int *info, cudaStream_t st)
+// One cluster per right-hand side: a CTA per 16 blocks (512 rows), up to 8.
+static cudaError_t launch_col(bool upper, bool unit, int nrhs, const uint32_t *A, size_t lda, uint32_t *B, size_t ldb,
+                              int m, const int *info, cudaStream_t st)
 {
-    const size_t bytes = (size_t)m * sizeof(double);
-    const void *fn = J <= 1 ? (const void *)trsm_col_kernel<UPPER, 1>
-                   : J <= 2 ? (const void *)trsm_col_kernel<UPPER, 2>
-                   : J <= 4 ? (const void *)trsm_col_kernel<UPPER, 4>
-                   : J <= 8 ? (const void *)trsm_col_kernel<UPPER, 8>
-                            : (const void *)trsm_col_kernel<UPPER, 16>;
-    if (bytes > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess)
-            return e;
-    }
-    void *args[] = {(void *)&A, (void *)&lda, (void *)&B, (void *)&ldb, (void *)&m, (void *)&unit, (void *)&info};
-    return cudaLaunchKernel(fn, dim3((unsigned)nrhs), dim3((unsigned)threads), args, bytes, st);
-}
-
-// Forward / backward solve launches: staged when the column fits in shared memory (with
-// the prefetching kernel up to 16 rows per thread).
-static cudaError_t launch_lln(int nrhs, int threads, const uint32_t *L, size_t ldl, uint32_t *B, size_t ldb,
-                              int m, bool unit, const int *info, cudaStream_t st)
-{
-    const size_t bytes = (size_t)m * sizeof(double);
-    const int J = (m + threads - 1) / threads;
-    if (bytes <= 227 * 1024 && J <= 16) {
-        const cudaError_t e = launch_col<false>(J, nrhs, threads, L, ldl, B, ldb, m, unit, info, st);
-        return e != cudaSuccess ? e : cudaGetLastError();
-    }
-    if (bytes <= 227 * 1024) {
-        if (bytes > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(trsm_lln_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)bytes);
-            if (e != cudaSuccess)
-                return e;
-        }
-        trsm_lln_kernel<true><<<nrhs, threads, bytes, st>>>(L, ldl, B, ldb, m, unit, info);
-    } else {
-        trsm_lln_kernel<false><<<nrhs, threads, 0, st>>>(L, ldl, B, ldb, m, unit, info);
-    }
-    return cudaGetLastError();
-}
-
-static cudaError_t launch_lun(int nrhs, int threads, const uint32_t *U, size_t ldu, uint32_t *B, size_t ldb,
-                              int m, bool unit, const int *info, cudaStream_t st)
-{
-    const size_t bytes = (size_t)m * sizeof(double);
-    const int J = (m + threads - 1) / threads;
-    if (bytes <= 227 * 1024 && J <= 16) {
-        const cudaError_t e = launch_col<true>(J, nrhs, threads, U, ldu, B, ldb, m, unit, info, st);
-        return e != cudaSuccess ? e : cudaGetLastError();
-    }
-    if (bytes <= 227 * 1024) {
-        if (bytes > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(trsm_lun_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)bytes);
-            if (e != cudaSuccess)
-                return e;
-        }
-        trsm_lun_kernel<true><<<nrhs, threads, bytes, st>>>(U, ldu, B, ldb, m, unit, info);
-    } else {
-        trsm_lun_kernel<false><<<nrhs, threads, 0, st>>>(U, ldu, B, ldb, m, unit, info);
-    }
-    return cudaGetLastError();
+    const int nb = (m + COL_BLK - 1) / COL_BLK;
+    const int ncta = std::min(COL_MAX_CTAS, (nb + COL_WARPS - 1) / COL_WARPS);
+    auto *fn = upper ? (unit ? trsm_block_kernel<true, true> : trsm_block_kernel<true, false>)
+                     : (unit ? trsm_block_kernel<false, true> : trsm_block_kernel<false, false>);
+    // no more warps than a CTA has blocks (nor, for the longest columns, than fit)
+    int warps = std::min(COL_WARPS, (nb + ncta - 1) / ncta);
+    while (warps > 1 && col_smem_bytes(nb, ncta, warps) > COL_SMEM_MAX)
+        --warps;
+    const size_t smem = col_smem_bytes(nb, ncta, warps);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+        return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nrhs * ncta));
+    cfg.blockDim = dim3((unsigned)(warps * 32));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ncta;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, A, lda, B, ldb, m, info);
 }
 
 // Lower, transposed (Rtrsm.cpp:175-186): one block per right-hand side; the column is
@@ -1330,7 +1351,7 @@ cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb,
                 const int nr = n - j - jb;
                 laswp_kernel<<<(nr + 127) / 128, 128, 0, st>>>(A + (size_t)(j + jb) * L, L, nr, j + 1, j + jb, ipiv,
                                                               1, info);
-                cudaError_t e = launch_lln(nr, 256, P, L, A + j + (size_t)(j + jb) * L, L, jb, true, info, st);
+                cudaError_t e = launch_col(false, true, nr, P, L, A + j + (size_t)(j + jb) * L, L, jb, info, st);
                 if (e != cudaSuccess)
                     return e;
             }
@@ -1490,11 +1511,11 @@ cudaError_t rpotrf_upper_launch(int n, uint32_t *A, int lda, int nb, int *info, 
 cudaError_t rgetrs_launch(int n, int nrhs, const uint32_t *A, int lda, const int *ipiv, uint32_t *B, int ldb,
                           cudaStream_t st)
 {
-    const int threads = 1024;
-    laswp_kernel<<<(nrhs + 127) / 128, 128, 0, st>>>(B, ldb, nrhs, 1, n, ipiv, 1, nullptr);
-    cudaError_t e = launch_lln(nrhs, threads, A, lda, B, ldb, n, true, nullptr, st);
+    cudaError_t e = launch_laswp_rhs(B, ldb, nrhs, n, ipiv, true, st);
     if (e == cudaSuccess)
-        e = launch_lun(nrhs, threads, A, lda, B, ldb, n, false, nullptr, st);
+        e = launch_col(false, true, nrhs, A, lda, B, ldb, n, nullptr, st);
+    if (e == cudaSuccess)
+        e = launch_col(true, false, nrhs, A, lda, B, ldb, n, nullptr, st);
     return e;
 }
 
@@ -1535,8 +1556,7 @@ static cudaError_t launch_ltx(bool upper, bool unit, int n, int nrhs, const uint
 // Rpotrs.cpp:95-106 (uplo = 'L'): L forward, L^T backward.
 cudaError_t rpotrs_lower_launch(int n, int nrhs, const uint32_t *A, int lda, uint32_t *B, int ldb, cudaStream_t st)
 {
-    const int threads = 1024;
-    cudaError_t e = launch_lln(nrhs, threads, A, lda, B, ldb, n, false, nullptr, st);
+    cudaError_t e = launch_col(false, false, nrhs, A, lda, B, ldb, n, nullptr, st);
     if (e != cudaSuccess)
         return e;
     return launch_ltx(false, false, n, nrhs, A, lda, B, ldb, nullptr, st);
@@ -1549,7 +1569,7 @@ cudaError_t rpotrs_upper_launch(int n, int nrhs, const uint32_t *A, int lda, uin
     cudaError_t e = launch_ltx(true, false, n, nrhs, A, lda, B, ldb, nullptr, st);
     if (e != cudaSuccess)
         return e;
-    return launch_lun(nrhs, 1024, A, lda, B, ldb, n, false, nullptr, st);
+    return launch_col(true, false, nrhs, A, lda, B, ldb, n, nullptr, st);
 }
 
 // Rgetrs.cpp:99-113 (trans = 'T' or 'C'): U^T forward (non-unit), L^T backward (unit),
@@ -1563,8 +1583,7 @@ cudaError_t rgetrs_trans_launch(int n, int nrhs, const uint32_t *A, int lda, con
     e = launch_ltx(false, true, n, nrhs, A, lda, B, ldb, nullptr, st);
     if (e != cudaSuccess)
         return e;
-    laswp_kernel<<<(nrhs + 127) / 128, 128, 0, st>>>(B, ldb, nrhs, 1, n, ipiv, -1, nullptr);
-    return cudaGetLastError();
+    return launch_laswp_rhs(B, ldb, nrhs, n, ipiv, false, st);
 }
 
 } // namespace pg
