@@ -92,9 +92,11 @@ struct OutsideTable {
 };
 static __device__ const OutsideTable g_outside_table;
 
-// x rounded as f64_round_outside, x not NaN, by the table.
+// x rounded as f64_round_outside, by the table.
 __device__ __forceinline__ double round_outside_tab(double x)
 {
+    if (x != x)
+        return x;
     const uint64_t b = f64_bits(x) & 0x7FFFFFFFFFFFFFFFull;
     const int ex = (int)(b >> 52) - 1023;
     const int i = ex < 0 ? max(ex + 121, 0) : min(ex - 108 + OutsideTable::NEG, OutsideTable::N - 1);
@@ -215,6 +217,26 @@ template <int UNR_>
 __device__ __forceinline__ int tile_step_count(int left)
 {
     return (min(BK, left) + UNR_ - 1) / UNR_ * UNR_;
+}
+
+// c + t*a and x*y rounded, for any operands: the fast step first, its rare exceptions after
+// it in little code (the panel kernels run a few iterations of long loops: code that does
+// not fit the instruction cache costs them more than it computes).
+__device__ __forceinline__ double mac_any(double c, double t, double a, const unsigned char *tab)
+{
+    double r = step_one(c, t, a, tab);
+    if (r != r) {
+        bool out;
+        r = step_any(c, t, a, tab, out);
+    }
+    return r;
+}
+__device__ __forceinline__ double mul_any(double x, double y, const unsigned char *tab)
+{
+    const double p = f64_mul(x, y);
+    const double C = *reinterpret_cast<const double *>(tab + ((f64_hi(p) >> 17) & 0x3FF8));
+    const double q = f64_add(f64_fma(x, y, C), -C);
+    return q == q ? q : round_outside_tab(p);
 }
 
 // alpha*b_lj as the NN/NT order rounds it (Rgemm.cpp:180, 222), b in FP64; NaN for NaR.

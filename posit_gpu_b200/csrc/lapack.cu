@@ -26,6 +26,7 @@
 #include "lapack.cuh"
 
 #include <algorithm>
+#include <limits.h>
 #include <cooperative_groups.h>
 #include "posit32.cuh"
 #include "trsm_chain.cuh"
@@ -197,34 +198,43 @@ __global__ void __launch_bounds__(PANEL_ROWS) lu_update_kernel(uint32_t *__restr
 // lu_pivot_kernel + lu_update_kernel -- iRamax with first-max tie-break, the interchange
 // across the panel, the scaling decision, the scaled column, the rank-1 update in the FP64
 // step -- in the same per-element order, one launch per panel.  Up to 8 CTAs of T threads
-// (T a multiple of 32, up to 1024).  The panel's rows are dealt out once, row i to CTA
-// i mod ncta, and there to slot r of thread t with i / ncta = r*T + t (R slots per thread,
-// jb FP64 values each, in shared memory); they never move: an interchange of rows k and p
-// swaps the logical row numbers the two slots hold (each thread keeps its slots' numbers in
-// registers, and every thread knows k and p, so each applies the swap to its own slots),
-// and the write-back stores each slot at the row it holds at the end.  Per column, with the
-// cluster's CTAs co-scheduled (no barrier waits for a CTA that never runs):
-//   * each thread's best (key, logical row, value, slot) over its slots holding rows >= k,
-//     reduced over the warp into the warp's slot in shared memory (double-buffered by
-//     column parity); a cluster barrier (a block barrier with one CTA); every warp reduces
-//     all warps' candidates, read through distributed shared memory -- every thread holds
-//     the pivot, the same bits everywhere;
-//   * threads read -u_kc from the pivot row's slot (in any CTA), one thread per CTA forms
-//     the scaling decision and the reciprocal; a block barrier;
-//   * each thread scales and updates its slots holding rows > k.
-// The pivot row's slot is not written again in the panel (but for a zero pivot below row k,
-// where the two slots trade back their column-k values: that column stays in place,
-// Rgetrf2.cpp:107-117), so reading it after the candidates' barrier races with nothing.  A
-// final cluster barrier keeps every CTA's shared memory alive until no other CTA reads it.
+// (T a multiple of 32, up to 1024), each holding a stretch of the panel's rows: row i of it
+// in slot r of thread t, i = r*T + t, jb FP64 values each, in shared memory.  Rows never
+// move: an interchange of rows k and p swaps the logical row numbers the two slots hold
+// (each thread keeps its slots' numbers in registers, and every thread knows k and p, so
+// each applies the swap to its own slots), and the write-back stores each slot at the row
+// it holds at the end.
+//
+// What bounds it: latency, column after column.  So the next pivot is looked for as early as
+// it can be and the bulk of the update runs while it travels.  Per column k:
+//   * wait for the CTAs' candidates of column k, pushed with their reciprocals and whole
+//     rows into every CTA's shared memory; every warp picks the winner (three warp
+//     reductions: the key's two words, the lowest logical row);
+//   * each thread scales its rows' column k and updates column k+1 only; the largest of
+//     column k+1 over the warp, the CTA (one block barrier); the warp that holds the CTA's
+//     candidate brings that one row up to date (a column per lane), forms the reciprocal
+//     (f64_posit_div) and pushes both to all CTAs;
+//   * arrive at the cluster barrier, and only then update columns k+2 .. of all rows.
+// The pushed rows are triple-buffered: a CTA may push column k+1's while another, past its
+// arrival for column k, still reads column k-1's.  The pivot row's slot is not written again
+// in the panel (but for a zero pivot below row k, where the two slots trade back their
+// column-k values: that column stays in place, Rgetrf2.cpp:107-117).  A final cluster barrier
+// keeps every CTA's shared memory alive until no other CTA writes it.
+// At n = 1024 a panel of 24 columns took 103 us when the update of all columns, one multiply-add
+// at a time, came before the search, the pivot row was read from its owner afterwards and
+// the reciprocal by pdiv_est stood in between: 4.2 us a column.  Now 55 us: about 400 cycles
+// to pick the winner, 500 to scale and update one column, 600 to find the CTA's candidate,
+// 500 for its row and reciprocal, 700 until every CTA has it, the update of the rest beside.
+// LU n = 1024: 5.3 -> 3.4 ms, 4096: 51.6 -> 32.7.
 // ---------------------------------------------------------------------------
-constexpr int PANEL1_THREADS = 1024;    // most threads per CTA
+constexpr int PANEL1_THREADS = 1024; // most threads per CTA
 constexpr int PANEL1_MAX_JB = 512;
 constexpr int PANEL1_MAX_CTAS = 8;
-constexpr int PANEL1_SMEM_ENTRIES = 24; // R * jb * T <= 24 * 1024 FP64 values of shared memory per CTA
-constexpr int PANEL1_MAX_R = 4;         // slots per thread (the LU panel keeps their row numbers in registers)
+constexpr int PANEL1_MAX_R = 4;          // slots per thread (the LU panel keeps their row numbers in registers)
 constexpr int PANEL1_ROWS_PER_CTA = 128; // the rows one CTA takes before another joins
+constexpr size_t PANEL1_SMEM = 227 * 1024 - 4096; // dynamic shared memory of a panel CTA
 
-// The barrier of a cluster panel: the cluster's, or the block's when the cluster is one CTA.
+// The barrier of a cluster: the cluster's, or the block's when the cluster is one CTA.
 __device__ __forceinline__ void panel_sync(cooperative_groups::cluster_group &cl, int ncta)
 {
     if (ncta == 1)
@@ -233,160 +243,248 @@ __device__ __forceinline__ void panel_sync(cooperative_groups::cluster_group &cl
         cl.sync();
 }
 
-// Pivot key of an FP64-held posit value: |x|, NaR (NaN) below everything, the order of
-// pabs() on patterns (iRamax.cpp:65-71 compares abs() in posit order).
-__device__ __forceinline__ double pivot_key(double x) { return x != x ? -1.0 : fabs(x); }
-
-// A pivot candidate: the largest key, the first (lowest logical row) among equal keys.
+// A pivot candidate.  The key is |x| as FP64 bits, NaR below everything (iRamax.cpp:65-71
+// compares abs() in posit order); among equal keys the lowest logical row wins.
 struct PivotCand {
-    double key, val;
-    int row;  // logical row, -1: none
-    int slot; // (r << 16) | (CTA rank << 10) | thread of the slot holding it
+    int hi;      // high word of |x|; -1 for NaR, INT_MIN for no candidate
+    uint32_t lo; // low word of |x|
+    int row;     // logical row
+    int slot;    // (r << 16) | thread of the slot holding it
+};
+struct PivotPush {
+    PivotCand c;
+    double val, recip; // the pivot; what the column below it is multiplied by
 };
 
-__device__ __forceinline__ void cand_merge(PivotCand &a, const PivotCand &b)
+__device__ __forceinline__ bool cand_better(const PivotCand &a, const PivotCand &b) // a over b
 {
-    if (b.row >= 0 && (a.row < 0 || b.key > a.key || (b.key == a.key && b.row < a.row)))
-        a = b;
+    return a.hi != b.hi ? a.hi > b.hi : (a.lo != b.lo ? a.lo > b.lo : a.row < b.row);
 }
 
-__device__ __forceinline__ PivotCand cand_shfl_down(const PivotCand &a, int off)
+// The lane holding the warp's best candidate.
+__device__ __forceinline__ int cand_best_lane(const PivotCand &c)
 {
-    PivotCand b;
-    b.key = __shfl_down_sync(0xFFFFFFFFu, a.key, off);
-    b.val = __shfl_down_sync(0xFFFFFFFFu, a.val, off);
-    b.row = __shfl_down_sync(0xFFFFFFFFu, a.row, off);
-    b.slot = __shfl_down_sync(0xFFFFFFFFu, a.slot, off);
-    return b;
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const int hi = __reduce_max_sync(FULL, c.hi);
+    const uint32_t lo = __reduce_max_sync(FULL, c.hi == hi ? c.lo : 0u);
+    const int row = __reduce_min_sync(FULL, c.hi == hi && c.lo == lo ? c.row : INT_MAX);
+    return __ffs(__ballot_sync(FULL, c.hi == hi && c.lo == lo && c.row == row)) - 1;
 }
 
-// Warp-wide best candidate, in lane 0 (and, with `all`, broadcast to every lane).
-__device__ __forceinline__ PivotCand cand_warp_reduce(PivotCand a, bool all)
+// rw[c*T] += -u[c] * l for the columns [c0, jb) of one row, PANEL_U at a time; up to
+// PANEL_U - 1 columns past jb are read and written too (u is zero there).
+constexpr int PANEL_U = 8;
+__host__ __device__ constexpr int panel_cols(int jb) { return jb + PANEL_U - 1; } // columns a row takes in shared memory
+inline size_t lu_panel_smem(int R, int T, int jb, int ncta)
 {
+    return STEP_TAB_BYTES + ((size_t)R * T + 3 * (size_t)ncta) * panel_cols(jb) * sizeof(double);
+}
+
+// The update of one row's columns [c0, jb).
+__device__ __forceinline__ void panel_row_update(double *rw, int T, const double *u, double l, int c0, int jb,
+                                                 const unsigned char *tab)
+{
+#pragma unroll 1
+    for (int c = c0; c < jb; c += PANEL_U) {
+        double y[PANEL_U];
+        double *p = rw + c * T;
+        bool bad = false;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-        cand_merge(a, cand_shfl_down(a, off));
-    if (all) {
-        a.key = __shfl_sync(0xFFFFFFFFu, a.key, 0);
-        a.val = __shfl_sync(0xFFFFFFFFu, a.val, 0);
-        a.row = __shfl_sync(0xFFFFFFFFu, a.row, 0);
-        a.slot = __shfl_sync(0xFFFFFFFFu, a.slot, 0);
+        for (int q = 0; q < PANEL_U; ++q) {
+            y[q] = step_one(p[q * T], -u[c + q], l, tab);
+            bad |= y[q] != y[q];
+        }
+        if (!bad) {
+#pragma unroll
+            for (int q = 0; q < PANEL_U; ++q)
+                p[q * T] = y[q];
+        } else {
+            bool out;
+#pragma unroll 1
+            for (int q = 0; q < PANEL_U; ++q)
+                p[q * T] = step_any(p[q * T], -u[c + q], l, tab, out);
+        }
     }
-    return a;
 }
 
-__global__ void __launch_bounds__(PANEL1_THREADS) lu_panel_cluster_kernel(uint32_t *__restrict__ P, size_t lda,
-                                                                          int M, int jb, int R, int row0,
-                                                                          int *__restrict__ ipiv,
-                                                                          int *__restrict__ info)
+// MAXT: the most threads a CTA of this instance has, MAXR: the most slots of a thread.  One CTA per SM is said to the compiler
+// so that it spends registers on overlapping a row's columns (62 instead of 40: 355 cycles for
+// 8 columns of a warp instead of 511).
+// One row of jb columns from the matrix into shared memory, zeros behind it; eight loads in
+// flight.
+__device__ __forceinline__ void panel_load_row(double *rw, int T, const uint32_t *p, size_t lda, int jb)
+{
+    constexpr int U = 8;
+#pragma unroll 1
+    for (int c = 0; c < panel_cols(jb); c += U) {
+        uint32_t v[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            v[q] = c + q < jb ? p[(size_t)(c + q) * lda] : 0u;
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (c + q < panel_cols(jb))
+                rw[(c + q) * T] = p32_to_double(v[q]);
+    }
+}
+
+template <int MAXT, int MAXR>
+__global__ void __launch_bounds__(MAXT, 1) lu_panel_cluster_kernel(uint32_t *__restrict__ P, size_t lda, int M, int jb,
+                                                                   int R, int row0, int *__restrict__ ipiv,
+                                                                   int *__restrict__ info)
 {
     namespace cgs = cooperative_groups;
     cgs::cluster_group cluster = cgs::this_cluster();
     const int rank = (int)cluster.block_rank(), ncta = (int)cluster.num_blocks();
-    extern __shared__ __align__(16) double s_rows[]; // [R][jb][T]: this CTA's slots, FP64
-    __shared__ PivotCand s_wc[2][32];                // each warp's candidate, by column parity
-    __shared__ double s_u[PANEL1_MAX_JB];            // -u_kc of the current pivot row
-    __shared__ PivotInfo s_pi;
-    __shared__ uint32_t s_tab[F64_CONST_ENTRIES]; // rounding constants (F64ConstTable)
+    extern __shared__ __align__(128) unsigned char smem_panel[];
+    __shared__ PivotCand s_wc[2][32];                  // each warp's candidate, by column parity
+    __shared__ PivotPush s_push[3][PANEL1_MAX_CTAS]; // the CTAs' candidates, by column mod 3
     if (*info < 0) // written only by earlier launches: the same in every CTA
         return;
-    const int T = (int)blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wpc = T >> 5;
-    for (int i = tid; i < F64_CONST_ENTRIES; i += T)
-        s_tab[i] = f64_round_const_top(i);
-    const F64ConstTable cof{s_tab}; // read only after the first barrier below
-    auto own = [&](int r, int c) -> double & { return s_rows[((size_t)r * jb + c) * T + tid]; };
-    int row[PANEL1_MAX_R]; // the logical row each slot holds (-1: none)
+    const int T = (int)blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
+    const unsigned char *tab = smem_panel;
+    double *s_rows = reinterpret_cast<double *>(smem_panel + STEP_TAB_BYTES); // [R][W][T]: this CTA's slots
+    const int W = panel_cols(jb);
+    double *s_cu = s_rows + (size_t)R * W * T; // [3][ncta][W]: the candidates' rows
+    __shared__ int s_piv[PANEL1_MAX_JB];       // the pivots' rows (written out at the end: a global store
+                                               // would hold up the next arrival)
+    step_tables_fill(smem_panel, tid, T);
+    auto slot_row = [&](int r, int t) { return s_rows + r * W * T + t; }; // column c at [c * T]
+    for (int e = tid; e < 3 * ncta * W; e += T)
+        s_cu[e] = 0.0; // past jb it stays
+    const int base = rank * (R * T);
+    int row[MAXR]; // the logical row each slot holds (-1: none)
 #pragma unroll
-    for (int r = 0; r < PANEL1_MAX_R; ++r) {
-        const int i = (r * T + tid) * ncta + rank;
+    for (int r = 0; r < MAXR; ++r) {
+        const int i = base + r * T + tid;
         row[r] = (r < R && i < M) ? i : -1;
         if (row[r] >= 0)
-            for (int c = 0; c < jb; ++c)
-                own(r, c) = p32_to_double(P[i + (size_t)c * lda]);
+            panel_load_row(slot_row(r, tid), T, P + i, lda, jb);
     }
-    const int nslots = ncta * wpc;
-    for (int k = 0; k < jb; ++k) {
-        PivotCand cand = {-2.0, 0.0, -1, 0};
+    panel_sync(cluster, ncta); // the tables are filled; every CTA has started
+
+    PivotCand cand;
+    auto cand_none = [&]() { cand = PivotCand{INT_MIN, 0u, INT_MAX, 0}; };
+    auto cand_add = [&](double v, int r) {
+        const double a = fabs(v);
+        const PivotCand c = {v != v ? -1 : __double2hiint(a), v != v ? 0u : (uint32_t)__double2loint(a), row[r],
+                             (r << 16) | tid};
+        if (cand_better(c, cand))
+            cand = c;
+    };
+    // The CTA's candidate of column c into every CTA; `u` and the rows' column c-1 bring its
+    // row up to date (c > 0).  Then the arrival for column c.
+    auto publish = [&](int c, const double *u) {
+        const int bl = cand_best_lane(cand);
+        if (lane == bl)
+            s_wc[c & 1][warp] = cand;
+        __syncthreads();
+        PivotCand best = lane < nw ? s_wc[c & 1][lane] : PivotCand{INT_MIN, 0u, INT_MAX, 0};
+        const int bw = cand_best_lane(best);
+        if (warp == bw) {
+            best = s_wc[c & 1][bw];
+            const double *rw = slot_row(best.slot >> 16, best.slot & 0xFFFF);
+            double v = 0.0;
+            if (best.hi != INT_MIN) {
+                const double l = c > 0 ? rw[(c - 1) * T] : 0.0;
+                v = rw[c * T];
+                for (int q = c + lane; q < jb; q += 32) {
+                    double x = rw[q * T];
+                    if (c > 0 && q > c)
+                        x = mac_any(x, -u[q], l, tab);
+                    double *to = s_cu + ((c % 3) * ncta + rank) * W + q;
+                    for (int r = 0; r < ncta; ++r)
+                        *cluster.map_shared_rank(to, r) = x;
+                }
+            }
+            // 1/pivot (Rgetrf2.cpp:119-131: |pivot| >= sfmin = FLT_MIN, minpos as a posit, holds for
+            // all but zero and NaR; a NaR pivot divides every element, which gives NaR as
+            // multiplying by NaR does; a zero one scales nothing)
+            const double recip = v == 0.0 ? 1.0 : f64_posit_div(1.0, v, 1.0 / v);
+            if (lane < ncta) {
+                PivotPush *to = cluster.map_shared_rank(&s_push[c % 3][rank], lane);
+                to->c = best;
+                to->val = v;
+                to->recip = recip;
+            }
+        }
+        __syncwarp();
+        if (ncta > 1)
+            cgs::this_cluster().barrier_arrive();
+    };
+    cand_none();
 #pragma unroll
-        for (int r = 0; r < PANEL1_MAX_R; ++r)
-            if (row[r] >= k) {
-                const double v = own(r, k);
-                cand_merge(cand, PivotCand{pivot_key(v), v, row[r], (r << 16) | (rank << 10) | tid});
-            }
-        cand = cand_warp_reduce(cand, false);
-        if (lane == 0)
-            s_wc[k & 1][warp] = cand;
-        panel_sync(cluster, ncta); // the warps' candidates, cluster-wide
-        cand = PivotCand{-2.0, 0.0, -1, 0};
-        for (int s = lane; s < nslots; s += 32)
-            cand_merge(cand, *cluster.map_shared_rank(&s_wc[k & 1][s % wpc], s / wpc));
-        cand = cand_warp_reduce(cand, true);
-        const int p = cand.row;
-        const uint32_t piv = p32_from_double_exact(cand.val);
-        // u from the pivot row's slot (after the interchange it is row k)
-        const int sr = cand.slot >> 16, sq = (cand.slot >> 10) & 63, st = cand.slot & 1023;
-        double *src = cluster.map_shared_rank(s_rows, sq) + (size_t)sr * jb * T + st;
-        for (int c = k + 1 + tid; c < jb; c += T)
-            s_u[c] = -src[(size_t)c * T];
-        if (tid == T - 1) {
-            PivotInfo pi;
-            pi.row = p;
-            pi.piv = piv;
-            if (piv == 0) {
-                pi.mode = 0;
-                pi.recip = 0;
-                if (rank == 0 && *info == 0)
-                    *info = row0 + k + 1;
-            } else if ((int32_t)pabs(piv) >= (int32_t)1u) { // |pivot| >= sfmin = FLT_MIN -> minpos
-                pi.mode = 1;
-                pi.recip = pdiv_est(P32_ONE, piv);
-            } else {
-                pi.mode = 2; // NaR pivot: element-wise division (Rgetrf2.cpp:124-126)
-                pi.recip = 0;
-            }
-            if (rank == 0)
-                ipiv[row0 + k] = row0 + p + 1; // 1-based, global
-            s_pi = pi;
+    for (int r = 0; r < MAXR; ++r)
+        if (row[r] >= 0)
+            cand_add(slot_row(r, tid)[0], r);
+    publish(0, nullptr);
+    for (int k = 0; k < jb; ++k) {
+        if (ncta > 1)
+            cgs::this_cluster().barrier_wait();
+        else
+            __syncthreads();
+        const PivotCand mine = lane < ncta ? s_push[k % 3][lane].c : PivotCand{INT_MIN, 0u, INT_MAX, 0};
+        const int win = cand_best_lane(mine);
+        const PivotPush pv = s_push[k % 3][win];
+        const double *u = s_cu + ((k % 3) * ncta + win) * W; // the pivot row, columns k ..
+        const int p = pv.c.row;
+        if (rank == 0 && tid == 0) {
+            s_piv[k] = row0 + p + 1; // 1-based, global
+            if (pv.val == 0.0 && *info == 0)
+                *info = row0 + k + 1;
         }
         if (p != k) {
-            if (piv == 0) {
+            if (pv.val == 0.0) {
                 // A zero pivot leaves its own column in place (Rgetrf2.cpp:107-117) while the
                 // recursion's Rlaswp calls move rows k and p in every other column: the two
-                // slots trade their column-k values back.  Only row k's holder touches them
-                // (the pivot's slot is read above at columns > k only).
+                // slots trade their column-k values back, by row k's holder.
+                double *src = cluster.map_shared_rank(s_rows, win) + (pv.c.slot >> 16) * W * T + (pv.c.slot & 0xFFFF);
 #pragma unroll
-                for (int r = 0; r < PANEL1_MAX_R; ++r)
+                for (int r = 0; r < MAXR; ++r)
                     if (row[r] == k) {
-                        src[(size_t)k * T] = own(r, k);
-                        own(r, k) = cand.val;
+                        src[k * T] = slot_row(r, tid)[k * T];
+                        slot_row(r, tid)[k * T] = pv.val;
                     }
             }
 #pragma unroll
-            for (int r = 0; r < PANEL1_MAX_R; ++r)
+            for (int r = 0; r < MAXR; ++r)
                 row[r] = row[r] == k ? p : (row[r] == p ? k : row[r]);
         }
-        __syncthreads(); // u and the scaling decision
-        const PivotInfo pi = s_pi;
-        const double drecip = p32_to_double(pi.recip);
+        const bool more = k + 1 < jb;
+        const double un = more ? -u[k + 1] : 0.0;
+        cand_none();
 #pragma unroll
-        for (int r = 0; r < PANEL1_MAX_R; ++r) {
+        for (int r = 0; r < MAXR; ++r)
             if (row[r] > k) {
-                double *rw = &own(r, 0);
-                // Rscal (x*recip, the FP64 product step) or the element-wise division
-                const double dl = pi.mode == 1 ? f64_posit_mul_checked(rw[(size_t)k * T], drecip, cof)
-                                               : p32_to_double(lu_scaled(p32_from_double_exact(rw[(size_t)k * T]), pi));
-                rw[(size_t)k * T] = dl;
-                for (int c = k + 1; c < jb; ++c) // a_ic + (-u_kc)*l_i in the FP64 step
-                    rw[(size_t)c * T] = f64_posit_mac_checked(rw[(size_t)c * T], s_u[c], dl, cof);
+                double *rw = slot_row(r, tid);
+                const double l = mul_any(rw[k * T], pv.recip, tab); // Rscal
+                rw[k * T] = l;
+                if (more) {
+                    const double x = mac_any(rw[(k + 1) * T], un, l, tab);
+                    rw[(k + 1) * T] = x;
+                    cand_add(x, r);
+                }
             }
+        if (more) {
+            publish(k + 1, u);
+            __syncwarp(); // the candidate's row has been read
         }
-    }
-    panel_sync(cluster, ncta); // no CTA leaves while another may still read its shared memory
 #pragma unroll
-    for (int r = 0; r < PANEL1_MAX_R; ++r)
+        for (int r = 0; r < MAXR; ++r)
+            if (row[r] > k) {
+                double *rw = slot_row(r, tid);
+                panel_row_update(rw, T, u, rw[k * T], k + 2, jb, tab);
+            }
+    }
+    panel_sync(cluster, ncta); // no CTA leaves while another may still write its shared memory
+    if (rank == 0)
+        for (int c = tid; c < jb; c += T)
+            ipiv[row0 + c] = s_piv[c];
+#pragma unroll
+    for (int r = 0; r < MAXR; ++r)
         if (row[r] >= 0)
             for (int c = 0; c < jb; ++c)
-                P[row[r] + (size_t)c * lda] = p32_from_double_exact(own(r, c));
+                P[row[r] + (size_t)c * lda] = p32_from_double_exact(slot_row(r, tid)[c * T]);
 }
 
 // After a panel of columns [j, j+jb) (jb <= ROWS_JB_MAX): the panel's row interchanges
@@ -1025,100 +1123,139 @@ __global__ void __launch_bounds__(PANEL_ROWS) chol_update_kernel(uint32_t *__res
     }
 }
 
-// Lower Cholesky panel in one thread-block cluster, held in shared memory (rows dealt out
-// as in lu_panel_cluster_kernel; here they never change places), the counterpart of
-// chol_diag_kernel + chol_update_kernel.  The thread holding row k forms l_kk and 1/l_kk
-// (Rpotrf2.cpp:90-97) right after its own update of column k-1 and writes the decision and
-// 1/l_kk into every CTA.  Per column: a cluster barrier (A); every thread scales its rows
-// below the diagonal (Rtrsm.cpp:265-268), the holders of the diagonal block's rows also
-// writing their -l_ck into every CTA; a cluster barrier (B); each thread updates its rows.
-// With one CTA the barriers are the block's.  A failed diagonal (info) ends the loop in
-// every CTA at the same column; the rows are written back either way.
-__global__ void __launch_bounds__(PANEL1_THREADS) chol_panel_cluster_kernel(uint32_t *__restrict__ P, size_t lda,
-                                                                            int M, int jb, int R, int row0,
-                                                                            int *__restrict__ info)
+// Lower Cholesky panel of up to 32 columns in one launch, the counterpart of chol_diag_kernel
+// + chol_update_kernel.  Below the diagonal block every row goes its own way once the block is
+// factored, so each CTA of 128 threads factors the block for itself, in shared memory, and
+// then takes 128 rows through it, one per thread: l_ik = (1/l_kk)*a_ik (Rtrsm.cpp:265-268),
+// a_ic += (-l_ck)*l_ik for c > k, in the FP64 step.  No CTA waits for another.
+// The block's factor: per column every warp forms l_kk (Rpotrf2.cpp:90-97) and 1/l_kk and
+// scales the column for itself, a row per lane, and updates every fourth of the columns right
+// of it; one block barrier.  A failed diagonal (a_kk <= 0, NaR included) stops with info after
+// the columns before it, in the rows below too.
+// Other CTAs still read the block when the first one is done, so its factor goes to `out`
+// and the next panel's launch (the next to touch the matrix there) puts it in place; the last
+// panel has one CTA and writes it itself.
+// What bounds it: the block's chain, about 850 cycles a column (root, reciprocal, scaling,
+// update, one after the other), then 15,000 for 32 columns of a row.  The cluster form this
+// replaced took two cluster barriers and one update at a time per column: Cholesky n = 1024
+// 3.9 -> 2.5 ms, 4096 27.6 -> 19.2.
+constexpr int CHOL_JB_MAX = 32;
+constexpr int CHOL_T = 128;
+constexpr int CHOL_LD = CHOL_JB_MAX + 1;
+constexpr size_t CHOL_BLOCKS_BYTES = 2 * CHOL_JB_MAX * CHOL_JB_MAX * 4; // two panels' blocks in the workspace
+
+static size_t chol_panel_smem(int jb)
 {
-    namespace cgs = cooperative_groups;
-    cgs::cluster_group cluster = cgs::this_cluster();
-    const int rank = (int)cluster.block_rank(), ncta = (int)cluster.num_blocks();
-    extern __shared__ __align__(16) double s_rows[]; // [R][jb][T]: this CTA's rows, FP64
-    __shared__ double s_l[PANEL1_MAX_JB];           // -l_ck of the current column
-    __shared__ uint32_t s_recip;                    // 1/l_kk
-    __shared__ int s_stop;                          // a_kk <= 0 or NaR
-    __shared__ uint32_t s_tab[F64_CONST_ENTRIES];   // rounding constants (F64ConstTable)
-    if (*info != 0) // written only by earlier launches: the same in every CTA
+    return STEP_TAB_BYTES + ((size_t)CHOL_JB_MAX * CHOL_LD + PANEL_U + CHOL_JB_MAX + (size_t)panel_cols(jb) * CHOL_T) * sizeof(double);
+}
+
+__global__ void __launch_bounds__(CHOL_T, 1) chol_panel_kernel(uint32_t *__restrict__ P, size_t lda, int M, int jb,
+                                                            int row0, int *__restrict__ info,
+                                                            uint32_t *__restrict__ out, uint32_t *__restrict__ prev,
+                                                            int prev_jb, const uint32_t *__restrict__ in)
+{
+    extern __shared__ __align__(128) unsigned char smem_chol[];
+    const unsigned char *tab = smem_chol;
+    double *s_d = reinterpret_cast<double *>(smem_chol + STEP_TAB_BYTES); // the block: a_ic at [c * CHOL_LD + i]
+    double *s_r = s_d + CHOL_JB_MAX * CHOL_LD + PANEL_U;                  // 1/l_kk
+    double *s_rows = s_r + CHOL_JB_MAX;                                   // [panel_cols(jb)][CHOL_T]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // info within this panel is this launch's own, by the first CTA
+    const int seen = *info;
+    if (blockIdx.x == 0 && prev_jb > 0 && (seen == 0 || seen > row0 - prev_jb))
+        for (int e = tid; e < prev_jb * prev_jb; e += CHOL_T) {
+            const int i = e % prev_jb, c = e / prev_jb;
+            if (i >= c)
+                prev[i + (size_t)c * lda] = in[e];
+        }
+    if (seen != 0 && seen <= row0)
         return;
-    const int T = (int)blockDim.x, tid = threadIdx.x;
-    for (int i = tid; i < F64_CONST_ENTRIES; i += T)
-        s_tab[i] = f64_round_const_top(i);
-    const F64ConstTable cof{s_tab}; // read only after the first barrier below
-    auto own = [&](int r, int c) -> double & { return s_rows[((size_t)r * jb + c) * T + tid]; };
-    auto row_of = [&](int r) { return (r * T + tid) * ncta + rank; };
-    for (int r = 0; r < R; ++r) {
-        const int i = row_of(r);
-        if (i < M)
-            for (int c = 0; c < jb; ++c)
-                own(r, c) = p32_to_double(P[i + (size_t)c * lda]);
+    step_tables_fill(smem_chol, tid, CHOL_T);
+    for (int e = tid; e < CHOL_JB_MAX * CHOL_LD + PANEL_U; e += CHOL_T)
+        s_d[e] = 0.0; // past a column's end it stays, or meets a column past jb
+    __syncthreads();
+    for (int e = tid; e < jb * jb; e += CHOL_T) {
+        const int i = e % jb, c = e / jb;
+        if (i >= c)
+            s_d[c * CHOL_LD + i] = p32_to_double(P[i + (size_t)c * lda]);
     }
-    // From the holder of row k: l_kk in place, the decision and 1/l_kk into every CTA.
-    auto diag = [&](int r, int k) {
-        const uint32_t akk = p32_from_double_exact(own(r, k));
-        const int stop = (int32_t)akk <= 0; // NaR included (Rpotrf2.cpp:90-93)
-        uint32_t recip = 0;
-        if (!stop) {
-            const uint32_t lkk = psqrt_est(akk);
-            own(r, k) = p32_to_double(lkk);
-            recip = pdiv_est(P32_ONE, lkk);
-        }
-        for (int q = 0; q < ncta; ++q) {
-            *cluster.map_shared_rank(&s_stop, q) = stop;
-            *cluster.map_shared_rank(&s_recip, q) = recip;
-        }
-    };
-    panel_sync(cluster, ncta); // every CTA has started: distributed shared memory may be written
-    for (int r = 0; r < R; ++r)
-        if (row_of(r) == 0)
-            diag(r, 0);
+    const int i = jb + blockIdx.x * CHOL_T + tid; // this thread's row
+    if (i < M)
+        panel_load_row(s_rows + tid, CHOL_T, P + i, lda, jb);
+    __syncthreads();
+    int stop = jb; // the first column whose diagonal fails
     for (int k = 0; k < jb; ++k) {
-        panel_sync(cluster, ncta); // A: the decision and 1/l_kk; every read of the last column's -l_ck done
-        if (s_stop) { // the same in every CTA
-            // written only here, after every CTA has passed its entry check of *info
-            if (rank == 0 && tid == 0)
-                *info = row0 + k + 1;
+        const double *dk = s_d + k * CHOL_LD;
+        const double akk = dk[k];
+        if (!(akk > 0.0)) { // the same in every thread
+            stop = k;
             break;
         }
-        const double drecip = p32_to_double(s_recip);
-        for (int r = 0; r < R; ++r) {
-            const int i = row_of(r);
-            if (i > k && i < M) { // (1/l_kk)*a_ik, the FP64 product step
-                const double l = f64_posit_mul_checked(own(r, k), drecip, cof);
-                own(r, k) = l;
-                if (i < jb)
-                    for (int q = 0; q < ncta; ++q)
-                        *cluster.map_shared_rank(&s_l[i], q) = -l;
+        const double lkk = f64_posit_sqrt(akk);
+        const double recip = f64_posit_div(1.0, lkk, 1.0 / lkk);
+        double l = 0.0;
+        if (lane > k && lane < jb)
+            l = mul_any(dk[lane], recip, tab);
+        // columns k+1+warp, +4, ...: rows lane >= column; l_ck is lane c's l
+        for (int c0 = k + 1 + warp; c0 < jb; c0 += 16) {
+            double y[4];
+            bool bad = false;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int c = c0 + 4 * q;
+                const double t = -__shfl_sync(0xFFFFFFFFu, l, c & 31);
+                const bool in_block = c < jb && lane >= c && lane < jb;
+                const double x = in_block ? s_d[c * CHOL_LD + lane] : 0.0;
+                y[q] = step_one(x, t, l, tab);
+                bad |= in_block && y[q] != y[q];
+            }
+            if (__any_sync(0xFFFFFFFFu, bad)) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int c = c0 + 4 * q;
+                    const double t = -__shfl_sync(0xFFFFFFFFu, l, c & 31);
+                    if (c < jb && lane >= c && lane < jb)
+                        y[q] = mac_any(s_d[c * CHOL_LD + lane], t, l, tab);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int c = c0 + 4 * q;
+                if (c < jb && lane >= c && lane < jb)
+                    s_d[c * CHOL_LD + lane] = y[q];
             }
         }
-        panel_sync(cluster, ncta); // B: the column's -l_ck in every CTA
-        for (int r = 0; r < R; ++r) {
-            const int i = row_of(r);
-            if (i > k && i < M) {
-                double *rw = &own(r, 0);
-                const double dl = rw[(size_t)k * T];
-                const int cend = min(jb - 1, i);
-                for (int c = k + 1; c <= cend; ++c) // a_ic + (-l_ck)*l_i in the FP64 step
-                    rw[(size_t)c * T] = f64_posit_mac_checked(rw[(size_t)c * T], s_l[c], dl, cof);
-                if (i == k + 1 && i < jb) // the next diagonal, from its holder's own update
-                    diag(r, k + 1);
+        __syncthreads(); // column k has been read, the columns right of it are up to date
+        if (warp == (k & 3) && lane >= k && lane < jb)
+            s_d[k * CHOL_LD + lane] = lane == k ? lkk : l;
+        if (tid == 0)
+            s_r[k] = recip;
+    }
+    __syncthreads();
+    if (blockIdx.x == 0) {
+        if (stop < jb && tid == 0)
+            *info = row0 + stop + 1;
+        for (int e = tid; e < jb * jb; e += CHOL_T) {
+            const int r = e % jb, c = e / jb;
+            if (r >= c) {
+                const uint32_t v = p32_from_double_exact(s_d[c * CHOL_LD + r]);
+                if (out)
+                    out[e] = v;
+                else
+                    P[r + (size_t)c * lda] = v;
             }
         }
     }
-    panel_sync(cluster, ncta); // no CTA leaves while another may still write its shared memory
-    for (int r = 0; r < R; ++r) {
-        const int i = row_of(r);
-        if (i < M)
-            for (int c = 0; c < jb; ++c)
-                P[i + (size_t)c * lda] = p32_from_double_exact(own(r, c));
+    if (i >= M)
+        return;
+    double *rw = s_rows + tid;
+    for (int k = 0; k < stop; ++k) {
+        const double l = mul_any(rw[k * CHOL_T], s_r[k], tab);
+        rw[k * CHOL_T] = l;
+        panel_row_update(rw, CHOL_T, s_d + k * CHOL_LD, l, k + 1, jb, tab);
     }
+    for (int c = 0; c < jb; ++c)
+        P[i + (size_t)c * lda] = p32_from_double_exact(rw[c * CHOL_T]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1264,8 +1401,7 @@ size_t rgetrf_workspace_bytes(int m, int n, int nb)
 
 // The panel form: the cluster panel held in shared memory when its rows fit (ncta CTAs,
 // one per PANEL1_ROWS_PER_CTA rows up to 8, T threads each -- the CTA's rows rounded up to
-// whole warps, at most 1024 -- R slots per thread, R * jb * T FP64 values of shared memory
-// at most 24 * 1024), else the two-launch form (ncta = 0).
+// whole warps, at most 1024 -- R slots per thread), else the two-launch form (ncta = 0).
 struct PanelForm {
     int ncta, R, T; // CTAs (0: the panel does not fit), slots per thread, threads per CTA
 };
@@ -1277,17 +1413,16 @@ static PanelForm panel_form(int M, int jb, int max_ctas)
     const int ncta = std::max(1, std::min(cap, (M + PANEL1_ROWS_PER_CTA - 1) / PANEL1_ROWS_PER_CTA));
     const int rpc = (M + ncta - 1) / ncta; // rows per CTA
     const int T = std::min(PANEL1_THREADS, (rpc + 31) / 32 * 32), R = (rpc + T - 1) / T;
-    if ((size_t)R * jb * T > (size_t)PANEL1_SMEM_ENTRIES * PANEL1_THREADS || R > PANEL1_MAX_R)
+    if (lu_panel_smem(R, T, jb, ncta) > PANEL1_SMEM || R > PANEL1_MAX_R)
         return {0, 0, 0};
     return {ncta, R, T};
 }
 
 template <class... Args>
-static cudaError_t launch_panel_cluster(void (*kernel)(Args...), PanelForm f, int jb, cudaStream_t st, Args... args)
+static cudaError_t launch_panel_cluster(void (*kernel)(Args...), PanelForm f, size_t smem, cudaStream_t st,
+                                        Args... args)
 {
-    const size_t smem = (size_t)f.R * jb * f.T * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         PANEL1_SMEM_ENTRIES * PANEL1_THREADS * (int)sizeof(double));
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL1_SMEM);
     if (e != cudaSuccess)
         return e;
     cudaLaunchConfig_t cfg = {};
@@ -1330,7 +1465,12 @@ cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb,
         uint32_t *lc = lcol + j; // indexed by panel-local row
         const PanelForm pf = panel_form(M, jb, max_ctas);
         if (pf.ncta > 0) {
-            cudaError_t e = launch_panel_cluster(lu_panel_cluster_kernel, pf, jb, st, P, L, M, jb, pf.R, j, ipiv, info);
+            cudaError_t e = launch_panel_cluster(pf.R > 1      ? lu_panel_cluster_kernel<PANEL1_THREADS, PANEL1_MAX_R>
+                                                 : pf.T <= 128 ? lu_panel_cluster_kernel<128, 1>
+                                                 : pf.T <= 512 ? lu_panel_cluster_kernel<512, 1>
+                                                               : lu_panel_cluster_kernel<PANEL1_THREADS, 1>,
+                                                 pf, lu_panel_smem(pf.R, pf.T, jb, pf.ncta),
+                                                 st, P, L, M, jb, pf.R, j, ipiv, info);
             if (e != cudaSuccess)
                 return e;
         } else {
@@ -1377,29 +1517,36 @@ size_t rpotrf_workspace_bytes(int n, int nb)
     if (nb < 1)
         nb = 1;
     int jb = imin(nb, n);
-    return panel_ws_bytes(n) + (n > jb ? gemm_workspace_bytes(n - jb, n - jb, jb) : 0);
+    return panel_ws_bytes(n) + CHOL_BLOCKS_BYTES + (n > jb ? gemm_workspace_bytes(n - jb, n - jb, jb) : 0);
 }
 
 // Lower Cholesky (Rpotrf.cpp:124-142 / Rpotrf2.cpp:132-146 order, blocked right-looking).
-cudaError_t rpotrf_lower_launch(int n, uint32_t *A, int lda, int nb, int *info, void *ws, cudaStream_t st,
-                                int max_ctas)
+cudaError_t rpotrf_lower_launch(int n, uint32_t *A, int lda, int nb, int *info, void *ws, cudaStream_t st)
 {
     if (nb < 1)
         nb = 1;
     CholSync *sync = reinterpret_cast<CholSync *>(ws);
+    uint32_t *blocks = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(ws) + panel_ws_bytes(n));
     uint32_t *lcol = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(ws) + 256);
-    void *gws = reinterpret_cast<unsigned char *>(ws) + panel_ws_bytes(n);
+    void *gws = reinterpret_cast<unsigned char *>(ws) + panel_ws_bytes(n) + CHOL_BLOCKS_BYTES;
     const size_t L = (size_t)lda;
     for (int j = 0; j < n; j += nb) {
         const int jb = imin(n - j, nb);
         const int M = n - j;
         uint32_t *P = A + j + (size_t)j * L;
         uint32_t *lc = lcol + j;
-        const PanelForm pf = panel_form(M, jb, max_ctas);
-        if (pf.ncta > 0) {
-            cudaError_t e = launch_panel_cluster(chol_panel_cluster_kernel, pf, jb, st, P, L, M, jb, pf.R, j, info);
+        if (jb <= CHOL_JB_MAX) {
+            const bool last = j + jb >= n;
+            const size_t smem = chol_panel_smem(jb);
+            cudaError_t e = cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)chol_panel_smem(CHOL_JB_MAX));
             if (e != cudaSuccess)
                 return e;
+            const int prev_jb = j > 0 ? nb : 0; // nb <= CHOL_JB_MAX for every panel but a lone first one
+            chol_panel_kernel<<<imax(1, (M - jb + CHOL_T - 1) / CHOL_T), CHOL_T, smem, st>>>(
+                P, L, M, jb, j, info, last ? nullptr : blocks + (j / nb & 1) * CHOL_JB_MAX * CHOL_JB_MAX,
+                nb <= CHOL_JB_MAX && j > 0 ? P - (size_t)nb * (L + 1) : nullptr, nb <= CHOL_JB_MAX ? prev_jb : 0,
+                blocks + (j / nb + 1 & 1) * CHOL_JB_MAX * CHOL_JB_MAX);
         } else {
             chol_diag_kernel<<<1, 256, 0, st>>>(P, L, M, jb, 0, j, info, sync, lc, -1);
             for (int k = 0; k < jb; ++k) {

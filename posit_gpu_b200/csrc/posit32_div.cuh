@@ -104,4 +104,20 @@ PG_HD double f64_posit_div(double t, double a, double rc)
     return p32_to_double(pdiv_est(p32_from_double_exact(t), p32_from_double_exact(a)));
 }
 
+// sqrt(a) rounded, a > 0 a posit32 value in FP64: the correctly rounded FP64 root onto the
+// posit grid, or the integer root where it is too near half way between two posits to tell
+// or outside the fast window.
+PG_HD double f64_posit_sqrt(double a)
+{
+    const double q = sqrt(a);
+    const uint32_t ch = f64_round_const_top(f64_hi(q) >> 20);
+    const double C = f64_from_hi(ch);
+    const double z = f64_add(f64_add(q, C), -C);
+    const double half = f64_from_hi((ch & 0x7FF00000u) - (53u << 20)); // half the grid's spacing
+    const double off = fabs(f64_add(fabs(f64_add(q, -z)), -half));
+    if (off > f64_mul(q, 8.8817841970012523e-16 /* 2^-50 */))
+        return z;
+    return p32_to_double(psqrt_est(p32_from_double_exact(a)));
+}
+
 } // namespace pg

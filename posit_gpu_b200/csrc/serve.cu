@@ -383,8 +383,7 @@ int launch_blocked(posit_server *s, Unit *u)
         cudaError_t e = r.q.kind == POSIT_BATCH_LU
                             ? pg::rgetrf_launch(n, n, f->dA, n, f->dipiv, serve_nb(s, r.q.kind, n), f->dinfo, ws, st,
                                                 SERVE_PANEL_CTAS)
-                            : pg::rpotrf_lower_launch(n, f->dA, n, serve_nb(s, r.q.kind, n), f->dinfo, ws, st,
-                                                      SERVE_PANEL_CTAS);
+                            : pg::rpotrf_lower_launch(n, f->dA, n, serve_nb(s, r.q.kind, n), f->dinfo, ws, st);
         cudaFreeAsync(ws, st);
         if (e != cudaSuccess)
             return fail_code(e);
