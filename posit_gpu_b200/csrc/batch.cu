@@ -2,339 +2,812 @@
 // persistent launch fed by a device work queue.
 //
 // Each CTA takes the next problem from the queue (an atomic counter over a list sorted by
-// decreasing size, so the largest problems start first) and factors and solves it alone:
-// right-looking, one column per step, the matrix and right-hand sides in global memory
-// (L2-resident for the sizes batched here).  Per-element operation order is the
-// reference's (see lapack.cu), so every factor, pivot and solution is bit-identical to
-// the per-call path (posit_rgetrf_dev + posit_rgetrs_dev, posit_rpotrf_dev +
-// posit_rpotrs_dev) and to the CPU routines.
+// decreasing size, so the largest problems start first) and factors and solves it alone.
+// Per-element operation order is the reference's (see lapack.cu), so every factor, pivot and
+// solution is bit-identical to the per-call path (posit_rgetrf_dev + posit_rgetrs_dev,
+// posit_rpotrf_dev + posit_rpotrs_dev) and to the CPU routines.
+//
+// A problem is factored by panels of up to 16 or 32 columns: the panel in shared memory as FP64,
+// the trailing matrix in global memory (L2) as patterns, updated by 64x64 tiles in the GEMM's
+// k-step (gemm_tile.cuh).  So an element is converted once per panel and its 16 or 32
+// multiply-adds run from registers; one column per step, the form this replaced, converted
+// every element for every multiply-add (about 80 instructions each).  The right-hand sides
+// follow in shared memory, the L^T solve by warp_chain (one thread's chain before).
 #include "batch.cuh"
+#include "gemm_tile.cuh"
 #include "posit32.cuh"
 #include "trsm_chain.cuh"
+
+#include <limits.h>
 
 namespace pg {
 
 namespace {
 
-constexpr int BT = 256; // threads per problem
-
-// The per-element steps are the FP64 form of p32_mul + p32_add (posit32.cuh,
-// f64_posit_mac_checked): operands converted from patterns, the result assembled back
-// without rounding.  Row k and column k of a factor step are staged in shared memory as
-// FP64 when 2n doubles fit in the staging buffer.
-constexpr int STAGE_DOUBLES = BATCH_MAX_N / 2; // s_row (BATCH_MAX_N words) as FP64
+// Two shapes of CTA.  Problems of more than BATCH_LARGE_N rows: 512 threads, panels of up to
+// 32 columns, one CTA per SM -- the longest problem bounds the launch, so it gets a whole SM.
+// The rest: 256 threads, panels of up to 16, two CTAs per SM.  (One shape of 256 threads for
+// all: an LU of n = 512 took 12.1 ms alone and 17.8 with a second CTA on its SM, as long as
+// all 2000 problems of the mix together.)
+template <int THREADS, int JB_, int AREA>
+struct BatchCfg {
+    static constexpr int T = THREADS;
+    static constexpr int GROUPS = T / 256;  // 256 threads work on a trailing tile
+    static constexpr int JB = JB_;          // most columns of a panel
+    static constexpr int CH = 64 * GROUPS;  // columns of the trailing matrix taken together
+    static constexpr int UL = CH + 2;       // doubles per row of U12 in shared memory
+    // Shared memory: tables; the rows of U12 of one stretch of columns; the rest: a panel
+    // [jb][PL], or the right-hand sides, or the L^T solves' columns and terms.
+    static constexpr int U_BYTES = (JB * UL * 8 + 127) / 128 * 128;
+    static constexpr int AREA_BYTES = AREA;
+    static constexpr int SMEM = STEP_TAB_BYTES + U_BYTES + AREA_BYTES;
+};
+using LargeCfg = BatchCfg<512, 32, (512 * 32 + 64) * 8>;
+using SmallCfg = BatchCfg<256, 16, 512 * 16 * 8 + 10 * 1024>;
+static_assert(LargeCfg::SMEM + 4096 <= 227 * 1024, "one CTA per SM");
+static_assert(2 * (SmallCfg::SMEM + 3072) <= 228 * 1024, "two CTAs per SM");
+constexpr int BJB = 32; // the larger JB
 
 __device__ __forceinline__ double pd(uint32_t u) { return p32_to_double(u); }
 
-// b <- b + t*a on patterns through the FP64 step
-__device__ __forceinline__ void mac_store(uint32_t *p, double t, double a)
-{
-    *p = p32_from_double_exact(f64_posit_mac_checked(pd(*p), t, a));
-}
-
-// Walks the rows x rows trailing block of step k as flat indexes e = tid, tid + BT, ...
-// (row fastest) without a division per element.
-struct TrailWalk {
-    int i, c;           // the current element (row, column)
-    int di, dc, lo, hi; // the step, and the row range [lo, hi)
-    __device__ TrailWalk(int rows, int k)
-        : i(k + 1 + (int)threadIdx.x % rows), c(k + 1 + (int)threadIdx.x / rows), di(BT % rows), dc(BT / rows),
-          lo(k + 1), hi(k + 1 + rows)
-    {
-    }
-    __device__ void next()
-    {
-        i += di;
-        c += dc;
-        if (i >= hi) {
-            i -= hi - lo;
-            ++c;
-        }
-    }
+struct BatchShared {
+    int hi[16], row[16]; // the warps' pivot candidates
+    uint32_t lo[16];
+    double val[16];
+    LtxRow ltx[2];
+    int piv[BJB];                     // the panel's pivots (rows of the matrix, 0-based)
+    int src[BJB], dst[BJB], from[BJB]; // net interchange: block row i <- src[i]; row dst[i] <- from[i] (dst < 0: none)
 };
 
-__device__ int iramax_block(const uint32_t *col, int k, int n, int32_t *s_key, int *s_idx)
+// The panel's operands in a trailing tile: as = panel rows, ts = U12 or the panel again.
+struct PanelOps {
+    static constexpr bool NEG = true; // c + (-u)*l
+    int pl, ul;
+    __device__ __forceinline__ int a(int q, int l) const { return l * pl + q * BLK; }
+    __device__ __forceinline__ int t(int q, int l) const { return l * ul + q * BLK; }
+};
+
+// rw[c * T] += -u[c] * l for c in [c0, c1).
+__device__ __forceinline__ void row_update(double *rw, int T, const double *u, double l, int c0, int c1,
+                                           const unsigned char *tab)
+{
+    constexpr int U = 4;
+    int c = c0;
+#pragma unroll 1
+    for (; c + U <= c1; c += U) {
+        double y[U], *p = rw + c * T;
+        bool bad = false;
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            y[q] = step_one(p[q * T], -u[c + q], l, tab);
+            bad |= y[q] != y[q];
+        }
+        if (bad)
+            break; // the rest one by one
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            p[q * T] = y[q];
+    }
+#pragma unroll 1
+    for (; c < c1; ++c)
+        rw[c * T] = mac_any(rw[c * T], -u[c], l, tab);
+}
+
+// The largest |x| (NaN below everything), the lowest row among equal ones, over the warp.
+struct Best {
+    int hi, row;
+    uint32_t lo;
+};
+__device__ __forceinline__ int best_lane(const Best &b)
+{
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const int hi = __reduce_max_sync(FULL, b.hi);
+    const uint32_t lo = __reduce_max_sync(FULL, b.hi == hi ? b.lo : 0u);
+    const int row = __reduce_min_sync(FULL, b.hi == hi && b.lo == lo ? b.row : INT_MAX);
+    return __ffs(__ballot_sync(FULL, b.hi == hi && b.lo == lo && b.row == row)) - 1;
+}
+
+// The panel of columns [j, j+jb): factored in shared memory, panel row r being matrix row j+r.
+// LU: s.piv; Cholesky: returns the column whose diagonal failed, or jb.  `info` (LU): the
+// first zero pivot, 1-based.
+template <class C, bool LU>
+__device__ __forceinline__ int factor_panel(double *pan, int PL, int M, int j, int jb, int &info, BatchShared &s,
+                                            const unsigned char *tab)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto cand_init = [](Best &b, double &bv) {
+        b = Best{INT_MIN, INT_MAX, 0u};
+        bv = 0.0;
+    };
+    auto cand_add = [](Best &b, double &bv, double v, int r) { // rows in increasing order
+        const int hi = v != v ? -1 : __double2hiint(fabs(v));
+        const uint32_t lo = v != v ? 0u : (uint32_t)__double2loint(v);
+        if (hi > b.hi || (hi == b.hi && lo > b.lo)) {
+            b = Best{hi, r, lo};
+            bv = v;
+        }
+    };
+    auto cand_put = [&](const Best &b, double bv) {
+        if (lane == best_lane(b)) {
+            s.hi[warp] = b.hi;
+            s.lo[warp] = b.lo;
+            s.row[warp] = b.row;
+            s.val[warp] = bv;
+        }
+    };
+    Best b;
+    double bv;
+    if (LU) {
+        cand_init(b, bv);
+        for (int r = tid; r < M; r += C::T)
+            cand_add(b, bv, pan[r], r);
+        cand_put(b, bv);
+        __syncthreads();
+    }
+    for (int k = 0; k < jb; ++k) {
+        double *ck = pan + k * PL;
+        double mult;
+        if (LU) {
+            Best cd = {INT_MIN, INT_MAX, 0u};
+            if (lane < C::T / 32)
+                cd = Best{s.hi[lane], s.row[lane], s.lo[lane]};
+            const int w = best_lane(cd), p = s.row[w];
+            const double v = s.val[w];
+            if (v == 0.0 && info == 0)
+                info = j + k + 1;
+            // a zero pivot leaves its own column in place (Rgetrf2.cpp:107-117)
+            if (p != k && tid < jb && !(tid == k && v == 0.0)) {
+                double *c2 = pan + tid * PL;
+                const double t = c2[k];
+                c2[k] = c2[p];
+                c2[p] = t;
+            }
+            if (tid == 0)
+                s.piv[k] = j + p;
+            // nothing scaled under a zero pivot; a NaR one makes the column NaR, as dividing by it does
+            mult = v == 0.0 ? 1.0 : f64_posit_div(1.0, v, 1.0 / v);
+            __syncthreads(); // the rows have changed places
+        } else {
+            const double akk = ck[k];
+            if (!(akk > 0.0)) // Rpotrf2.cpp:90-93; the same in every thread
+                return k;
+            const double lkk = f64_posit_sqrt(akk);
+            mult = f64_posit_div(1.0, lkk, 1.0 / lkk);
+            __syncthreads(); // every thread has read a_kk
+            if (tid == 0)
+                ck[k] = lkk;
+            for (int r = k + 1 + tid; r < M; r += C::T)
+                ck[r] = mul_any(ck[r], mult, tab);
+            __syncthreads(); // the column's l_ck
+        }
+        const double *u = LU ? pan + k : ck; // u[c]: row k's column c (LU), or l_ck
+        cand_init(b, bv);
+        for (int r = tid; r < M; r += C::T)
+            if (r > k) {
+                double l = ck[r];
+                if (LU) {
+                    l = mul_any(l, mult, tab);
+                    ck[r] = l;
+                    // row k's columns lie PL apart: through registers, four at a time
+                    int c = k + 1;
+#pragma unroll 1
+                    for (; c < jb; c += 4) {
+                        double y[4];
+                        bool bad = false;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int cc = min(c + q, jb - 1);
+                            y[q] = step_one(pan[cc * PL + r], -u[cc * PL], l, tab);
+                            bad |= y[q] != y[q];
+                        }
+                        if (bad) {
+#pragma unroll 1
+                            for (int q = 0; q < 4 && c + q < jb; ++q)
+                                pan[(c + q) * PL + r] = mac_any(pan[(c + q) * PL + r], -u[(c + q) * PL], l, tab);
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                if (c + q < jb)
+                                    pan[(c + q) * PL + r] = y[q];
+                        }
+                    }
+                    if (k + 1 < jb)
+                        cand_add(b, bv, pan[(k + 1) * PL + r], r);
+                } else {
+                    row_update(pan + r, PL, u, l, k + 1, min(jb, r + 1), tab);
+                }
+            }
+        if (LU && k + 1 < jb)
+            cand_put(b, bv);
+        __syncthreads();
+    }
+    return jb;
+}
+
+// The panel's interchanges as one permutation (s.src, s.dst, s.from), by the first warp: the
+// interchanges in order as exchanges between lanes, of row numbers (lapack.cu, lu_rows_kernel).
+__device__ __forceinline__ void net_interchange(int j, int jb, BatchShared &s)
+{
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const int t = lane < jb ? s.piv[lane] : -1;
+    int alias = -1; // pivots below the block: the first lane with that row keeps its content
+    if (t >= j + jb) {
+        alias = lane;
+        for (int q = 0; q < lane; ++q)
+            if (s.piv[q] == t) {
+                alias = q;
+                break;
+            }
+    }
+    int v = j + lane, w = t;
+    for (int i = 0; i < jb; ++i) {
+        const int ti = __shfl_sync(FULL, t, i), ai = __shfl_sync(FULL, alias, i);
+        if (ti == j + i)
+            continue;
+        const bool in = ti < j + jb;
+        const int o = in ? ti - j : ai;
+        const int vi = __shfl_sync(FULL, v, i), vo = __shfl_sync(FULL, in ? v : w, o);
+        if (lane == o) {
+            if (in)
+                v = vi;
+            else
+                w = vi;
+        }
+        if (lane == i)
+            v = vo;
+    }
+    if (lane < jb) {
+        s.src[lane] = v;
+        s.dst[lane] = alias == lane ? t : -1;
+        s.from[lane] = w;
+    }
+}
+
+// One column outside the panel through its interchanges.  Every value is read before one is
+// written.
+template <int JB>
+__device__ __forceinline__ void permute_column(uint32_t *col, int j, int jb, const BatchShared &s)
+{
+    uint32_t v[JB], w[JB];
+#pragma unroll
+    for (int i = 0; i < JB; ++i) {
+        v[i] = i < jb && s.src[i] != j + i ? col[s.src[i]] : 0u;
+        w[i] = i < jb && s.dst[i] >= 0 ? col[s.from[i]] : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < JB; ++i)
+        if (i < jb) {
+            if (s.dst[i] >= 0)
+                col[s.dst[i]] = w[i];
+            if (s.src[i] != j + i)
+                col[j + i] = v[i];
+        }
+}
+
+// The unit-lower solve of the block's rows of one column, in place: x_i += -l_ik * x_k in the
+// order of k (no multiplier is skipped: the factorization's rank-1 updates).  `u`: the block's
+// rows of the column; pan[k * PL + i] = l_ik.  By 16 rows in registers.
+__device__ __forceinline__ void u12_column(uint32_t *u, const double *pan, int PL, int jb, const unsigned char *tab)
+{
+    constexpr int R = 16;
+    bool bad = false;
+#pragma unroll 1
+    for (int i0 = 0; i0 < jb; i0 += R) {
+        double x[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            x[i] = i0 + i < jb ? pd(u[i0 + i]) : 0.0;
+#pragma unroll 1
+        for (int k = 0; k < i0; ++k) {
+            const double xk = -pd(u[k]), *l = pan + k * PL + i0;
+#pragma unroll
+            for (int i = 0; i < R; ++i) // (past jb: a row below the block, into an x not stored)
+                x[i] = step_one(x[i], xk, l[i], tab);
+        }
+#pragma unroll
+        for (int k = 0; k + 1 < R; ++k)
+            if (i0 + k < jb) {
+                const double xk = -x[k], *l = pan + (i0 + k) * PL + i0;
+#pragma unroll
+                for (int i = k + 1; i < R; ++i)
+                    x[i] = step_one(x[i], xk, l[i], tab);
+            }
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            bad |= i0 + i < jb && x[i] != x[i];
+        if (bad) { // step by step, in place
+#pragma unroll 1
+            for (int k = 0; k < min(jb, i0 + R); ++k) {
+                const double xk = -pd(u[k]);
+#pragma unroll 1
+                for (int i = max(k + 1, i0); i < min(jb, i0 + R); ++i)
+                    u[i] = p32_from_double_exact(mac_any(pd(u[i]), xk, pan[k * PL + i], tab));
+            }
+            bad = false;
+        } else {
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                if (i0 + i < jb)
+                    u[i0 + i] = p32_from_double_exact(x[i]);
+        }
+    }
+}
+
+// 64x64 outputs of the trailing matrix at (row0, col0): C += -(rows of the panel) * (ts), jb
+// steps.  LOWER: only row >= column.
+template <bool LOWER>
+__device__ __forceinline__ void trailing_tile(uint32_t *A, size_t lda, int n, int row0, int col0, const double *as,
+                                              const double *ts, PanelOps ops, int steps, const unsigned char *tab)
+{
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16 % 16;
+    double acc[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = row0 + own_off(tx, i), col = col0 + own_off(ty, q);
+            const bool in = row < n && col < n && (!LOWER || row >= col);
+            acc[i][q] = in ? pd(A[row + (size_t)col * lda]) : 1.0;
+        }
+    bool slow = false;
+    tile_steps<2>(acc, as, ts, steps, tab, tx, ty, ops, slow);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = row0 + own_off(tx, i), col = col0 + own_off(ty, q);
+            if (row < n && col < n && (!LOWER || row >= col))
+                A[row + (size_t)col * lda] = p32_from_double_exact(acc[i][q]);
+        }
+}
+
+// Rgetrf / Rpotrf('L') of one problem; returns info.
+template <class C, bool LU>
+__device__ __forceinline__ int factor_one(const BatchProblem &pr, unsigned char *smem, BatchShared &s)
+{
+    const int n = pr.n, tid = threadIdx.x;
+    uint32_t *A = pr.A;
+    const size_t lda = (size_t)pr.lda;
+    const unsigned char *tab = smem;
+    double *U = reinterpret_cast<double *>(smem + STEP_TAB_BYTES);
+    double *pan = reinterpret_cast<double *>(smem + STEP_TAB_BYTES + C::U_BYTES);
+    const int group = tid / 256;
+    int info = 0;
+    for (int j = 0, jb = 0; j < n; j += jb) {
+        const int M = n - j, PL = (M + 1) & ~1;
+        // (64 doubles over: a tile at the edge reads past the panel's last row)
+        const int fit = ((int)(C::AREA_BYTES / sizeof(double)) - 64) / PL & ~1;
+        jb = min(min(C::JB, fit), M);
+        for (int c = 0; c < jb; ++c)
+            for (int r = tid; r < M; r += C::T)
+                pan[c * PL + r] = (LU || r >= c) ? pd(A[(j + r) + (size_t)(j + c) * lda]) : 0.0;
+        __syncthreads();
+        const int done = factor_panel<C, LU>(pan, PL, M, j, jb, info, s, tab);
+        if (!LU && done < jb) // the columns before the failed one still update the rest
+            info = j + done + 1;
+        for (int c = 0; c < jb; ++c)
+            for (int r = tid; r < M; r += C::T)
+                if (LU || r >= c)
+                    A[(j + r) + (size_t)(j + c) * lda] = p32_from_double_exact(pan[c * PL + r]);
+        if (LU) {
+            if (tid < jb)
+                pr.ipiv[j + tid] = s.piv[tid] + 1;
+            if (tid < 32)
+                net_interchange(j, jb, s);
+            __syncthreads();
+            // the columns outside the panel: interchanges and, right of it, U12
+            for (int c = tid; c < n - jb; c += C::T) {
+                uint32_t *col = A + (size_t)(c < j ? c : c + jb) * lda;
+                permute_column<C::JB>(col, j, jb, s);
+                if (c >= j)
+                    u12_column(col + j, pan, PL, jb, tab);
+            }
+            __syncthreads();
+        }
+        const int steps = (done + 1) & ~1;
+        if (steps > done) { // an odd count of steps: one more of zeros
+            __syncthreads();
+            for (int r = tid; r < M; r += C::T)
+                if (done < jb || fit > jb) // (a panel of an odd count is the last one or a failed one)
+                    pan[done * PL + r] = 0.0;
+            __syncthreads();
+        }
+        const PanelOps ops{PL, LU ? C::UL : PL};
+        for (int c0 = j + jb; c0 < n; c0 += C::CH) {
+            if (LU) { // U12 of these columns, from where the step above left it
+                for (int e = tid; e < jb * C::CH; e += C::T) {
+                    const int k = e % jb, c = e / jb;
+                    U[k * C::UL + c] = c0 + c < n ? pd(A[(j + k) + (size_t)(c0 + c) * lda]) : 0.0;
+                }
+                __syncthreads();
+            }
+            const int cg = c0 + 64 * group; // this group's 64 columns
+            if (cg < n)
+                for (int r0 = LU ? j + jb : cg; r0 < n; r0 += 64)
+                    trailing_tile<!LU>(A, lda, n, r0, cg, pan + (r0 - j), LU ? U + 64 * group : pan + (cg - j), ops, steps,
+                                       tab);
+            if (LU)
+                __syncthreads(); // U is done with
+        }
+        if (!LU && done < jb)
+            break;
+        __syncthreads();
+    }
+    return info;
+}
+
+// b_i - b_k*a_ik for the rows of one step of an axpy-form solve, all right-hand sides of the
+// group; the thread with row `next` then divides it (Rtrsm.cpp:127, 145; a zero is left
+// alone, as the reference skips it).
+constexpr int B_PRE = 2; // rows per thread whose coefficients are loaded a step ahead
+
+// Rtrsm('L', LOWER ? 'L' : 'U', 'N') on the columns X (shared memory, [nrhs][n], FP64).
+template <class C, bool LOWER, bool UNIT>
+__device__ __forceinline__ void axpy_solve(const uint32_t *A, size_t lda, int n, double *X, int nrhs,
+                                           const unsigned char *tab)
 {
     const int tid = threadIdx.x;
-    int32_t best = INT32_MIN;
-    int bidx = -1;
-    for (int i = k + tid; i < n; i += blockDim.x) {
-        int32_t key = (int32_t)pabs(col[i]);
-        if (bidx < 0 || key > best) {
-            best = key;
-            bidx = i;
+    auto col_of = [&](int st) { return LOWER ? st : n - 1 - st; };
+    auto finish = [&](int i) {
+        const double d = pd(A[i + (size_t)i * lda]), rc = 1.0 / d;
+        for (int r = 0; r < nrhs; ++r) {
+            double *x = X + (size_t)r * n;
+            if (x[i] != 0.0)
+                x[i] = f64_posit_div(x[i], d, rc);
         }
-    }
-    s_key[tid] = best;
-    s_idx[tid] = bidx;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (tid < s) {
-            int32_t k2 = s_key[tid + s];
-            int i2 = s_idx[tid + s];
-            if (i2 >= 0 && (s_idx[tid] < 0 || k2 > s_key[tid] || (k2 == s_key[tid] && i2 < s_idx[tid]))) {
-                s_key[tid] = k2;
-                s_idx[tid] = i2;
-            }
-        }
+    };
+    uint32_t cur[B_PRE], nxt[B_PRE];
+#pragma unroll
+    for (int q = 0; q < B_PRE; ++q)
+        cur[q] = tid + q * C::T < n ? A[(tid + q * C::T) + (size_t)col_of(0) * lda] : 0u;
+    if (!UNIT) {
+        if (tid == col_of(0) % C::T)
+            finish(col_of(0));
         __syncthreads();
     }
-    int p = s_idx[0];
-    __syncthreads();
-    return p;
-}
-
-// Rgetrf (as unblocked right-looking LU) + Rgetrs('N') for one problem.
-__device__ void lu_solve_one(const BatchProblem &pr, bool factor, int32_t *s_key, int *s_idx, uint32_t *s_row)
-{
-    const int n = pr.n, tid = threadIdx.x;
-    uint32_t *A = pr.A;
-    const size_t lda = (size_t)pr.lda;
-    int info = 0;
-    __shared__ uint32_t s_piv, s_recip;
-    __shared__ int s_mode;
-    for (int k = 0; k < (factor ? n : 0); ++k) {
-        uint32_t *ck = A + (size_t)k * lda;
-        const int p = iramax_block(ck, k, n, s_key, s_idx);
-        const uint32_t piv = ck[p];
-        if (tid == 0) {
-            pr.ipiv[k] = p + 1;
-            if (piv == 0) {
-                s_mode = 0;
-            } else if ((int32_t)pabs(piv) >= 1) {
-                s_mode = 1;
-                s_recip = pdiv_est(P32_ONE, piv);
-            } else {
-                s_mode = 2;
+    for (int st = 0; st < n; ++st) {
+        const int k = col_of(st), kn = col_of(st + 1);
+        const uint32_t *ak = A + (size_t)k * lda;
+#pragma unroll
+        for (int q = 0; q < B_PRE; ++q)
+            nxt[q] = (st + 1 < n && tid + q * C::T < n) ? A[(tid + q * C::T) + (size_t)kn * lda] : 0u;
+        auto update = [&](int i, uint32_t a) {
+            if (LOWER ? i > k : i < k) {
+                const double l = pd(a);
+                for (int r = 0; r < nrhs; ++r) {
+                    double *x = X + (size_t)r * n;
+                    const double xk = x[k];
+                    if (xk != 0.0) // zero multipliers skipped (Rtrsm.cpp:125-126, 143-144)
+                        x[i] = mac_any(x[i], -xk, l, tab);
+                }
             }
-            s_piv = piv;
-        }
-        if (piv == 0 && info == 0)
-            info = k + 1;
+        };
+#pragma unroll
+        for (int q = 0; q < B_PRE; ++q)
+            if (tid + q * C::T < n)
+                update(tid + q * C::T, cur[q]);
+#pragma unroll 1
+        for (int i = tid + B_PRE * C::T; i < n; i += C::T)
+            update(i, ak[i]);
+        if (!UNIT && st + 1 < n && tid == kn % C::T)
+            finish(kn);
         __syncthreads();
-        if (p != k) { // interchange whole rows (Rlaswp on both sides)
-            // A zero pivot leaves its own column in place (Rgetrf2.cpp:107-117) while the
-            // recursion's Rlaswp calls still move rows k and p in every other column.
-            for (int c = tid; c < n; c += blockDim.x) {
-                if (c == k && piv == 0)
-                    continue;
-                uint32_t *pc = A + (size_t)c * lda;
-                uint32_t t = pc[k];
-                pc[k] = pc[p];
-                pc[p] = t;
-            }
-        }
-        __syncthreads();
-        const int mode = s_mode;
-        for (int i = k + 1 + tid; i < n; i += blockDim.x) {
-            uint32_t l = ck[i];
-            if (mode == 1)
-                l = pmul(s_recip, l);
-            else if (mode == 2)
-                l = pdiv_est(l, s_piv);
-            ck[i] = l;
-        }
-        const bool stage = 2 * n <= STAGE_DOUBLES;
-        double *s_rowd = reinterpret_cast<double *>(s_row), *s_cold = s_rowd + n;
-        for (int c = k + 1 + tid; c < n; c += blockDim.x) {
-            const uint32_t v = pneg(A[k + (size_t)c * lda]);
-            if (stage)
-                s_rowd[c] = pd(v);
-            else
-                s_row[c] = v;
-        }
-        if (stage)
-            for (int i = k + 1 + tid; i < n; i += blockDim.x)
-                s_cold[i] = pd(ck[i]);
-        __syncthreads();
-        const int rows = n - k - 1;
-        if (rows > 0) {
-            TrailWalk w(rows, k);
-            for (; w.c < n; w.next()) {
-                const double t = stage ? s_rowd[w.c] : pd(s_row[w.c]);
-                const double l = stage ? s_cold[w.i] : pd(ck[w.i]);
-                mac_store(A + w.i + (size_t)w.c * lda, t, l);
-            }
-        }
-        __syncthreads();
-    }
-    if (tid == 0 && factor)
-        *pr.info = info;
-    // Rgetrs 'N': interchanges, L (unit) forward, U backward; the right-hand sides in
-    // parallel (each column's per-element order is Rtrsm's, Rtrsm.cpp:121-154)
-    const int nrhs = pr.nrhs;
-    const size_t ldb = (size_t)pr.ldb;
-    for (int r = tid; r < nrhs; r += blockDim.x) { // Rlaswp, in order, on the own column
-        uint32_t *b = pr.B + (size_t)r * ldb;
-        for (int i = 0; i < n; ++i) {
-            const int ip = pr.ipiv[i] - 1;
-            if (ip != i) {
-                const uint32_t t = b[i];
-                b[i] = b[ip];
-                b[ip] = t;
-            }
-        }
-    }
-    __syncthreads();
-    for (int k = 0; k < n; ++k) {
-        const int rows = n - k - 1;
-        const uint32_t *lk = A + (size_t)k * lda;
-        for (int e = tid; e < rows * nrhs; e += blockDim.x) {
-            uint32_t *b = pr.B + (size_t)(e / rows) * ldb;
-            const int i = k + 1 + e % rows;
-            const uint32_t bk = b[k];
-            if (bk != 0)
-                mac_store(b + i, -pd(bk), pd(lk[i]));
-        }
-        __syncthreads();
-    }
-    for (int k = n - 1; k >= 0; --k) {
-        const uint32_t *uk = A + (size_t)k * lda;
-        for (int r = tid; r < nrhs; r += blockDim.x) {
-            uint32_t *b = pr.B + (size_t)r * ldb;
-            if (b[k] != 0)
-                b[k] = pdiv_est(b[k], uk[k]);
-        }
-        __syncthreads();
-        for (int e = tid; e < k * nrhs; e += blockDim.x) {
-            uint32_t *b = pr.B + (size_t)(e / k) * ldb;
-            const int i = e % k;
-            const uint32_t bk = b[k];
-            if (bk != 0)
-                mac_store(b + i, -pd(bk), pd(uk[i]));
-        }
-        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < B_PRE; ++q)
+            cur[q] = nxt[q];
     }
 }
 
-// Rpotrf('L') (as unblocked right-looking Cholesky) + Rpotrs('L') for one problem.
-__device__ void chol_solve_one(const BatchProblem &pr, bool factor, uint32_t *s_row)
+// The right-hand sides: Rgetrs('N') or Rpotrs('L').
+template <class C, bool LU>
+__device__ __forceinline__ void solve_one(const BatchProblem &pr, unsigned char *smem, BatchShared &s)
 {
     const int n = pr.n, tid = threadIdx.x;
-    uint32_t *A = pr.A;
-    const size_t lda = (size_t)pr.lda;
-    __shared__ uint32_t s_recip;
-    __shared__ int s_fail;
-    int info = 0;
-    for (int k = 0; k < (factor ? n : 0); ++k) {
-        uint32_t *ck = A + (size_t)k * lda;
-        if (tid == 0) {
-            uint32_t akk = ck[k];
-            s_fail = (int32_t)akk <= 0;
-            if (!s_fail) {
-                uint32_t lkk = psqrt_est(akk);
-                ck[k] = lkk;
-                s_recip = pdiv_est(P32_ONE, lkk);
-            }
-        }
-        __syncthreads();
-        if (s_fail) {
-            info = k + 1;
-            break;
-        }
-        const bool stage = n <= STAGE_DOUBLES;
-        double *s_cold = reinterpret_cast<double *>(s_row);
-        for (int i = k + 1 + tid; i < n; i += blockDim.x) {
-            const uint32_t l = pmul(s_recip, ck[i]);
-            ck[i] = l;
-            if (stage)
-                s_cold[i] = pd(l);
-            else
-                s_row[i] = l;
-        }
-        __syncthreads();
-        // lower part of the trailing matrix: a_ic += (-l_ck)*l_ik, k < c <= i
-        const int rows = n - k - 1;
-        if (rows > 0) {
-            TrailWalk w(rows, k);
-            for (; w.c < n; w.next()) {
-                if (w.i >= w.c) {
-                    const double lc = stage ? s_cold[w.c] : pd(s_row[w.c]);
-                    const double li = stage ? s_cold[w.i] : pd(s_row[w.i]);
-                    mac_store(A + w.i + (size_t)w.c * lda, -lc, li);
+    const unsigned char *tab = smem;
+    unsigned char *area = smem + STEP_TAB_BYTES + C::U_BYTES;
+    double *X = reinterpret_cast<double *>(area);
+    const int group = max(1, (int)((C::AREA_BYTES - 4 * (size_t)n) / (8 * (size_t)n)));
+    for (int r0 = 0; r0 < pr.nrhs; r0 += group) {
+        const int cnt = min(group, pr.nrhs - r0);
+        uint32_t *B = pr.B + (size_t)r0 * pr.ldb;
+        for (int r = 0; r < cnt; ++r)
+            for (int i = tid; i < n; i += C::T)
+                X[(size_t)r * n + i] = pd(B[(size_t)r * pr.ldb + i]);
+        if (LU) { // Rlaswp, in order, a thread per column
+            int *piv = reinterpret_cast<int *>(X + (size_t)cnt * n);
+            for (int i = tid; i < n; i += C::T)
+                piv[i] = pr.ipiv[i] - 1;
+            __syncthreads();
+            for (int r = tid; r < cnt; r += C::T) {
+                double *x = X + (size_t)r * n;
+                for (int i = 0; i < n; ++i) {
+                    const int p = piv[i];
+                    const double t = x[i];
+                    x[i] = x[p];
+                    x[p] = t;
                 }
             }
         }
         __syncthreads();
+        axpy_solve<C, true, LU>(pr.A, (size_t)pr.lda, n, X, cnt, tab);
+        if (LU)
+            axpy_solve<C, false, false>(pr.A, (size_t)pr.lda, n, X, cnt, tab);
+        for (int r = 0; r < cnt; ++r)
+            for (int i = tid; i < n; i += C::T)
+                B[(size_t)r * pr.ldb + i] = p32_from_double_exact(X[(size_t)r * n + i]);
+        __syncthreads();
     }
-    if (tid == 0 && factor)
-        *pr.info = info;
-    if (info != 0)
+    if (LU)
         return;
-    // Rpotrs 'L': L forward (Rtrsm.cpp:139-154, non-unit), the right-hand sides in
-    // parallel; then L^T backward, one thread's chain per right-hand side (trsm_chain.cuh)
-    const int nrhs = pr.nrhs;
-    const size_t ldb = (size_t)pr.ldb;
+    // L^T backward.  Few right-hand sides: one after the other, a warp adding and the others
+    // forming terms; more: a warp for each, as many at a time as fit.
+    const size_t one = 2 * ChainTerms64::bytes(n) + (size_t)n * 8;
+    if (pr.nrhs <= 2 && one <= (size_t)C::AREA_BYTES) {
+        LtxCol64 x;
+        x.b = reinterpret_cast<double *>(area + 2 * ChainTerms64::bytes(n));
+        for (int r = 0; r < pr.nrhs; ++r) {
+            uint32_t *b = pr.B + (size_t)r * pr.ldb;
+            for (int i = tid; i < n; i += C::T)
+                x.set(i, pd(b[i]));
+            block_ltx_solve<C::T, false, ChainTerms64>(pr.A, (size_t)pr.lda, x, n, false, area, s.ltx);
+            for (int i = tid; i < n; i += C::T)
+                b[i] = p32_from_double_exact(x.get(i));
+            __syncthreads();
+        }
+        return;
+    }
+    const size_t per = ChainTerms64::bytes(n) + (((size_t)n * 8 + 15) & ~(size_t)15);
+    const int warps = min(C::T / 32, (int)(C::AREA_BYTES / per)), warp = tid >> 5, lane = tid & 31;
+    if (warp < warps) {
+        ChainTerms64 q;
+        q.q = reinterpret_cast<double *>(area + warp * per);
+        double *x = reinterpret_cast<double *>(area + warp * per + ChainTerms64::bytes(n));
+        for (int r = warp; r < pr.nrhs; r += warps) {
+            uint32_t *b = pr.B + (size_t)r * pr.ldb;
+            for (int i = lane; i < n; i += 32)
+                x[i] = pd(b[i]);
+            __syncwarp();
+            warp_llt_solve(pr.A, (size_t)pr.lda, x, n, q);
+            for (int i = lane; i < n; i += 32)
+                b[i] = p32_from_double_exact(x[i]);
+            __syncwarp();
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Problems of up to 32 rows: a warp each, a row per lane, the matrix in shared memory.
+// ---------------------------------------------------------------------------
+// A CTA's barriers cost such a problem more than its arithmetic; eight of them run side by
+// side in a CTA instead.
+constexpr int SMALL_N = 32;
+constexpr int SMALL_LD = SMALL_N + 1;
+struct SmallArea {
+    double a[SMALL_N * SMALL_LD]; // a_ic at [c * SMALL_LD + i]
+    double x[SMALL_N];
+    double terms[36]; // ChainTerms64 of 32
+    int piv[SMALL_N];
+};
+static_assert(ChainTerms64::GROUP_DOUBLES * (SMALL_N / 16) == 36, "");
+static_assert(sizeof(SmallArea) * (SmallCfg::T / 32) <= SmallCfg::U_BYTES + SmallCfg::AREA_BYTES, "a problem per warp");
+
+template <bool LU>
+__device__ __forceinline__ int small_factor(SmallArea &w, int n, const unsigned char *tab)
+{
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    int info = 0;
     for (int k = 0; k < n; ++k) {
-        const uint32_t *lk = A + (size_t)k * lda;
-        for (int r = tid; r < nrhs; r += blockDim.x) {
-            uint32_t *b = pr.B + (size_t)r * ldb;
-            if (b[k] != 0)
-                b[k] = pdiv_est(b[k], lk[k]);
+        double *ck = w.a + k * SMALL_LD;
+        double mult;
+        const double mine = ck[lane];
+        if (LU) {
+            Best b = {INT_MIN, INT_MAX, 0u};
+            if (lane >= k && lane < n)
+                b = Best{mine != mine ? -1 : __double2hiint(fabs(mine)), lane,
+                         mine != mine ? 0u : (uint32_t)__double2loint(mine)};
+            const int p = best_lane(b);
+            const double v = __shfl_sync(FULL, mine, p);
+            if (v == 0.0 && info == 0)
+                info = k + 1;
+            if (p != k && lane < n && !(lane == k && v == 0.0)) { // a column per lane
+                double *c2 = w.a + lane * SMALL_LD;
+                const double t = c2[k];
+                c2[k] = c2[p];
+                c2[p] = t;
+            }
+            if (lane == 0)
+                w.piv[k] = p;
+            mult = v == 0.0 ? 1.0 : f64_posit_div(1.0, v, 1.0 / v);
+            __syncwarp();
+        } else {
+            const double akk = __shfl_sync(FULL, mine, k);
+            if (!(akk > 0.0))
+                return k + 1;
+            const double lkk = f64_posit_sqrt(akk);
+            mult = f64_posit_div(1.0, lkk, 1.0 / lkk);
+            if (lane == k)
+                ck[k] = lkk;
         }
-        __syncthreads();
-        const int rows = n - k - 1;
-        for (int e = tid; e < rows * nrhs; e += blockDim.x) {
-            uint32_t *b = pr.B + (size_t)(e / rows) * ldb;
-            const int i = k + 1 + e % rows;
-            const uint32_t bk = b[k];
-            if (bk != 0)
-                mac_store(b + i, -pd(bk), pd(lk[i]));
+        double l = 0.0;
+        if (lane > k && lane < n) {
+            l = mul_any(ck[lane], mult, tab);
+            ck[lane] = l;
         }
+        __syncwarp(); // LU: row k in place; Cholesky: the column's l_ck
+#pragma unroll 1
+        for (int c = k + 1; c < n; c += 4) {
+            double y[4];
+            bool bad = false;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int cc = min(c + q, n - 1);
+                y[q] = step_one(w.a[cc * SMALL_LD + lane], -(LU ? w.a[cc * SMALL_LD + k] : ck[cc]), l, tab);
+                bad |= y[q] != y[q];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                double *e = w.a + (c + q) * SMALL_LD;
+                if (c + q < n && lane < n && (LU ? lane > k : lane >= c + q))
+                    e[lane] = bad ? mac_any(e[lane], -(LU ? e[k] : ck[c + q]), l, tab) : y[q];
+            }
+        }
+        __syncwarp();
+    }
+    return info;
+}
+
+template <bool LU>
+__device__ __forceinline__ void run_small(const BatchProblem &pr, SmallArea &w, const unsigned char *tab)
+{
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const int n = pr.n, lane = threadIdx.x & 31;
+    const size_t lda = (size_t)pr.lda;
+    const bool factor = !(pr.kind & BATCH_SOLVE_ONLY);
+    for (int c = 0; c < n; ++c)
+        w.a[c * SMALL_LD + lane] = (lane < n && (LU || lane >= c)) ? pd(pr.A[lane + (size_t)c * lda]) : 0.0;
+    __syncwarp();
+    if (factor) {
+        const int info = small_factor<LU>(w, n, tab);
+        for (int c = 0; c < n; ++c)
+            if (lane < n && (LU || lane >= c))
+                pr.A[lane + (size_t)c * lda] = p32_from_double_exact(w.a[c * SMALL_LD + lane]);
+        if (LU && lane < n)
+            pr.ipiv[lane] = w.piv[lane] + 1;
+        if (lane == 0)
+            *pr.info = info;
+        if (!LU && info != 0)
+            return;
+    } else if (LU) {
+        if (lane < n)
+            w.piv[lane] = pr.ipiv[lane] - 1;
+    }
+    __syncwarp();
+    double d = 1.0;
+    if (lane < n)
+        d = w.a[lane * SMALL_LD + lane];
+    const double rc = 1.0 / d;
+    for (int r = 0; r < pr.nrhs; ++r) {
+        uint32_t *b = pr.B + (size_t)r * pr.ldb;
+        double x = lane < n ? pd(b[lane]) : 0.0;
+        if (LU)
+            for (int i = 0; i < n; ++i) { // Rlaswp
+                const int p = w.piv[i];
+                const double xi = __shfl_sync(FULL, x, i), xp = __shfl_sync(FULL, x, p);
+                x = lane == i ? xp : (lane == p ? xi : x);
+            }
+        for (int k = 0; k < n; ++k) { // L forward, zero multipliers skipped
+            if (!LU && lane == k && x != 0.0)
+                x = f64_posit_div(x, d, rc);
+            const double xk = __shfl_sync(FULL, x, k);
+            if (xk != 0.0 && lane > k && lane < n)
+                x = mac_any(x, -xk, w.a[k * SMALL_LD + lane], tab);
+        }
+        if (LU) { // U backward
+            for (int k = n - 1; k >= 0; --k) {
+                if (lane == k && x != 0.0)
+                    x = f64_posit_div(x, d, rc);
+                const double xk = __shfl_sync(FULL, x, k);
+                if (xk != 0.0 && lane < k)
+                    x = mac_any(x, -xk, w.a[k * SMALL_LD + lane], tab);
+            }
+        } else {
+            w.x[lane] = x;
+            __syncwarp();
+            ChainTerms64 q;
+            q.q = w.terms;
+            warp_llt_solve(pr.A, lda, w.x, n, q);
+            x = w.x[lane];
+            __syncwarp();
+        }
+        if (lane < n)
+            b[lane] = p32_from_double_exact(x);
+    }
+}
+
+template <class C, bool LU>
+__device__ __forceinline__ void run_one(const BatchProblem &pr, unsigned char *smem, BatchShared &s)
+{
+    int info = 0;
+    if (!(pr.kind & BATCH_SOLVE_ONLY)) {
+        info = factor_one<C, LU>(pr, smem, s);
+        if (threadIdx.x == 0)
+            *pr.info = info;
         __syncthreads();
     }
-    // L^T backward: the right-hand sides staged in shared memory when they fit
-    const bool staged = n * nrhs <= BATCH_MAX_N;
-    if (staged)
-        for (int e = tid; e < n * nrhs; e += blockDim.x)
-            s_row[e] = pr.B[(size_t)(e / n) * ldb + e % n];
-    __syncthreads();
-    for (int r = tid; r < nrhs; r += blockDim.x)
-        llt_chain(A, lda, staged ? s_row + (size_t)r * n : pr.B + (size_t)r * ldb, n, false);
-    __syncthreads();
-    if (staged)
-        for (int e = tid; e < n * nrhs; e += blockDim.x)
-            pr.B[(size_t)(e / n) * ldb + e % n] = s_row[e];
+    if (pr.n > 0 && pr.nrhs > 0 && (LU || info == 0))
+        solve_one<C, LU>(pr, smem, s);
 }
 
 } // namespace
 
-#ifndef PG_BATCH_MIN_CTAS
-#define PG_BATCH_MIN_CTAS 6 // 40 registers: 6 resident CTAs per SM (measured best of 2, 3, 4, 6, 8)
-#endif
-__global__ void __launch_bounds__(BT, PG_BATCH_MIN_CTAS) batch_factor_kernel(const BatchProblem *__restrict__ probs, int nprob,
-                                                          const int *__restrict__ order, int *__restrict__ next)
+// The problems [first, last) of the list, from the queue `next` (which counts from 0).
+template <class C>
+__global__ void __launch_bounds__(C::T, 512 / C::T) batch_factor_kernel(const BatchProblem *__restrict__ probs, int first,
+                                                                        int last, const int *__restrict__ order,
+                                                                        int *__restrict__ next)
 {
-    __shared__ int32_t s_key[BT];
-    __shared__ int s_idx[BT];
+    extern __shared__ __align__(128) unsigned char smem_batch[];
+    __shared__ BatchShared s;
     __shared__ int s_item;
-    __shared__ __align__(16) uint32_t s_row[BATCH_MAX_N]; // also staged FP64 (8-byte aligned)
+    step_tables_fill(smem_batch, threadIdx.x, C::T);
     for (;;) {
         if (threadIdx.x == 0)
-            s_item = atomicAdd(next, 1);
+            s_item = first + atomicAdd(next, 1);
         __syncthreads();
         const int item = s_item;
         __syncthreads();
-        if (item >= nprob)
+        if (item >= last)
             return;
         const BatchProblem pr = probs[order ? order[item] : item];
-        const bool factor = !(pr.kind & BATCH_SOLVE_ONLY);
+        if (C::T == SmallCfg::T && order && pr.n <= SMALL_N) { // sorted: so are all that follow
+            SmallArea &w = reinterpret_cast<SmallArea *>(smem_batch + STEP_TAB_BYTES)[threadIdx.x >> 5];
+            const bool lead = (threadIdx.x & 31) == 0;
+            auto take = [&]() { return __shfl_sync(0xFFFFFFFFu, lead ? first + atomicAdd(next, 1) : 0, 0); };
+            for (int mine = threadIdx.x < 32 ? item : take(); mine < last; mine = take()) {
+                const BatchProblem ps = probs[order[mine]];
+                if (ps.n > 0) {
+                    if ((ps.kind & 1) == BATCH_LU)
+                        run_small<true>(ps, w, smem_batch);
+                    else
+                        run_small<false>(ps, w, smem_batch);
+                    __syncwarp();
+                } else if (lead && !(ps.kind & BATCH_SOLVE_ONLY)) {
+                    *ps.info = 0;
+                }
+            }
+            return;
+        }
         if ((pr.kind & 1) == BATCH_LU)
-            lu_solve_one(pr, factor, s_key, s_idx, s_row);
+            run_one<C, true>(pr, smem_batch, s);
         else
-            chol_solve_one(pr, factor, s_row);
+            run_one<C, false>(pr, smem_batch, s);
         __syncthreads();
     }
 }
 
-cudaError_t batch_factor_launch(const BatchProblem *probs, int nprob, const int *order, int *next, int ctas,
-                                cudaStream_t st)
+template <class C>
+static cudaError_t launch_cfg(const BatchProblem *probs, int first, int last, const int *order, int *next, int ctas,
+                              cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(next, 0, sizeof(int), st);
+    cudaError_t e = cudaFuncSetAttribute(batch_factor_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(next, 0, sizeof(int), st);
     if (e != cudaSuccess)
         return e;
-    batch_factor_kernel<<<ctas, BT, 0, st>>>(probs, nprob, order, next);
+    const int count = last - first;
+    batch_factor_kernel<C><<<count < ctas ? count : ctas, C::T, C::SMEM, st>>>(probs, first, last, order, next);
     return cudaGetLastError();
+}
+
+cudaError_t batch_factor_launch(bool large, const BatchProblem *probs, int first, int last, const int *order, int *next,
+                                int sms, cudaStream_t st)
+{
+    if (last <= first)
+        return cudaSuccess;
+    return large ? launch_cfg<LargeCfg>(probs, first, last, order, next, sms, st)
+                 : launch_cfg<SmallCfg>(probs, first, last, order, next, 2 * sms, st);
 }
 
 } // namespace pg

@@ -8,6 +8,7 @@ namespace pg {
 constexpr int BATCH_LU = 0;
 constexpr int BATCH_CHOL = 1;
 constexpr int BATCH_MAX_N = 4096; // largest n a batched problem may have
+constexpr int BATCH_LARGE_N = 224;  // a problem of more rows takes an SM for itself
 
 // One problem: A (n x n, column-major, lda) is factored in place, B (n x nrhs, ldb)
 // overwritten with the solution; ipiv (LU) receives n 1-based pivots, info the
@@ -23,9 +24,11 @@ struct BatchProblem {
     int *info;
 };
 
-// Runs problems probs[order[i]] (order may be null) on `ctas` persistent CTAs; `next`
-// is a device counter the launch zeroes first.
-cudaError_t batch_factor_launch(const BatchProblem *probs, int nprob, const int *order, int *next, int ctas,
-                                cudaStream_t st);
+// Runs problems probs[order[i]] (order null: probs[i]), first <= i < last, on persistent CTAs;
+// `order` sorts by decreasing n.  `large`: one CTA per SM (problems of more than
+// BATCH_LARGE_N rows), else two smaller ones.  `next` is a device counter the launch zeroes
+// first.  A null order may be in any order, of any sizes.
+cudaError_t batch_factor_launch(bool large, const BatchProblem *probs, int first, int last, const int *order, int *next,
+                                int sms, cudaStream_t st);
 
 } // namespace pg

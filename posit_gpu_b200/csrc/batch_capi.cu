@@ -53,35 +53,64 @@ extern "C" int posit_batch_plan_create(const posit_batch_problem *probs, int npr
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    p->ctas = sms * 8;
+    p->ctas = sms;
     // largest problems first (work grows like n^3)
     std::vector<int> order(nprob);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return probs[a].n > probs[b].n; });
+    int nlarge = 0;
+    while (nlarge < nprob && probs[order[nlarge]].n > pg::BATCH_LARGE_N)
+        ++nlarge;
     cudaError_t e = cudaMalloc((void **)&p->d_probs, sizeof(pg::BatchProblem) * (nprob > 0 ? nprob : 1));
     if (e == cudaSuccess)
         e = cudaMalloc(&p->d_order, sizeof(int) * (nprob > 0 ? nprob : 1));
     if (e == cudaSuccess)
-        e = cudaMalloc(&p->d_next, sizeof(int));
+        e = cudaMalloc(&p->d_next, 2 * sizeof(int));
     if (e == cudaSuccess && nprob > 0)
         e = cudaMemcpy(p->d_probs, probs, sizeof(pg::BatchProblem) * nprob, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && nprob > 0)
         e = cudaMemcpy(p->d_order, order.data(), sizeof(int) * nprob, cudaMemcpyHostToDevice);
-    // capture: reset the queue counter, run the persistent kernel
-    cudaStream_t cs = nullptr;
+    // capture: the large problems' persistent kernel and the others', side by side (the small
+    // problems' CTAs move in as SMs run out of large ones)
+    cudaStream_t cs = nullptr, side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     if (e == cudaSuccess)
         e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+        e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+        e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+        e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
     if (e == cudaSuccess) {
         e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            cudaError_t le = pg::batch_factor_launch(reinterpret_cast<pg::BatchProblem *>(p->d_probs), nprob,
-                                                     reinterpret_cast<int *>(p->d_order), p->d_next, p->ctas, cs);
+            const auto *d = reinterpret_cast<pg::BatchProblem *>(p->d_probs);
+            const auto *o = reinterpret_cast<int *>(p->d_order);
+            cudaError_t le = cudaEventRecord(fork, cs);
+            if (le == cudaSuccess)
+                le = cudaStreamWaitEvent(side, fork, 0);
+            if (le == cudaSuccess)
+                le = pg::batch_factor_launch(true, d, 0, nlarge, o, p->d_next, p->ctas, cs);
+            if (le == cudaSuccess)
+                le = pg::batch_factor_launch(false, d, nlarge, nprob, o, p->d_next + 1, p->ctas, side);
+            if (le == cudaSuccess)
+                le = cudaEventRecord(join, side);
+            if (le == cudaSuccess)
+                le = cudaStreamWaitEvent(cs, join, 0);
             e = cudaStreamEndCapture(cs, &p->graph);
             if (e == cudaSuccess)
                 e = le;
         }
-        cudaStreamDestroy(cs);
     }
+    if (cs)
+        cudaStreamDestroy(cs);
+    if (side)
+        cudaStreamDestroy(side);
+    if (fork)
+        cudaEventDestroy(fork);
+    if (join)
+        cudaEventDestroy(join);
     if (e == cudaSuccess)
         e = cudaGraphInstantiate(&p->exec, p->graph, 0);
     if (e != cudaSuccess) {

@@ -222,7 +222,8 @@ __global__ void __launch_bounds__(TILE_THREADS, MIN_CTAS_PER_SM)
         kt_stop = kt;
         const bool arrived = mbar_wait_bounded(&full[s], parity);
         const double *as = stages + (size_t)s * NBLK * BLK_DBL;
-        tile_steps<TM, TN, BLK, 8>(acc, as, as + (TM / 2) * BLK_DBL, tile_step_count<8>(k - kt * BK), tab, tx, ty, slow);
+        tile_steps<8>(acc, as, as + (TM / 2) * BLK_DBL, tile_step_count<8>(k - kt * BK), tab, tx, ty,
+                      BlockedOps<BLK>{}, slow);
         // every thread is done with stage s before it is refilled
         bad = __syncthreads_or(!arrived) != 0;
         if (bad)

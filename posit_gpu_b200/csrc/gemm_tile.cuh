@@ -126,32 +126,39 @@ __device__ __forceinline__ double step_any(double c, double t, double a, const u
     return r;
 }
 
-// The operands of step l: as = [TM_/2][16][LD], ts = [TN_/2][16][LD], LD >= 32 doubles per
-// step of a block.
-template <int TM_, int TN_, int LD>
-__device__ __forceinline__ void load_operands(const double *as, const double *ts, int l, int tx, int ty,
+// Where a tile's operands lie in shared memory: as = [TM_/2 blocks][step][32], ts likewise.
+template <int LD> // a block's steps LD doubles apart, its blocks after one another
+struct BlockedOps {
+    static constexpr bool NEG = false;
+    __device__ __forceinline__ int a(int q, int l) const { return q * BK * LD + l * LD; }
+    __device__ __forceinline__ int t(int q, int l) const { return q * BK * LD + l * LD; }
+};
+
+// The operands of step l.
+template <int TM_, int TN_, class Ops>
+__device__ __forceinline__ void load_operands(const double *as, const double *ts, int l, int tx, int ty, Ops ops,
                                               double (&a)[TM_], double (&t)[TN_])
 {
 #pragma unroll
     for (int q = 0; q < TM_ / 2; ++q) {
-        const double2 v = *reinterpret_cast<const double2 *>(as + q * BK * LD + l * LD + 2 * tx);
+        const double2 v = *reinterpret_cast<const double2 *>(as + ops.a(q, l) + 2 * tx);
         a[2 * q] = v.x;
         a[2 * q + 1] = v.y;
     }
 #pragma unroll
     for (int q = 0; q < TN_ / 2; ++q) {
-        const double2 v = *reinterpret_cast<const double2 *>(ts + q * BK * LD + l * LD + 2 * ty);
-        t[2 * q] = v.x;
-        t[2 * q + 1] = v.y;
+        const double2 v = *reinterpret_cast<const double2 *>(ts + ops.t(q, l) + 2 * ty);
+        t[2 * q] = Ops::NEG ? -v.x : v.x;
+        t[2 * q + 1] = Ops::NEG ? -v.y : v.y;
     }
 }
 
-template <int TM_, int TN_, int LD>
+template <int TM_, int TN_, class Ops>
 __device__ __forceinline__ void step_fast(double (&acc)[TM_][TN_], const double *as, const double *ts, int l,
-                                          const unsigned char *tab, int tx, int ty)
+                                          const unsigned char *tab, int tx, int ty, Ops ops)
 {
     double a[TM_], t[TN_];
-    load_operands<TM_, TN_, LD>(as, ts, l, tx, ty, a, t);
+    load_operands<TM_, TN_>(as, ts, l, tx, ty, ops, a, t);
 #pragma unroll
     for (int i = 0; i < TM_; ++i)
 #pragma unroll
@@ -165,9 +172,9 @@ __device__ __forceinline__ void step_fast(double (&acc)[TM_][TN_], const double 
 // is.  `slow` is the warp's state: after a tile with a step outside the fast window the next
 // one is done step by step with a test, until a tile has none (data of a wide dynamic range
 // has such steps everywhere, and doing those tiles twice would not pay).
-template <int TM_, int TN_, int LD, int UNR_>
+template <int UNR_, int TM_, int TN_, class Ops>
 __device__ __forceinline__ void tile_steps(double (&acc)[TM_][TN_], const double *as, const double *ts, int steps,
-                                           const unsigned char *tab, int tx, int ty, bool &slow)
+                                           const unsigned char *tab, int tx, int ty, Ops ops, bool &slow)
 {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     if (!slow) {
@@ -181,7 +188,7 @@ __device__ __forceinline__ void tile_steps(double (&acc)[TM_][TN_], const double
         for (int l0 = 0; l0 < steps; l0 += UNR_) {
 #pragma unroll
             for (int l = 0; l < UNR_; ++l)
-                step_fast<TM_, TN_, LD>(acc, as, ts, l0 + l, tab, tx, ty);
+                step_fast<TM_, TN_>(acc, as, ts, l0 + l, tab, tx, ty, ops);
         }
         bool any = false;
 #pragma unroll
@@ -202,7 +209,7 @@ __device__ __forceinline__ void tile_steps(double (&acc)[TM_][TN_], const double
 #pragma unroll 1
     for (int l = 0; l < steps; ++l) {
         double a[TM_], t[TN_];
-        load_operands<TM_, TN_, LD>(as, ts, l, tx, ty, a, t);
+        load_operands<TM_, TN_>(as, ts, l, tx, ty, ops, a, t);
 #pragma unroll
         for (int i = 0; i < TM_; ++i)
 #pragma unroll
@@ -419,7 +426,7 @@ __device__ __forceinline__ void fused_tile(const TileArgs &P, int mt, int nt, un
             tile_load<TN_>(rb, P.B, P.ldb, !P.notb, col0, P.n, (kt + 1) * BK, P.k);
         }
         __syncthreads(); // this buffer is full; every thread is done with the other one
-        tile_steps<TM_, TN_, TILE_LD, UNR>(acc, b, b + ABUF, tile_step_count<UNR>(P.k - kt * BK), tab, tx, ty, slow);
+        tile_steps<UNR>(acc, b, b + ABUF, tile_step_count<UNR>(P.k - kt * BK), tab, tx, ty, BlockedOps<TILE_LD>{}, slow);
     }
     tile_finish<TRI, TM_, TN_>(dot, acc, nar_bits, row0, col0, P.m, P.n, P.alpha, P.beta, P.C, P.ldc, tx, ty,
                                [&](int i, int j) { return (rnar[i] | cnar[j]) != 0; });

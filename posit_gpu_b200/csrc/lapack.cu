@@ -898,41 +898,11 @@ __global__ void __launch_bounds__(32) trsm_llt_kernel(const uint32_t *__restrict
 // NaR travels as NaN; a NaR term sets its row's flag and is replaced by 0.
 constexpr int LTX_THREADS = 128;
 
-// The solution column in shared memory: FP64, or patterns where the columns are long.
-struct LtxCol64 {
-    double *b;
-    static constexpr size_t BYTES = 8;
-    __device__ double get(int k) const { return b[k]; }
-    __device__ void set(int k, double v) const { b[k] = v; }
-};
-struct LtxCol32 {
-    uint32_t *b;
-    static constexpr size_t BYTES = 4;
-    __device__ double get(int k) const { return p32_to_double(b[k]); }
-    __device__ void set(int k, double v) const { b[k] = p32_from_double_exact(v); }
-};
-template <class Terms>
-struct LtxColOf;
-template <>
-struct LtxColOf<ChainTerms64> {
-    using Col = LtxCol64;
-};
-template <>
-struct LtxColOf<ChainTerms32> {
-    using Col = LtxCol32;
-};
 template <class Terms>
 static size_t ltx_smem_bytes(int m)
 {
     return 2 * Terms::bytes(m) + (size_t)m * LtxColOf<Terms>::Col::BYTES;
 }
-
-// What warp 0 needs of a row besides its terms.
-struct LtxRow {
-    double diag, recip; // a_ii and fl(1/a_ii)
-    double near;        // the coefficient of the b finished last
-    int nar;            // a term was NaR
-};
 
 template <class Terms, bool UPPER>
 __global__ void __launch_bounds__(LTX_THREADS) trsm_ltx_kernel(const uint32_t *__restrict__ L, size_t ldl,
@@ -941,105 +911,16 @@ __global__ void __launch_bounds__(LTX_THREADS) trsm_ltx_kernel(const uint32_t *_
 {
     extern __shared__ __align__(16) unsigned char smem_ltx[];
     __shared__ LtxRow s_row[2];
-    using Col = typename LtxColOf<Terms>::Col;
     if (info && *info != 0) // a factorization stopped before this solve
         return;
-    auto terms = [&](int half) {
-        Terms q;
-        q.q = reinterpret_cast<decltype(q.q)>(smem_ltx + half * Terms::bytes(m));
-        return q;
-    };
-    Col s_b;
-    s_b.b = reinterpret_cast<decltype(s_b.b)>(smem_ltx + 2 * Terms::bytes(m));
+    typename LtxColOf<Terms>::Col x;
+    x.b = reinterpret_cast<decltype(x.b)>(smem_ltx + 2 * Terms::bytes(m));
     uint32_t *bcol = B + (size_t)blockIdx.x * ldb;
-    const int tid = threadIdx.x;
-    for (int k = tid; k < m; k += LTX_THREADS)
-        s_b.set(k, p32_to_double(bcol[k]));
-    // Terms outside a row's range are zero for warp_chain: rows grow, so what no earlier row
-    // wrote is still this.
-    for (int k = tid; k < (int)(2 * Terms::bytes(m) / sizeof(typename Terms::Word)); k += LTX_THREADS)
-        reinterpret_cast<typename Terms::Word *>(smem_ltx)[k] = 0;
-    auto row_of = [&](int step) { return UPPER ? step : m - 1 - step; };
-    // the row's diagonal and nearest coefficient
-    auto head = [&](int step) {
-        const int i = row_of(step);
-        const uint32_t *li = L + (size_t)i * ldl;
-        LtxRow &r = s_row[step & 1];
-        r.diag = unit ? 1.0 : p32_to_double(li[i]);
-        r.recip = 1.0 / r.diag;
-        r.near = step > 0 ? p32_to_double(li[UPPER ? i - 1 : i + 1]) : 0.0;
-    };
-    if (tid < 2)
-        s_row[tid].nar = 0;
-    if (tid == 32)
-        head(0);
-    __syncthreads();
-    double x = 0.0; // the b finished last (warp 0)
-    for (int step = 0; step < m; ++step) {
-        const int i = row_of(step), cur = step & 1;
-        if (tid < 32) {
-            const LtxRow r = s_row[cur];
-            double t = s_b.get(i);
-            bool nar = t != t || r.nar;
-            double near = 0.0; // -a*b of the b just finished
-            if (step > 0) {
-                near = f64_posit_mul_checked(-x, r.near, F64ConstComputed{});
-                if (near != near) {
-                    nar = true;
-                    near = 0.0;
-                }
-            }
-            if (nar)
-                t = 0.0;
-            if (!UPPER && step > 0) {
-                t = f64_round_any(f64_add(t, near));
-                t = warp_chain(t, terms(cur), i + 2, m);
-            }
-            if (UPPER && step > 0) {
-                t = warp_chain(t, terms(cur), 0, i - 1);
-                t = f64_round_any(f64_add(t, near));
-            }
-            x = nar ? p32_to_double(P32_NAR) : t;
-            if (!unit)
-                x = f64_posit_div(x, r.diag, r.recip);
-            __syncwarp(); // every lane has read the row
-            if (tid == 0) {
-                s_b.set(i, x);
-                s_row[cur].nar = 0;
-            }
-        } else if (step + 1 < m) {
-            // the terms of the next row whose b_k are final: k = i+1 .. m-1 of row i-1
-            // (lower), k = 0 .. i-1 of row i+1 (upper)
-            const int kbeg = UPPER ? 0 : i + 1, kend = UPPER ? i : m;
-            const uint32_t *lp = L + (size_t)row_of(step + 1) * ldl;
-            if (tid == 32)
-                head(step + 1);
-            const Terms q = terms(cur ^ 1);
-            int nar = 0;
-            constexpr int P = LTX_THREADS - 32, U = 8; // U loads in flight per thread
-            for (int k = kbeg + (tid - 32); k < kend; k += U * P) {
-                uint32_t l[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    l[u] = k + u * P < kend ? lp[k + u * P] : 0u;
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if (k + u * P < kend) {
-                        double v = f64_posit_mul_checked(-s_b.get(k + u * P), p32_to_double(l[u]), F64ConstComputed{});
-                        if (v != v) {
-                            nar = 1;
-                            v = 0.0;
-                        }
-                        q.set(k + u * P, v);
-                    }
-            }
-            if (nar)
-                s_row[cur ^ 1].nar = 1;
-        }
-        __syncthreads();
-    }
-    for (int k = tid; k < m; k += LTX_THREADS)
-        bcol[k] = p32_from_double_exact(s_b.get(k));
+    for (int k = threadIdx.x; k < m; k += LTX_THREADS)
+        x.set(k, p32_to_double(bcol[k]));
+    block_ltx_solve<LTX_THREADS, UPPER, Terms>(L, ldl, x, m, unit, smem_ltx, s_row);
+    for (int k = threadIdx.x; k < m; k += LTX_THREADS)
+        bcol[k] = p32_from_double_exact(x.get(k));
 }
 
 // ---------------------------------------------------------------------------

@@ -358,8 +358,7 @@ int launch_batched(posit_server *s, Unit *u)
     int *d_next = reinterpret_cast<int *>(static_cast<unsigned char *>(dd) + desc_bytes);
     cudaError_t e = cudaMemcpyAsync(dd, L.h_desc, sizeof(pg::BatchProblem) * np, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
-        e = pg::batch_factor_launch(static_cast<pg::BatchProblem *>(dd), np, nullptr, d_next,
-                                    std::min(np, s->sms * 8), st);
+        e = pg::batch_factor_launch(false, static_cast<pg::BatchProblem *>(dd), 0, np, nullptr, d_next, s->sms, st);
     cudaFreeAsync(dd, st);
     if (e != cudaSuccess)
         return fail_code(e);

@@ -425,7 +425,8 @@ constexpr int CHAIN_WINDOW_MIN = 64; // addends left for a window to pay
 // long for that): packed.
 struct ChainTerms64 {
     double *q;
-    static __host__ __device__ size_t bytes(int n) { return (size_t)((n + 15) / 16) * 18 * sizeof(double); }
+    static constexpr int GROUP_DOUBLES = 18;
+    static __host__ __device__ size_t bytes(int n) { return (size_t)((n + 15) / 16) * GROUP_DOUBLES * sizeof(double); }
     using Word = double;
     __device__ static int at(int k) { return k + (k >> 4) * 2; }
     __device__ void set(int k, double v) const { q[at(k)] = v; }
@@ -610,6 +611,191 @@ __device__ double warp_chain(double t, Q q, int pos, int end)
         }
     }
     return t;
+}
+
+// L^-T b for one right-hand side by one warp (Rtrsm('L', 'L', 'T', 'N'), as llt_chain): the
+// terms of a row, one per lane and stretch of 32, then their chain.  x (shared memory, the
+// column as FP64, NaN for NaR) is overwritten; `q` holds m terms, its buffer is cleared here.
+template <class Q>
+__device__ void warp_llt_solve(const uint32_t *__restrict__ L, size_t ldl, double *x, int m, Q q)
+{
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    constexpr int PRE = 8; // a row's first coefficients, loaded while the row before it is summed
+    const int lane = threadIdx.x & 31;
+    for (int k = lane; k < (int)(Q::bytes(m) / sizeof(typename Q::Word)); k += 32)
+        q.q[k] = 0;
+    __syncwarp();
+    uint32_t pre[PRE], dn = L[(m - 1) + (size_t)(m - 1) * ldl];
+#pragma unroll
+    for (int j = 0; j < PRE; ++j)
+        pre[j] = 0;
+    for (int i = m - 1; i >= 0; --i) {
+        const uint32_t *li = L + (size_t)i * ldl;
+        bool nar = false;
+        auto term = [&](int k, uint32_t l) {
+            double v = f64_posit_mul_checked(-x[k], p32_to_double(l), F64ConstComputed{});
+            if (v != v) {
+                nar = true;
+                v = 0.0;
+            }
+            q.set(k, v);
+        };
+#pragma unroll
+        for (int j = 0; j < PRE; ++j)
+            if (i + 1 + lane + 32 * j < m)
+                term(i + 1 + lane + 32 * j, pre[j]);
+#pragma unroll 1
+        for (int k = i + 1 + lane + 32 * PRE; k < m; k += 32)
+            term(k, li[k]);
+        const double d = p32_to_double(dn);
+        if (i > 0) {
+            dn = li[-(ptrdiff_t)ldl + i - 1];
+#pragma unroll
+            for (int j = 0; j < PRE; ++j) {
+                const int k = i + lane + 32 * j;
+                pre[j] = k < m ? li[k - (ptrdiff_t)ldl] : 0u;
+            }
+        }
+        const double rc = 1.0 / d;
+        nar = __any_sync(FULL, nar) || x[i] != x[i];
+        __syncwarp(); // the terms are in place
+        double t = nar ? 0.0 : warp_chain(x[i], q, i + 1, m);
+        t = f64_posit_div(nar ? p32_to_double(P32_NAR) : t, d, rc);
+        __syncwarp();
+        if (lane == 0)
+            x[i] = t;
+        __syncwarp();
+    }
+}
+
+// The solution column in shared memory: FP64, or patterns where the columns are long.
+struct LtxCol64 {
+    double *b;
+    static constexpr size_t BYTES = 8;
+    __device__ double get(int k) const { return b[k]; }
+    __device__ void set(int k, double v) const { b[k] = v; }
+};
+struct LtxCol32 {
+    uint32_t *b;
+    static constexpr size_t BYTES = 4;
+    __device__ double get(int k) const { return p32_to_double(b[k]); }
+    __device__ void set(int k, double v) const { b[k] = p32_from_double_exact(v); }
+};
+template <class Terms>
+struct LtxColOf;
+template <>
+struct LtxColOf<ChainTerms64> {
+    using Col = LtxCol64;
+};
+template <>
+struct LtxColOf<ChainTerms32> {
+    using Col = LtxCol32;
+};
+// What the adding warp needs of a row besides its terms.
+struct LtxRow {
+    double diag, recip; // a_ii and fl(1/a_ii)
+    double near;        // the coefficient of the b finished last
+    int nar;            // a term was NaR
+};
+
+// L^-T x (UPPER: U^-T x) for one right-hand side by a block of NT threads: warp 0 sums a row's
+// terms (warp_chain) while the others compute the next row's, all whose x_k are final, into
+// the other half of a double buffer, and its diagonal's reciprocal; the term of the x_k just
+// finished (the first one, UPPER: the last) warp 0 forms itself.  `buf`: 2 * Terms::bytes(m).
+// NaR travels as NaN; a NaR term sets its row's flag and is replaced by 0.
+template <int NT, bool UPPER, class Terms, class Col>
+__device__ __forceinline__ void block_ltx_solve(const uint32_t *__restrict__ L, size_t ldl, Col x, int m, bool unit,
+                                                unsigned char *buf, LtxRow *s_row)
+{
+    const int tid = threadIdx.x;
+    auto terms = [&](int half) {
+        Terms q;
+        q.q = reinterpret_cast<decltype(q.q)>(buf + half * Terms::bytes(m));
+        return q;
+    };
+    // Terms outside a row's range are zero for warp_chain: rows grow, so what no earlier row
+    // wrote is still this.
+    for (int k = tid; k < (int)(2 * Terms::bytes(m) / sizeof(typename Terms::Word)); k += NT)
+        reinterpret_cast<typename Terms::Word *>(buf)[k] = 0;
+    auto row_of = [&](int step) { return UPPER ? step : m - 1 - step; };
+    // the row's diagonal and nearest coefficient
+    auto head = [&](int step) {
+        const int i = row_of(step);
+        const uint32_t *li = L + (size_t)i * ldl;
+        LtxRow &r = s_row[step & 1];
+        r.diag = unit ? 1.0 : p32_to_double(li[i]);
+        r.recip = 1.0 / r.diag;
+        r.near = step > 0 ? p32_to_double(li[UPPER ? i - 1 : i + 1]) : 0.0;
+    };
+    if (tid < 2)
+        s_row[tid].nar = 0;
+    if (tid == 32)
+        head(0);
+    __syncthreads();
+    double last = 0.0; // the x_k finished last (warp 0)
+    for (int step = 0; step < m; ++step) {
+        const int i = row_of(step), cur = step & 1;
+        if (tid < 32) {
+            const LtxRow r = s_row[cur];
+            double t = x.get(i);
+            bool nar = t != t || r.nar;
+            double near = 0.0; // -a*x_k of the one just finished
+            if (step > 0) {
+                near = f64_posit_mul_checked(-last, r.near, F64ConstComputed{});
+                if (near != near) {
+                    nar = true;
+                    near = 0.0;
+                }
+            }
+            if (nar)
+                t = 0.0;
+            if (!UPPER && step > 0) {
+                t = f64_round_any(f64_add(t, near));
+                t = warp_chain(t, terms(cur), i + 2, m);
+            }
+            if (UPPER && step > 0) {
+                t = warp_chain(t, terms(cur), 0, i - 1);
+                t = f64_round_any(f64_add(t, near));
+            }
+            last = nar ? p32_to_double(P32_NAR) : t;
+            if (!unit)
+                last = f64_posit_div(last, r.diag, r.recip);
+            __syncwarp(); // every lane has read the row
+            if (tid == 0) {
+                x.set(i, last);
+                s_row[cur].nar = 0;
+            }
+        } else if (step + 1 < m) {
+            // the terms of the next row whose x_k are final: k = i+1 .. m-1 of row i-1
+            // (lower), k = 0 .. i-1 of row i+1 (upper)
+            const int kbeg = UPPER ? 0 : i + 1, kend = UPPER ? i : m;
+            const uint32_t *lp = L + (size_t)row_of(step + 1) * ldl;
+            if (tid == 32)
+                head(step + 1);
+            const Terms q = terms(cur ^ 1);
+            int nar = 0;
+            constexpr int P = NT - 32, U = 8; // U loads in flight per thread
+            for (int k = kbeg + (tid - 32); k < kend; k += U * P) {
+                uint32_t l[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    l[u] = k + u * P < kend ? lp[k + u * P] : 0u;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (k + u * P < kend) {
+                        double v = f64_posit_mul_checked(-x.get(k + u * P), p32_to_double(l[u]), F64ConstComputed{});
+                        if (v != v) {
+                            nar = 1;
+                            v = 0.0;
+                        }
+                        q.set(k + u * P, v);
+                    }
+            }
+            if (nar)
+                s_row[cur ^ 1].nar = 1;
+        }
+        __syncthreads();
+    }
 }
 #endif
 
