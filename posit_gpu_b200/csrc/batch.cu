@@ -61,7 +61,8 @@ struct BatchShared {
 
 // The panel's operands in a trailing tile: as = panel rows, ts = U12 or the panel again.
 struct PanelOps {
-    static constexpr bool NEG = true; // c + (-u)*l
+    static constexpr bool NEG = true;  // c + (-u)*l
+    static constexpr bool NANS = true; // NaR travels as NaN
     int pl, ul;
     __device__ __forceinline__ int a(int q, int l) const { return l * pl + q * BLK; }
     __device__ __forceinline__ int t(int q, int l) const { return l * ul + q * BLK; }

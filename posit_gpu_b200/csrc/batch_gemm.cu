@@ -46,7 +46,7 @@ __device__ __forceinline__ void batch_tile(const BatchGemmDesc &P, int mt, int n
 {
     const TileArgs T{P.nota != 0, P.notb != 0, P.m,   P.n, P.k,           P.alpha, P.beta,
                      P.A,         (size_t)P.lda, P.B, (size_t)P.ldb, P.C, (size_t)P.ldc};
-    fused_tile<TRI_FULL, TM_, TN_>(T, mt, nt, smem);
+    fused_tile<TRI_FULL, TM_, TN_, false>(T, mt, nt, smem);
 }
 
 __global__ void __launch_bounds__(BG_THREADS, BATCH_GEMM_CTAS_PER_SM)

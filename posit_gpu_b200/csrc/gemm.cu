@@ -196,6 +196,8 @@ __global__ void __launch_bounds__(TILE_THREADS, MIN_CTAS_PER_SM)
         for (int s = 0; s < STAGES; ++s)
             mbar_init(&full[s], 1);
         mbar_fence_init();
+        for (int s = 0; s < STAGES && s < KT; ++s)
+            fetch(s, s);
     }
     step_tables_fill(tab, tid, TILE_THREADS);
     // blocks that do not exist hold 1.0 throughout: their lanes stay on the fast path
@@ -205,15 +207,18 @@ __global__ void __launch_bounds__(TILE_THREADS, MIN_CTAS_PER_SM)
             if (q < TM / 2 ? q >= na : q - TM / 2 >= nbk)
                 stages[e] = 1.0;
         }
-    __syncthreads();
-    if (tid == 0)
-        for (int s = 0; s < STAGES && s < KT; ++s)
-            fetch(s, s);
-
+    __syncthreads(); // the barriers are initialised, the tables filled
     double acc[TM][TN];
     uint32_t nar_bits;
-    tile_start<TM, TN>(dot, acc, nar_bits, mt * BM, nt * BN, m, n, beta, C, ldc, tx, ty);
+    {
+        uint32_t cu[TM][TN];
+        tile_load_c<TM, TN>(!dot && beta != 0, cu, mt * BM, nt * BN, m, n, C, ldc, tx, ty);
+        tile_start<TM, TN>(dot, acc, nar_bits, beta, cu);
+    }
 
+    // One block barrier per k tile, although a barrier per stage would do: it keeps the warps
+    // in step, and with them the unrolled steps (14 KB) in the instruction cache (warps
+    // that ran on by themselves took 333 ms for 8192^3 instead of 285).
     bool bad = false, slow = false;
     int kt_stop = 0, s = 0;
     uint32_t parity = 0;
@@ -222,7 +227,7 @@ __global__ void __launch_bounds__(TILE_THREADS, MIN_CTAS_PER_SM)
         kt_stop = kt;
         const bool arrived = mbar_wait_bounded(&full[s], parity);
         const double *as = stages + (size_t)s * NBLK * BLK_DBL;
-        tile_steps<8>(acc, as, as + (TM / 2) * BLK_DBL, tile_step_count<8>(k - kt * BK), tab, tx, ty,
+        tile_steps<4>(acc, as, as + (TM / 2) * BLK_DBL, tile_step_count<4>(k - kt * BK), tab, tx, ty,
                       BlockedOps<BLK>{}, slow);
         // every thread is done with stage s before it is refilled
         bad = __syncthreads_or(!arrived) != 0;
@@ -264,8 +269,7 @@ __global__ void __launch_bounds__(TILE_THREADS, TM_ * TN_ >= 16 ? 2 : (TM_ * TN_
     if (TRI == TRI_UPPER && (int)(blockIdx.x * BM) > (int)(blockIdx.y * BN + BN - 1))
         return;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    step_tables_fill(smem_raw, threadIdx.x, TILE_THREADS);
-    fused_tile<TRI, TM_, TN_>(P, blockIdx.x, blockIdx.y, smem_raw);
+    fused_tile<TRI, TM_, TN_, true>(P, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 // C <- 0 or beta*C (alpha == 0, Rgemm.cpp:142-156; NN/NT with k == 0, Rgemm.cpp:169-177), or,
@@ -389,7 +393,9 @@ GemmRoute gemm_route(bool nota, bool notb, int m, int n, int k, const uint32_t *
          spans_overlap(C, span(m, n, ldc), B, notb ? span(k, n, ldb) : span(n, k, ldb))))
         return GEMM_STAGED;
     const long long t44 = ceil_div(m, 64) * ceil_div(n, 64), t42 = ceil_div(m, 64) * ceil_div(n, 32);
-    if (t44 >= 2 * SM_COUNT && (double)m * n * k >= GEMM_STAGED_MIN_MADS)
+    // From 2^24 multiply-adds on 100 tiles the second launch is worth it: 1024 x 1024 x 24 39.9
+    // against 44.4 us fused, 2048^2 x 32 121 / 125, 1000 x 1000 x 500 356 / 418, 700^3 272 / 301.
+    if (t44 >= GEMM_STAGED_MIN_TILES && (double)m * n * k >= GEMM_STAGED_MIN_MADS)
         return GEMM_STAGED;
     return t44 >= 2 * SM_COUNT ? GEMM_FUSED_64x64 : (t42 >= SM_COUNT ? GEMM_FUSED_64x32 : GEMM_FUSED_32x32);
 }

@@ -92,10 +92,11 @@ struct OutsideTable {
 };
 static __device__ const OutsideTable g_outside_table;
 
-// x rounded as f64_round_outside, by the table.
+// x rounded as f64_round_outside, by the table.  NANS: x may be NaN, and stays it.
+template <bool NANS>
 __device__ __forceinline__ double round_outside_tab(double x)
 {
-    if (x != x)
+    if (NANS && x != x)
         return x;
     const uint64_t b = f64_bits(x) & 0x7FFFFFFFFFFFFFFFull;
     const int ex = (int)(b >> 52) - 1023;
@@ -106,13 +107,14 @@ __device__ __forceinline__ double round_outside_tab(double x)
 
 // The same step for any operands (f64_posit_mac_exact with its tables); `out` is set when the
 // product or the sum was outside the fast window.
+template <bool NANS>
 __device__ __forceinline__ double step_any(double c, double t, double a, const unsigned char *tab, bool &out)
 {
     const double p = f64_mul(t, a);
     const double Cp = *reinterpret_cast<const double *>(tab + ((f64_hi(p) >> 17) & 0x3FF8));
     double q = f64_add(f64_fma(t, a, Cp), -Cp);
     if (q != q) {
-        q = round_outside_tab(p);
+        q = round_outside_tab<NANS>(p);
         out = true;
     }
     const double s = f64_add(c, q);
@@ -120,7 +122,7 @@ __device__ __forceinline__ double step_any(double c, double t, double a, const u
         f64_from_hi(*reinterpret_cast<const uint32_t *>(tab + STEP_TAB_P_BYTES + ((f64_hi(s) >> 18) & 0x1FFC)));
     double r = f64_add(f64_add(s, Cs), -Cs);
     if (r != r) {
-        r = round_outside_tab(s);
+        r = round_outside_tab<NANS>(s);
         out = true;
     }
     return r;
@@ -129,7 +131,8 @@ __device__ __forceinline__ double step_any(double c, double t, double a, const u
 // Where a tile's operands lie in shared memory: as = [TM_/2 blocks][step][32], ts likewise.
 template <int LD> // a block's steps LD doubles apart, its blocks after one another
 struct BlockedOps {
-    static constexpr bool NEG = false;
+    static constexpr bool NEG = false;  // t is taken negated
+    static constexpr bool NANS = false; // operands and accumulators may be NaN (NaR)
     __device__ __forceinline__ int a(int q, int l) const { return q * BK * LD + l * LD; }
     __device__ __forceinline__ int t(int q, int l) const { return q * BK * LD + l * LD; }
 };
@@ -167,8 +170,8 @@ __device__ __forceinline__ void step_fast(double (&acc)[TM_][TN_], const double 
 }
 
 // The k-steps of a tile: one p32_mul and one p32_add per k and accumulator, in k order; the
-// accumulators and operands are posit32 values held in FP64 (no NaR: the callers carry it
-// in flags).  `steps` is a multiple of UNR_; steps past k have t = 0, which leaves c as it
+// accumulators and operands are posit32 values held in FP64 (no NaR unless Ops::NANS: the
+// callers carry it in flags).  `steps` is a multiple of UNR_; steps past k have t = 0, which leaves c as it
 // is.  `slow` is the warp's state: after a tile with a step outside the fast window the next
 // one is done step by step with a test, until a tile has none (data of a wide dynamic range
 // has such steps everywhere, and doing those tiles twice would not pay).
@@ -214,7 +217,7 @@ __device__ __forceinline__ void tile_steps(double (&acc)[TM_][TN_], const double
         for (int i = 0; i < TM_; ++i)
 #pragma unroll
             for (int j = 0; j < TN_; ++j)
-                acc[i][j] = step_any(acc[i][j], t[j], a[i], tab, any);
+                acc[i][j] = step_any<Ops::NANS>(acc[i][j], t[j], a[i], tab, any);
     }
     slow = __any_sync(FULL, any);
 }
@@ -234,7 +237,7 @@ __device__ __forceinline__ double mac_any(double c, double t, double a, const un
     double r = step_one(c, t, a, tab);
     if (r != r) {
         bool out;
-        r = step_any(c, t, a, tab, out);
+        r = step_any<true>(c, t, a, tab, out);
     }
     return r;
 }
@@ -243,7 +246,7 @@ __device__ __forceinline__ double mul_any(double x, double y, const unsigned cha
     const double p = f64_mul(x, y);
     const double C = *reinterpret_cast<const double *>(tab + ((f64_hi(p) >> 17) & 0x3FF8));
     const double q = f64_add(f64_fma(x, y, C), -C);
-    return q == q ? q : round_outside_tab(p);
+    return q == q ? q : round_outside_tab<true>(p);
 }
 
 // alpha*b_lj as the NN/NT order rounds it (Rgemm.cpp:180, 222), b in FP64; NaN for NaR.
@@ -331,28 +334,38 @@ __device__ __forceinline__ void tile_store(const uint32_t (&raw)[TQ_], double *d
     }
 }
 
-// The start values of a tile's accumulators: NN/NT beta*C (Rgemm.cpp:169-177, 211-219), TN/TT
-// zero.  A NaR start value is remembered in nar_bits (the output stays NaR whatever
-// follows) and replaced by 1.0.
+// The entries of C a tile starts from, as patterns: 1.0 outside the matrix and where C is not
+// read.  Loaded ahead of everything else a CTA does; tile_start converts them.
 template <int TM_, int TN_>
-__device__ __forceinline__ void tile_start(bool dot, double (&acc)[TM_][TN_], uint32_t &nar_bits, int row0,
-                                           int col0, int m, int n, uint32_t beta, const uint32_t *C, size_t ldc,
-                                           int tx, int ty)
+__device__ __forceinline__ void tile_load_c(bool reads_c, uint32_t (&u)[TM_][TN_], int row0, int col0, int m, int n,
+                                            const uint32_t *C, size_t ldc, int tx, int ty)
+{
+#pragma unroll
+    for (int i = 0; i < TM_; ++i)
+#pragma unroll
+        for (int j = 0; j < TN_; ++j) {
+            const int row = row0 + own_off(tx, i), col = col0 + own_off(ty, j);
+            u[i][j] = reads_c && row < m && col < n ? C[(size_t)row + (size_t)col * ldc] : P32_ONE;
+        }
+}
+
+// The start values of a tile's accumulators: NN/NT beta*C (Rgemm.cpp:169-177, 211-219; with
+// beta == 0, C is not read), TN/TT zero.  A NaR start value is remembered in nar_bits (the
+// output stays NaR whatever follows) and replaced by 1.0.
+template <int TM_, int TN_>
+__device__ __forceinline__ void tile_start(bool dot, double (&acc)[TM_][TN_], uint32_t &nar_bits, uint32_t beta,
+                                           const uint32_t (&c)[TM_][TN_])
 {
     nar_bits = 0;
 #pragma unroll
     for (int i = 0; i < TM_; ++i) {
 #pragma unroll
         for (int j = 0; j < TN_; ++j) {
-            const int row = row0 + own_off(tx, i), col = col0 + own_off(ty, j);
             uint32_t u = 0;
-            if (!dot && beta != 0) { // Rgemm.cpp:170-173: with beta == 0, C is not read
-                u = P32_ONE;
-                if (row < m && col < n) {
-                    u = C[(size_t)row + (size_t)col * ldc];
-                    if (beta != P32_ONE)
-                        u = pmul(beta, u);
-                }
+            if (!dot && beta != 0) {
+                u = c[i][j];
+                if (beta != P32_ONE)
+                    u = pmul(beta, u);
                 if (u == P32_NAR) {
                     nar_bits |= 1u << (i * TN_ + j);
                     u = P32_ONE;
@@ -391,9 +404,10 @@ __device__ __forceinline__ void tile_finish(bool dot, const double (&acc)[TM_][T
 }
 
 // Tile (mt, nt) of the product, 16*TM_ x 16*TN_ outputs, by 256 threads.  `smem` is laid out
-// as tile_smem_bytes, its tables filled.  The next k tile's patterns are loaded while the
+// as tile_smem_bytes, its tables filled (FILL: here, while the first loads are in flight).  The
+// next k tile's patterns are loaded while the
 // current one is multiplied, converted into the other buffer: one barrier per k tile.
-template <int TRI, int TM_, int TN_>
+template <int TRI, int TM_, int TN_, bool FILL>
 __device__ __forceinline__ void fused_tile(const TileArgs &P, int mt, int nt, unsigned char *smem)
 {
     constexpr int BM_ = 16 * TM_, BN_ = 16 * TN_;
@@ -408,12 +422,15 @@ __device__ __forceinline__ void fused_tile(const TileArgs &P, int mt, int nt, un
     uint32_t ra[TM_], rb[TN_];
     tile_load<TM_>(ra, P.A, P.lda, P.nota, row0, P.m, 0, P.k);
     tile_load<TN_>(rb, P.B, P.ldb, !P.notb, col0, P.n, 0, P.k);
+    double acc[TM_][TN_];
+    uint32_t nar_bits, cu[TM_][TN_];
+    tile_load_c<TM_, TN_>(!dot && P.beta != 0, cu, row0, col0, P.m, P.n, P.C, P.ldc, tx, ty);
     for (int i = tid; i < BM_ + BN_; i += TILE_THREADS)
         rnar[i] = 0;
-    double acc[TM_][TN_];
-    uint32_t nar_bits;
-    tile_start<TM_, TN_>(dot, acc, nar_bits, row0, col0, P.m, P.n, P.beta, P.C, P.ldc, tx, ty);
-    __syncthreads(); // the flags are clear (and, on a CTA's first tile, the tables filled)
+    if (FILL)
+        step_tables_fill(smem, tid, TILE_THREADS);
+    tile_start<TM_, TN_>(dot, acc, nar_bits, P.beta, cu);
+    __syncthreads(); // the flags are clear, the tables filled
     bool slow = false;
     const int KT = (P.k + BK - 1) / BK;
 #pragma unroll 1

@@ -302,7 +302,7 @@ __device__ __forceinline__ void panel_row_update(double *rw, int T, const double
             bool out;
 #pragma unroll 1
             for (int q = 0; q < PANEL_U; ++q)
-                p[q * T] = step_any(p[q * T], -u[c + q], l, tab, out);
+                p[q * T] = step_any<true>(p[q * T], -u[c + q], l, tab, out);
         }
     }
 }
@@ -926,86 +926,7 @@ __global__ void __launch_bounds__(LTX_THREADS) trsm_ltx_kernel(const uint32_t *_
 // ---------------------------------------------------------------------------
 // Cholesky panel (lower)
 // ---------------------------------------------------------------------------
-// Two launches per panel column k, as for LU:
-//   chol_update_kernel  blocks over (rows > k) x (column groups in (k, jb)): l_ik =
-//                       (1/l_kk)*a_ik for the rows below the diagonal block (those of the
-//                       block were scaled by the diagonal step; Rtrsm.cpp:265-268), then
-//                       a_ic += (-l_ck)*l_ik for k < c <= i.  Column k is only read; the
-//                       first column group writes the new l_ik to a scratch column.
-//   chol_diag_kernel    one block: the scratch column into column k, then the diagonal step
-//                       of column k+1: l_kk = sqrt(a_kk) -- a_kk <= 0 in posit order, NaR
-//                       included, stops with info (Rpotrf2.cpp:90-93) -- and
-//                       l_ck = (1/l_kk)*a_ck for the rows c in (k, jb).
-struct CholSync {
-    uint32_t recip; // 1/l_kk of the current column
-};
-
-__global__ void chol_diag_kernel(uint32_t *__restrict__ P, size_t lda, int M, int jb, int k, int row0,
-                                 int *__restrict__ info, CholSync *__restrict__ sync,
-                                 const uint32_t *__restrict__ lcol, int copy_col)
-{
-    __shared__ uint32_t s_recip;
-    __shared__ int s_stop;
-    if (*info != 0)
-        return;
-    if (copy_col >= 0) {
-        uint32_t *pc = P + (size_t)copy_col * lda;
-        for (int r = (copy_col + 1 > jb ? copy_col + 1 : jb) + threadIdx.x; r < M; r += blockDim.x)
-            pc[r] = lcol[r];
-    }
-    if (k >= jb)
-        return;
-    uint32_t *pk = P + (size_t)k * lda;
-    if (threadIdx.x == 0) {
-        uint32_t akk = pk[k];
-        s_stop = (int32_t)akk <= 0;
-        if (s_stop) {
-            *info = row0 + k + 1;
-        } else {
-            uint32_t lkk = psqrt_est(akk);
-            s_recip = pdiv_est(P32_ONE, lkk);
-            pk[k] = lkk;
-            sync->recip = s_recip;
-        }
-    }
-    __syncthreads();
-    if (s_stop)
-        return;
-    for (int c = k + 1 + threadIdx.x; c < jb; c += blockDim.x)
-        pk[c] = pmul(s_recip, pk[c]);
-}
-
-__global__ void __launch_bounds__(PANEL_ROWS) chol_update_kernel(uint32_t *__restrict__ P, size_t lda, int M,
-                                                                 int jb, int k, const int *__restrict__ info,
-                                                                 const CholSync *__restrict__ sync,
-                                                                 uint32_t *__restrict__ lcol)
-{
-    __shared__ double s_l[PANEL_CG]; // -l_ck for this block's columns, FP64
-    if (*info != 0)
-        return;
-    const uint32_t recip = sync->recip;
-    const uint32_t *pk = P + (size_t)k * lda;
-    const int c0 = k + 1 + blockIdx.y * PANEL_CG;
-    if (threadIdx.x < PANEL_CG && c0 + (int)threadIdx.x < jb)
-        s_l[threadIdx.x] = -p32_to_double(pk[c0 + threadIdx.x]); // scaled by the diagonal step
-    __syncthreads();
-    const int i = k + 1 + blockIdx.x * PANEL_ROWS + threadIdx.x;
-    if (i >= M)
-        return;
-    const uint32_t a = pk[i];
-    const uint32_t l = i >= jb ? pmul(recip, a) : a;
-    if (blockIdx.y == 0 && i >= jb)
-        lcol[i] = l;
-    const double dl = p32_to_double(l);
-    const int cn = min(min(PANEL_CG, jb - c0), i - c0 + 1);
-    for (int j = 0; j < cn; ++j) { // a_ic + (-l_ck)*l_i in the FP64 step (posit32.cuh)
-        uint32_t *pc = P + i + (size_t)(c0 + j) * lda;
-        *pc = p32_from_double_exact(f64_posit_mac_checked(p32_to_double(*pc), s_l[j], dl));
-    }
-}
-
-// Lower Cholesky panel of up to 32 columns in one launch, the counterpart of chol_diag_kernel
-// + chol_update_kernel.  Below the diagonal block every row goes its own way once the block is
+// Lower Cholesky panel of up to 32 columns in one launch.  Below the diagonal block every row goes its own way once the block is
 // factored, so each CTA of 128 threads factors the block for itself, in shared memory, and
 // then takes 128 rows through it, one per thread: l_ik = (1/l_kk)*a_ik (Rtrsm.cpp:265-268),
 // a_ic += (-l_ck)*l_ik for c > k, in the FP64 step.  No CTA waits for another.
@@ -1261,8 +1182,8 @@ int tuned_panel_width(bool lu, int n)
     struct Row {
         int n, lu, chol;
     };
-    static const Row rows[] = {{0, 24, 16},    {512, 24, 24},  {1024, 24, 16},   {2048, 24, 24},
-                               {4096, 32, 32}, {8192, 32, 24}, {16384, 128, 128}};
+    static const Row rows[] = {{0, 32, 32},    {512, 32, 32},  {1024, 32, 16},   {2048, 32, 32},
+                               {4096, 32, 32}, {8192, 32, 32}, {16384, 128, 32}};
     int nb = 16;
     for (const Row &r : rows)
         if (n >= r.n)
@@ -1395,10 +1316,8 @@ cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb,
 
 size_t rpotrf_workspace_bytes(int n, int nb)
 {
-    if (nb < 1)
-        nb = 1;
-    int jb = imin(nb, n);
-    return panel_ws_bytes(n) + CHOL_BLOCKS_BYTES + (n > jb ? gemm_workspace_bytes(n - jb, n - jb, jb) : 0);
+    const int jb = imin(imin(imax(nb, 1), CHOL_JB_MAX), n);
+    return CHOL_BLOCKS_BYTES + (n > jb ? gemm_workspace_bytes(n - jb, n - jb, jb) : 0);
 }
 
 // Lower Cholesky (Rpotrf.cpp:124-142 / Rpotrf2.cpp:132-146 order, blocked right-looking).
@@ -1406,39 +1325,30 @@ cudaError_t rpotrf_lower_launch(int n, uint32_t *A, int lda, int nb, int *info, 
 {
     if (nb < 1)
         nb = 1;
-    CholSync *sync = reinterpret_cast<CholSync *>(ws);
-    uint32_t *blocks = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(ws) + panel_ws_bytes(n));
-    uint32_t *lcol = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(ws) + 256);
-    void *gws = reinterpret_cast<unsigned char *>(ws) + panel_ws_bytes(n) + CHOL_BLOCKS_BYTES;
+    // The factor does not depend on the panel width, and wider panels in one launch per
+    // column are slower at every size (n = 1024: 2.5 ms at 32, 11 at 48).
+    nb = imin(nb, CHOL_JB_MAX);
+    uint32_t *blocks = reinterpret_cast<uint32_t *>(ws);
+    void *gws = reinterpret_cast<unsigned char *>(ws) + CHOL_BLOCKS_BYTES;
     const size_t L = (size_t)lda;
     for (int j = 0; j < n; j += nb) {
         const int jb = imin(n - j, nb);
         const int M = n - j;
         uint32_t *P = A + j + (size_t)j * L;
-        uint32_t *lc = lcol + j;
-        if (jb <= CHOL_JB_MAX) {
-            const bool last = j + jb >= n;
-            const size_t smem = chol_panel_smem(jb);
-            cudaError_t e = cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)chol_panel_smem(CHOL_JB_MAX));
-            if (e != cudaSuccess)
-                return e;
-            const int prev_jb = j > 0 ? nb : 0; // nb <= CHOL_JB_MAX for every panel but a lone first one
-            chol_panel_kernel<<<imax(1, (M - jb + CHOL_T - 1) / CHOL_T), CHOL_T, smem, st>>>(
-                P, L, M, jb, j, info, last ? nullptr : blocks + (j / nb & 1) * CHOL_JB_MAX * CHOL_JB_MAX,
-                nb <= CHOL_JB_MAX && j > 0 ? P - (size_t)nb * (L + 1) : nullptr, nb <= CHOL_JB_MAX ? prev_jb : 0,
-                blocks + (j / nb + 1 & 1) * CHOL_JB_MAX * CHOL_JB_MAX);
-        } else {
-            chol_diag_kernel<<<1, 256, 0, st>>>(P, L, M, jb, 0, j, info, sync, lc, -1);
-            for (int k = 0; k < jb; ++k) {
-                chol_update_kernel<<<panel_grid(M, jb, k), PANEL_ROWS, 0, st>>>(P, L, M, jb, k, info, sync, lc);
-                chol_diag_kernel<<<1, 256, 0, st>>>(P, L, M, jb, k + 1, j, info, sync, lc, k);
-            }
-        }
+        const bool last = j + jb >= n, first = j == 0;
+        cudaError_t e = cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)chol_panel_smem(CHOL_JB_MAX));
+        if (e != cudaSuccess)
+            return e;
+        const int turn = j / nb & 1;
+        chol_panel_kernel<<<imax(1, (M - jb + CHOL_T - 1) / CHOL_T), CHOL_T, chol_panel_smem(jb), st>>>(
+            P, L, M, jb, j, info, last ? nullptr : blocks + turn * CHOL_JB_MAX * CHOL_JB_MAX,
+            first ? nullptr : P - (size_t)nb * (L + 1), first ? 0 : nb,
+            blocks + (turn ^ 1) * CHOL_JB_MAX * CHOL_JB_MAX);
         if (j + jb < n) {
             const int nr = n - j - jb;
             const uint32_t *L21 = A + (j + jb) + (size_t)j * L;
-            cudaError_t e = gemm_launch_tri(TRI_LOWER, true, false, nr, nr, jb, 0xC0000000u /* -1 */, L21, lda, L21,
+            e = gemm_launch_tri(TRI_LOWER, true, false, nr, nr, jb, 0xC0000000u /* -1 */, L21, lda, L21,
                                               lda, P32_ONE, A + (j + jb) + (size_t)(j + jb) * L, lda, gws, st, info);
             if (e != cudaSuccess)
                 return e;

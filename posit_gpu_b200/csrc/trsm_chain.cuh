@@ -396,28 +396,21 @@ PG_HD double chain_add_run_reg(double t, Q q, int count)
 // the binade iff w's high word is C's and the low word in (2^fb, 2^(fb+1)) -- 2^fb itself is
 // given up, since the exact sum may have been below it, where the grid is finer.
 //
-//   runs     8 steps are run, then tested at once; where one left the binade they are done
-//            again by the fixed-width step or, across a change of fraction width, by
-//            f64_posit_add.
-//   windows  512 addends at once, 16 per lane.  A step moves M by an amount that depends on
-//            M's parity alone (ties), so a lane's 16 steps are two displacements, found by
-//            running them from an even and from an odd M; a warp scan composes them
-//            (mod 2^32: past the first step that left the binade nothing is used), and each
-//            lane runs its steps again from its true start, tested at once.  The window
-//            ends where the first lane with a step outside starts.
+// So 512 addends are taken at once (a window), 16 per lane.  A step moves M by an amount that
+// depends on M's parity alone (ties), so a lane's 16 steps are two displacements, found by
+// running them from an even and from an odd M; a warp scan composes them (mod 2^32: past the
+// first step that left the binade nothing is used), and each lane runs its steps again from
+// its true start, tested at once.  The window ends where the first lane with a step outside
+// starts.  There the value is near a power of two and often crosses it again soon: blocks of
+// 16 in the fixed-width step (which crosses powers of two, not fraction widths; f64_posit_add
+// does) follow until one stayed in its binade.
 //
-// After a cut window the value is near a power of two and often crosses it again soon:
-// runs follow until CHAIN_CALM of them in a row stayed inside.
-//
-// What bounds it: latency.  A dependent FP64 addition takes 8.1 cycles, a run of 8 with its
-// test 98 at best, a window of 512 about 900, a repeated run 500; in a Cholesky solve of
-// order 2048 a row of 1024 addends meets 3.7 windows (2 of them cut), 13 clean runs and 9
-// repeated ones: 13,500 cycles, half of them around the places where the value crosses a
-// power of two several times.  Rpotrs, one right-hand side: n = 1024 10.5 -> 6.5 ms, 4096
-// 92 -> 61, 8192 325 -> 196, against a scan of one step map per addend over four warps with
-// fixed-width steps between its windows.
+// What bounds it: latency.  A dependent FP64 addition takes 8.1 cycles, a window about 900, a
+// fixed-width step 32 and its block's tests and branches 150 (so 16 steps, not 8).  (Blocks of 8 one-addition steps first, repeated where
+// they left the binade, were slower: half of them did, and each start in a new binade cost
+// 200.)
 #if defined(__CUDACC__)
-constexpr int CHAIN_CALM = 4;        // clean runs before the next window
+constexpr int CHAIN_E = 16;          // addends per lane of a window, 8 or 16
 constexpr int CHAIN_WINDOW_MIN = 64; // addends left for a window to pay
 
 // A row's addends in shared memory, in groups of 16.  FP64: a group every 18 doubles, so that
@@ -473,45 +466,37 @@ __device__ double warp_chain(double t, Q q, int pos, int end)
 {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
-    bool calm = true;
-    int clean = 0;
     pos &= ~7; // from here on a multiple of 8: adding a zero changes nothing
     while (pos < end) {
         const uint32_t th = f64_hi(t);
         const int32_t eb = (int32_t)((th >> 20) & 0x7FF);
-        if (f64_outside_fast(eb)) { // zero among them: no grid to sit on, step by step
-            for (int k = 0; k < 8; ++k)
-                t = f64_round_any(f64_add(t, q.get(pos + k)));
-            pos += 8;
-            continue;
-        }
-        const uint32_t chi = f64_round_const_hi(eb) | (th & 0x80000000u);
-        const double C = f64_from_hi(chi);
-        const int32_t run = (int32_t)((chi >> 20) & 0x7FF) - eb - 24;
-        const uint32_t lim = 1u << (28 - run); // 2^fb
-        double w = f64_add(C, t);
-        for (;;) { // in this binade
-            if (calm && end - pos >= CHAIN_WINDOW_MIN) {
-                const int g0 = pos >> 4, k0 = (g0 + lane) * 16;
-                const int wend = min(end, (g0 + 32) * 16);
-                double v[16];
+        if (end - pos >= CHAIN_WINDOW_MIN && !f64_outside_fast(eb)) {
+            const uint32_t chi = f64_round_const_hi(eb) | (th & 0x80000000u);
+            const double C = f64_from_hi(chi);
+            const uint32_t lim = 1u << (28 - ((int32_t)((chi >> 20) & 0x7FF) - eb - 24)); // 2^fb
+            double w = f64_add(C, t);
+            bool left = false;
+            do { // windows in this binade
+                const int g0 = pos / CHAIN_E, k0 = (g0 + lane) * CHAIN_E;
+                const int wend = min(end, (g0 + 32) * CHAIN_E);
+                double v[CHAIN_E];
                 if (k0 < end) {
                     q.load(k0, v);
-                    if (k0 < pos) { // the group's first half is done
+                    if (CHAIN_E > 8 && k0 < pos) { // the group's first half is done
 #pragma unroll
                         for (int e = 0; e < 8; ++e)
                             v[e] = 0.0;
                     }
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 16; ++e)
+                    for (int e = 0; e < CHAIN_E; ++e)
                         v[e] = 0.0;
                 }
                 // the lane's displacements: of an even M, and by how much an odd one's differs
                 constexpr uint32_t M0 = 1u << 28;
                 double w0 = __hiloint2double((int)chi, (int)M0), w1 = __hiloint2double((int)chi, (int)(M0 + 1));
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
+                for (int e = 0; e < CHAIN_E; ++e) {
                     w0 = f64_add(w0, v[e]);
                     w1 = f64_add(w1, v[e]);
                 }
@@ -534,7 +519,7 @@ __device__ double warp_chain(double t, Q q, int pos, int end)
                 double y = __hiloint2double((int)chi, (int)M);
                 uint32_t bad = 0, mn = 0xFFFFFFFFu, mx = 0;
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
+                for (int e = 0; e < CHAIN_E; ++e) {
                     y = f64_add(y, v[e]);
                     const uint32_t lo = (uint32_t)__double2loint(y);
                     bad |= (uint32_t)__double2hiint(y) ^ chi;
@@ -543,72 +528,83 @@ __device__ double warp_chain(double t, Q q, int pos, int end)
                 }
                 const unsigned bal = __ballot_sync(FULL, bad != 0 || mn <= lim || mx >= 2 * lim);
                 const uint32_t Mend = __shfl_sync(FULL, (uint32_t)__double2loint(y), 31);
-                if (bal == 0) {
+                left = bal != 0;
+                if (!left) {
                     w = __hiloint2double((int)chi, (int)Mend);
                     pos = wend;
-                    if (pos < end)
-                        continue;
-                    return f64_add(w, -C);
+                } else {
+                    const int src = __ffs(bal) - 1;
+                    w = __hiloint2double((int)chi, (int)__shfl_sync(FULL, M, src));
+                    pos = max(pos, (g0 + src) * CHAIN_E);
                 }
-                const int src = __ffs(bal) - 1;
-                w = __hiloint2double((int)chi, (int)__shfl_sync(FULL, M, src));
-                pos = max(pos, (g0 + src) * 16);
-                calm = false;
-                clean = 0;
-            }
-            // runs of 8
-            double v[8], wb;
+            } while (!left && end - pos >= CHAIN_WINDOW_MIN);
+            t = f64_add(w, -C);
+            if (pos >= end)
+                break;
+        }
+        // blocks of 16 in the fixed-width step, its constant kept while the width is
+        double v[8], v2[8], Cs = 0.0;
+        uint32_t wlo = 1, wspan = 0; // |t|'s high words of this fraction width: [wlo, wlo + wspan)
+        auto width = [&]() {
+            const int32_t eb = f64_binade(t), k = (eb - 1023) >> 2, run = (k ^ (k >> 31)) + 1;
+            // the binades of regime k; around 1, those of regimes 0 and -1
+            wlo = (uint32_t)((run == 1 ? -4 : 4 * k) + 1023) << 20;
+            wspan = f64_outside_fast(eb) ? 0u : (run == 1 ? 8u : 4u) << 20;
+            Cs = f64_split_const(run);
+        };
+        auto fetch = [&]() {
             q.load(pos, v);
-            bool left;
-            for (;;) {
-                wb = w;
-                uint32_t bad = 0, mn = 0xFFFFFFFFu, mx = 0;
+            if (pos + 8 < end) {
+                q.load(pos + 8, v2);
+            } else {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    w = f64_add(w, v[e]);
-                    const uint32_t lo = (uint32_t)__double2loint(w);
-                    bad |= (uint32_t)__double2hiint(w) ^ chi;
-                    mn = min(mn, lo);
-                    mx = max(mx, lo);
-                }
-                left = bad != 0 || mn <= lim || mx >= 2 * lim;
-                if (left)
-                    break;
-                pos += 8;
-                if (pos >= end || ++clean >= CHAIN_CALM)
-                    break;
-                q.load(pos, v);
+                for (int e = 0; e < 8; ++e)
+                    v2[e] = 0.0;
             }
-            if (!left) {
-                calm = end - pos >= CHAIN_WINDOW_MIN;
-                if (pos < end)
-                    continue;
-                return f64_add(w, -C);
-            }
-            // the run again: the fixed-width step, or f64_posit_add
-            clean = 0;
-            calm = false;
-            const double t0 = f64_add(wb, -C), Cs = f64_split_const(run);
-            uint32_t flag = 0;
-            t = t0;
+        };
+        width();
+        fetch();
+        bool crossed;
+        do {
+            const double t0 = t;
+            uint32_t out = wspan == 0, cross = 0;
+            auto step = [&](double x) {
+                const double s = f64_add(t, x);
+                const double g = f64_mul(Cs, s);
+                t = f64_add(g, f64_add(s, -g));
+                // off the dependent path
+                const uint32_t h = f64_hi(s);
+                out |= (h & 0x7FFFFFFFu) - wlo >= wspan;
+                cross |= h ^ f64_hi(t0);
+            };
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-                t = f64_posit_add_split(t, v[e], Cs, run, flag);
-            if (flag & 0x40000000u) {
+                step(v[e]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                step(v2[e]);
+            if (out) { // across fraction widths: with the constant of every step's own binade
                 t = t0;
-                flag = 0;
+                uint32_t flag = 0;
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
                     t = f64_posit_add(t, v[e], flag);
-                if (flag & 0x40000000u) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    t = f64_posit_add(t, v2[e], flag);
+                if (flag & 0x40000000u) { // zero, or outside the fast window
                     t = t0;
-                    for (int e = 0; e < 8; ++e)
-                        t = f64_round_any(f64_add(t, q.get(pos + e)));
+                    for (int e = 0; e < 16; ++e)
+                        if (pos + e < end)
+                            t = f64_round_any(f64_add(t, q.get(pos + e)));
                 }
+                width();
             }
-            pos += 8;
-            break;
-        }
+            crossed = (cross >> 20) != 0;
+            pos += 16;
+            if (pos < end)
+                fetch();
+        } while (pos < end && (crossed || end - pos < CHAIN_WINDOW_MIN));
     }
     return t;
 }
