@@ -10,7 +10,7 @@
 // operand prescale (alpha*B for NN/NT), the accumulator's start value and the
 // epilogue.  Two routes, the same k-step (gemm_tile.cuh) and the same bits:
 //
-//  * staged (large products): a pre-pass converts op(A) and op(B) (times alpha for NN/NT,
+//  * staged (large products, see gemm_route): a pre-pass converts op(A) and op(B) (times alpha for NN/NT,
 //    rounded exactly as the reference rounds alpha*b_lj) ONCE per element to FP64 (posit32
 //    values are exact there) into a workspace of 32 x 16 blocks, [block][k-tile][l][32],
 //    plus a NaR flag per row and column; transposition is absorbed here.  The main kernel,
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(TILE_THREADS, MIN_CTAS_PER_SM)
 
     // One block barrier per k tile, although a barrier per stage would do: it keeps the warps
     // in step, and with them the unrolled steps (14 KB) in the instruction cache (warps
-    // that ran on by themselves took 333 ms for 8192^3 instead of 285).
+    // that ran on by themselves took 333 ms for 8192^3 instead of 289).
     bool bad = false, slow = false;
     int kt_stop = 0, s = 0;
     uint32_t parity = 0;

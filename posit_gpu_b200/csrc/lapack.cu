@@ -11,17 +11,17 @@
 // block size bit for bit (the zero-multiplier skips of Rtrsm/Rsyrk add zero and change
 // nothing unless a NaR is present), and the device code may block the work its own way:
 //
-//   panel (nb columns)   two kernels per column, ordered by the kernel boundary alone:
-//                        the pivot (LU: iRamax and the row interchange) or diagonal
-//                        (Cholesky: square root) step of one CTA, then the scaling of
-//                        the column and the rank-1 update of the rest of the panel over
-//                        all rows in parallel;
+//   panel (nb columns)   one launch: LU on a thread-block cluster holding the panel in shared
+//                        memory, Cholesky on independent CTAs; LU panels too tall or wide
+//                        for shared memory take two launches per column, ordered by the
+//                        kernel boundary alone (the pivot step of one CTA, then the scaling
+//                        and the rank-1 update over all rows in parallel);
 //   U block row          Rtrsm("L","L","N","U"), a warp or a CTA per column;
 //   row interchanges     Rlaswp on the columns outside the panel;
 //   trailing update      the posit32 GEMM of gemm.cu (NN for LU; NT restricted to the
 //                        lower triangle for Cholesky).
 // The matrix never leaves the device.  Upper Cholesky (dot-then-combine order, block size
-// dependent) is not implemented on the device.
+// dependent) follows the caller's block size.
 #include "gemm.cuh"
 #include "lapack.cuh"
 
@@ -824,6 +824,34 @@ __global__ void __launch_bounds__(COL_WARPS * 32, 1) trsm_block_kernel(const uin
     }
 }
 
+// A column that does not fit in the shared memory of 8 CTAs (more than 202,752 rows: a triangle of
+// 164 GB): the column stays in B, one CTA of 1024 threads per right-hand side, a row a step.
+template <bool UPPER>
+__global__ void __launch_bounds__(1024) trsm_long_kernel(const uint32_t *__restrict__ A, size_t lda, uint32_t *B,
+                                                         size_t ldb, int m, bool unit, const int *__restrict__ info)
+{
+    if (info && *info < 0)
+        return;
+    uint32_t *x = B + (size_t)blockIdx.x * ldb;
+    for (int s = 0; s < m; ++s) {
+        const int k = UPPER ? m - 1 - s : s;
+        const uint32_t *ak = A + (size_t)k * lda;
+        uint32_t bk = x[k];
+        if (bk != 0) {
+            if (!unit) {
+                bk = pdiv_est(bk, ak[k]);
+                __syncthreads(); // every thread has read x[k]
+                if (threadIdx.x == 0)
+                    x[k] = bk;
+            }
+            const int end = UPPER ? k : m;
+            for (int i = (UPPER ? 0 : k + 1) + (int)threadIdx.x; i < end; i += (int)blockDim.x)
+                x[i] = padd(x[i], pmul(0u - bk, ak[i]));
+        }
+        __syncthreads();
+    }
+}
+
 // One cluster per right-hand side: a CTA per 16 blocks (512 rows), up to 8.
 static cudaError_t launch_col(bool upper, bool unit, int nrhs, const uint32_t *A, size_t lda, uint32_t *B, size_t ldb,
                               int m, const int *info, cudaStream_t st)
@@ -837,6 +865,13 @@ static cudaError_t launch_col(bool upper, bool unit, int nrhs, const uint32_t *A
     while (warps > 1 && col_smem_bytes(nb, ncta, warps) > COL_SMEM_MAX)
         --warps;
     const size_t smem = col_smem_bytes(nb, ncta, warps);
+    if (smem > COL_SMEM_MAX) {
+        if (upper)
+            trsm_long_kernel<true><<<nrhs, 1024, 0, st>>>(A, lda, B, ldb, m, unit, info);
+        else
+            trsm_long_kernel<false><<<nrhs, 1024, 0, st>>>(A, lda, B, ldb, m, unit, info);
+        return cudaGetLastError();
+    }
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;
@@ -894,17 +929,18 @@ __global__ void __launch_bounds__(32) trsm_llt_kernel(const uint32_t *__restrict
 // other half of a double buffer, and its diagonal's reciprocal, meanwhile.  Warp 0 sums a row
 // with warp_chain (trsm_chain.cuh); the term of the b just finished (the first one, UPPER:
 // the last) it forms itself.  Four warps: one per sub-partition of the SM, so nothing else
-// issues where the chain runs.
+// issues where the chain runs.  Rpotrs, one right-hand side, against four warps that scanned one
+// step map per addend: n = 1024 10.5 -> 5.7 ms, 4096 92 -> 52 ms.
 // NaR travels as NaN; a NaR term sets its row's flag and is replaced by 0.
 constexpr int LTX_THREADS = 128;
 
-template <class Terms>
+template <class Terms, class Col>
 static size_t ltx_smem_bytes(int m)
 {
-    return 2 * Terms::bytes(m) + (size_t)m * LtxColOf<Terms>::Col::BYTES;
+    return 2 * Terms::bytes(m) + (Col::GLOBAL ? 0 : (size_t)m * 8);
 }
 
-template <class Terms, bool UPPER>
+template <class Terms, class Col, bool UPPER>
 __global__ void __launch_bounds__(LTX_THREADS) trsm_ltx_kernel(const uint32_t *__restrict__ L, size_t ldl,
                                                                uint32_t *__restrict__ B, size_t ldb, int m, bool unit,
                                                                const int *__restrict__ info)
@@ -913,14 +949,19 @@ __global__ void __launch_bounds__(LTX_THREADS) trsm_ltx_kernel(const uint32_t *_
     __shared__ LtxRow s_row[2];
     if (info && *info != 0) // a factorization stopped before this solve
         return;
-    typename LtxColOf<Terms>::Col x;
-    x.b = reinterpret_cast<decltype(x.b)>(smem_ltx + 2 * Terms::bytes(m));
+    Col x;
     uint32_t *bcol = B + (size_t)blockIdx.x * ldb;
-    for (int k = threadIdx.x; k < m; k += LTX_THREADS)
-        x.set(k, p32_to_double(bcol[k]));
-    block_ltx_solve<LTX_THREADS, UPPER, Terms>(L, ldl, x, m, unit, smem_ltx, s_row);
-    for (int k = threadIdx.x; k < m; k += LTX_THREADS)
-        bcol[k] = p32_from_double_exact(x.get(k));
+    if constexpr (Col::GLOBAL) {
+        x.b = bcol;
+        block_ltx_solve<LTX_THREADS, UPPER, Terms>(L, ldl, x, m, unit, smem_ltx, s_row);
+    } else {
+        x.b = reinterpret_cast<double *>(smem_ltx + 2 * Terms::bytes(m));
+        for (int k = threadIdx.x; k < m; k += LTX_THREADS)
+            x.set(k, p32_to_double(bcol[k]));
+        block_ltx_solve<LTX_THREADS, UPPER, Terms>(L, ldl, x, m, unit, smem_ltx, s_row);
+        for (int k = threadIdx.x; k < m; k += LTX_THREADS)
+            bcol[k] = p32_from_double_exact(x.get(k));
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1201,7 +1242,7 @@ size_t rgetrf_workspace_bytes(int m, int n, int nb)
     return panel_ws_bytes(m) + g;
 }
 
-// The panel form: the cluster panel held in shared memory when its rows fit (ncta CTAs,
+// The LU panel's form: the cluster panel held in shared memory when its rows fit (ncta CTAs,
 // one per PANEL1_ROWS_PER_CTA rows up to 8, T threads each -- the CTA's rows rounded up to
 // whole warps, at most 1024 -- R slots per thread), else the two-launch form (ncta = 0).
 struct PanelForm {
@@ -1460,18 +1501,20 @@ cudaError_t rgetrs_launch(int n, int nrhs, const uint32_t *A, int lda, const int
 // The dot-form solves with the triangle transposed: L^-T B (Rtrsm('L', 'L', 'T'),
 // Rtrsm.cpp:175-186) or, with `upper`, U^-T B (Rtrsm('L', 'U', 'T'), Rtrsm.cpp:160-173).
 // One block per right-hand side: trsm_ltx_kernel where its terms fit in shared memory
-// (FP64 where 26n bytes do, patterns where 12n do), else one thread's chain.
+// (FP64 where 26n bytes do, five bytes each where 10n do, n <= 23,232), else one thread's chain.
 // A nonzero *info (when given) turns the solve into a no-op.
 static cudaError_t launch_ltx(bool upper, bool unit, int n, int nrhs, const uint32_t *A, int lda, uint32_t *B,
                               int ldb, const int *info, cudaStream_t st)
 {
     cudaError_t e = cudaSuccess;
-    const size_t b64 = ltx_smem_bytes<ChainTerms64>(n), b32 = ltx_smem_bytes<ChainTerms32>(n);
-    if (b64 <= (size_t)LLT_SMEM_MAX || b32 <= (size_t)LLT_SMEM_MAX) {
+    const size_t b64 = ltx_smem_bytes<ChainTerms64, LtxCol64>(n), b40 = ltx_smem_bytes<ChainTerms40, LtxColGlobal>(n);
+    if (b64 <= (size_t)LLT_SMEM_MAX || b40 <= (size_t)LLT_SMEM_MAX) {
         const bool f64 = b64 <= (size_t)LLT_SMEM_MAX;
-        const size_t bytes = f64 ? b64 : b32;
-        auto *fn = f64 ? (upper ? trsm_ltx_kernel<ChainTerms64, true> : trsm_ltx_kernel<ChainTerms64, false>)
-                       : (upper ? trsm_ltx_kernel<ChainTerms32, true> : trsm_ltx_kernel<ChainTerms32, false>);
+        const size_t bytes = f64 ? b64 : b40;
+        auto *fn = f64 ? (upper ? trsm_ltx_kernel<ChainTerms64, LtxCol64, true>
+                                : trsm_ltx_kernel<ChainTerms64, LtxCol64, false>)
+                       : (upper ? trsm_ltx_kernel<ChainTerms40, LtxColGlobal, true>
+                                : trsm_ltx_kernel<ChainTerms40, LtxColGlobal, false>);
         if (bytes > 48 * 1024) {
             e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
             if (e != cudaSuccess)

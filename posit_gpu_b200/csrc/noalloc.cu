@@ -20,7 +20,7 @@
 //
 // All calls on a device share the one array and it keeps whatever the last call left in
 // it.  Nothing in it has to start at zero from an earlier call: on every call the GEMM
-// launch clears the region of per-row and per-column NaR flags (a stream-ordered memset)
+// launch that uses the workspace clears the region of per-row and per-column NaR flags (a stream-ordered memset)
 // before the decode pre-pass sets the flags it finds, and the decode pre-pass writes every
 // byte of the operand-tile region before the main kernel reads it.  Two calls whose work
 // overlaps on the GPU (e.g. issued on different streams without ordering) race on the

@@ -6,14 +6,14 @@
 // Each b_i's sum starts from the b_{i+1} just finished, so one right-hand side is a single
 // chain of m(m-1)/2 dependent multiply-subtracts with two roundings each.  Three forms:
 //   * llt_chain: one thread runs a right-hand side's whole chain with the accumulator
-//     held in the decoded integer form (the batched kernel; very long columns);
+//     held in the decoded integer form (very long columns);
 //   * chain_add_run / chain_add_run_reg: one thread's chain of additions in FP64, the
 //     products computed elsewhere (chain_add_run is the sequence the tests hold the others
 //     to);
 //   * warp_chain (end of this file): a warp sums a row's additions with the running value
 //     biased onto its binade's grid, one FP64 addition per step, and where the value is calm
 //     as a parallel prefix of step maps (lapack.cu's transposed-solve kernel and the
-//     batched kernel).  The scan form it grew from, one map per addend, stays written out
+//     batched kernels).  The scan form it grew from, one map per addend, stays written out
 //     for the host.
 //
 // For the one-thread chains latency is everything.  Only the addition depends on the previous step: loads,
@@ -414,8 +414,7 @@ constexpr int CHAIN_E = 16;          // addends per lane of a window, 8 or 16
 constexpr int CHAIN_WINDOW_MIN = 64; // addends left for a window to pay
 
 // A row's addends in shared memory, in groups of 16.  FP64: a group every 18 doubles, so that
-// the lanes of a warp reading a group each spread over the banks.  Patterns (columns too
-// long for that): packed.
+// the lanes of a warp reading a group each spread over the banks.
 struct ChainTerms64 {
     double *q;
     static constexpr int GROUP_DOUBLES = 18;
@@ -436,23 +435,35 @@ struct ChainTerms64 {
         }
     }
 };
-struct ChainTerms32 {
-    uint32_t *q;
-    static __host__ __device__ size_t bytes(int n) { return (size_t)((n + 15) / 16) * 16 * sizeof(uint32_t); }
+// Five bytes an addend, for columns too long for FP64: a posit has at most 27 fraction bits, so
+// the low word's upper byte holds all that the high word does not.  Patterns instead (4 bytes,
+// converted by the adding warp at each load) took Rpotrs n = 16384 1618 ms; this takes 838.
+struct ChainTerms40 {
+    unsigned char *q; // a buffer of n addends: the high words, then the bytes
+    int n16;          // n, up to a multiple of 16
+    static __host__ __device__ size_t bytes(int n) { return (size_t)((n + 15) / 16) * 80; }
     using Word = uint32_t;
-    __device__ void set(int k, double v) const { q[k] = p32_from_double_exact(v); }
-    __device__ double get(int k) const { return p32_to_double(q[k]); }
-    template <int N>
+    __device__ uint32_t *hi() const { return reinterpret_cast<uint32_t *>(q); }
+    __device__ unsigned char *lo() const { return q + (size_t)n16 * 4; }
+    __device__ void set(int k, double v) const
+    {
+        hi()[k] = (uint32_t)__double2hiint(v);
+        lo()[k] = (unsigned char)((uint32_t)__double2loint(v) >> 24);
+    }
+    __device__ double get(int k) const { return __hiloint2double((int)hi()[k], (int)((uint32_t)lo()[k] << 24)); }
+    template <int N> // as above, N a multiple of 8
     __device__ void load(int k, double (&v)[N]) const
     {
-        const uint4 *p = reinterpret_cast<const uint4 *>(q + k);
+        const uint4 *h = reinterpret_cast<const uint4 *>(hi() + k);
+        const uint2 *l = reinterpret_cast<const uint2 *>(lo() + k);
 #pragma unroll
         for (int j = 0; j < N / 4; ++j) {
-            const uint4 x = p[j];
-            v[4 * j] = p32_to_double(x.x);
-            v[4 * j + 1] = p32_to_double(x.y);
-            v[4 * j + 2] = p32_to_double(x.z);
-            v[4 * j + 3] = p32_to_double(x.w);
+            const uint4 x = h[j];
+            const uint32_t y = j & 1 ? l[j / 2].y : l[j / 2].x;
+            v[4 * j] = __hiloint2double((int)x.x, (int)(y << 24));
+            v[4 * j + 1] = __hiloint2double((int)x.y, (int)__byte_perm(y, 0, 0x1444));
+            v[4 * j + 2] = __hiloint2double((int)x.z, (int)__byte_perm(y, 0, 0x2444));
+            v[4 * j + 3] = __hiloint2double((int)x.w, (int)(y & 0xFF000000u));
         }
     }
 };
@@ -664,33 +675,25 @@ __device__ void warp_llt_solve(const uint32_t *__restrict__ L, size_t ldl, doubl
     }
 }
 
-// The solution column in shared memory: FP64, or patterns where the columns are long.
+// The solution column: FP64 in shared memory, or where the columns are long the patterns in
+// global memory.
 struct LtxCol64 {
     double *b;
-    static constexpr size_t BYTES = 8;
+    static constexpr bool GLOBAL = false;
     __device__ double get(int k) const { return b[k]; }
     __device__ void set(int k, double v) const { b[k] = v; }
 };
-struct LtxCol32 {
+struct LtxColGlobal {
     uint32_t *b;
-    static constexpr size_t BYTES = 4;
+    static constexpr bool GLOBAL = true;
     __device__ double get(int k) const { return p32_to_double(b[k]); }
     __device__ void set(int k, double v) const { b[k] = p32_from_double_exact(v); }
-};
-template <class Terms>
-struct LtxColOf;
-template <>
-struct LtxColOf<ChainTerms64> {
-    using Col = LtxCol64;
-};
-template <>
-struct LtxColOf<ChainTerms32> {
-    using Col = LtxCol32;
 };
 // What the adding warp needs of a row besides its terms.
 struct LtxRow {
     double diag, recip; // a_ii and fl(1/a_ii)
     double near;        // the coefficient of the b finished last
+    double b;           // the right-hand side's entry (Col::GLOBAL)
     int nar;            // a term was NaR
 };
 
@@ -707,6 +710,8 @@ __device__ __forceinline__ void block_ltx_solve(const uint32_t *__restrict__ L, 
     auto terms = [&](int half) {
         Terms q;
         q.q = reinterpret_cast<decltype(q.q)>(buf + half * Terms::bytes(m));
+        if constexpr (Col::GLOBAL)
+            q.n16 = (m + 15) & ~15;
         return q;
     };
     // Terms outside a row's range are zero for warp_chain: rows grow, so what no earlier row
@@ -722,6 +727,8 @@ __device__ __forceinline__ void block_ltx_solve(const uint32_t *__restrict__ L, 
         r.diag = unit ? 1.0 : p32_to_double(li[i]);
         r.recip = 1.0 / r.diag;
         r.near = step > 0 ? p32_to_double(li[UPPER ? i - 1 : i + 1]) : 0.0;
+        if (Col::GLOBAL)
+            r.b = x.get(i);
     };
     if (tid < 2)
         s_row[tid].nar = 0;
@@ -733,7 +740,7 @@ __device__ __forceinline__ void block_ltx_solve(const uint32_t *__restrict__ L, 
         const int i = row_of(step), cur = step & 1;
         if (tid < 32) {
             const LtxRow r = s_row[cur];
-            double t = x.get(i);
+            double t = Col::GLOBAL ? r.b : x.get(i);
             bool nar = t != t || r.nar;
             double near = 0.0; // -a*x_k of the one just finished
             if (step > 0) {
@@ -773,13 +780,18 @@ __device__ __forceinline__ void block_ltx_solve(const uint32_t *__restrict__ L, 
             constexpr int P = NT - 32, U = 8; // U loads in flight per thread
             for (int k = kbeg + (tid - 32); k < kend; k += U * P) {
                 uint32_t l[U];
+                double xk[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u)
+                for (int u = 0; u < U; ++u) {
                     l[u] = k + u * P < kend ? lp[k + u * P] : 0u;
+                    xk[u] = Col::GLOBAL && k + u * P < kend ? x.get(k + u * P) : 0.0;
+                }
 #pragma unroll
                 for (int u = 0; u < U; ++u)
                     if (k + u * P < kend) {
-                        double v = f64_posit_mul_checked(-x.get(k + u * P), p32_to_double(l[u]), F64ConstComputed{});
+                        if (!Col::GLOBAL)
+                            xk[u] = x.get(k + u * P);
+                        double v = f64_posit_mul_checked(-xk[u], p32_to_double(l[u]), F64ConstComputed{});
                         if (v != v) {
                             nar = 1;
                             v = 0.0;

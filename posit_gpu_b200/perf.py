@@ -3,7 +3,8 @@
 The GEMM main kernel runs each posit multiply-add as FP64 operations plus a little
 integer work (posit32.cuh, f64_posit_mac): it is bound by instruction issue -- each SM
 sub-partition (4 per SM, 148 SMs on B200) issues at most one warp instruction per cycle --
-with the FP64 pipe (half rate) the busiest pipe.  The roofline therefore compares the
+with the FP64 pipe (half rate) the busiest pipe: an FP64 warp instruction takes two issue
+slots, so the issue figure below cannot reach 1 (6 of 14 instructions take two).  The roofline therefore compares the
 kernel's issued warp instructions per second with 148 * 4 * f_SM warp instructions per
 second, f_SM being the SM clock sampled during the run.  The instruction count per posit
 multiply-add is a property of the compiled kernel (its fast path is branch-free),
@@ -19,16 +20,17 @@ SM_MAX_MHZ = 1965.0
 
 # Warp instructions issued by gemm_main_kernel per posit multiply-add:
 # smsp__inst_executed.sum / (m*n*k) for one NN launch at m = n = k = 4096
-# (48,162,455,398 / 68,719,476,736 = 0.7009, i.e. 22.43 thread instructions).  Of those,
-# 10 per multiply-add run on the FP64 pipe (DMUL, DFMA, 6 DADD, 2 DSETP): FP64 pipe
-# 62.9 %, ALU pipe 36.1 %, LSU 30.8 %, issue 70.9 % busy in the same capture.
-WARP_INST_PER_MAD = 0.7009
-FP64_WARP_INST_PER_MAD = 10 / 32
-INST_SOURCE = ("ncu --set full, gemm_main_kernel<0,0>, NN 4096^3 U[-1,1] "
+# (30,100,779,008 / 68,719,476,736 = 0.4380, i.e. 14.02 thread instructions).  Of those,
+# 6 per multiply-add run on the FP64 pipe (DMUL, DFMA, 4 DADD; smsp__inst_executed_pipe_fp64.sum
+# 12,952,535,040 = 0.1885): FP64 pipe 61.7 %, ALU pipe 41.7 %, LSU 46.1 %, issue 71.7 % busy in
+# the same capture.
+WARP_INST_PER_MAD = 0.4380
+FP64_WARP_INST_PER_MAD = 6 / 32
+INST_SOURCE = ("ncu, gemm_main_kernel<0>, NN 4096^3 U[-1,1] "
                "(profiles/gemm_main_kernel_nn_4096.md)")
 # DRAM bytes (read + write) per posit multiply-add of the same launch:
-# (7,488,873,000 + 121,976,832) / 68,719,476,736.
-MAIN_KERNEL_DRAM_BYTES_PER_MAD = 0.1108
+# (3,935,058,432 + 70,387,968) / 68,719,476,736.
+MAIN_KERNEL_DRAM_BYTES_PER_MAD = 0.0583
 
 
 def issue_peak_warp_inst_per_s(sm_mhz):
@@ -46,7 +48,7 @@ def fp64_pipe_peak_warp_inst_per_s(sm_mhz):
 # the benchmark recomputes the digest and, when it differs, marks the count stale and
 # reports no roofline fraction from it.
 KERNEL_SOURCES = ["csrc/gemm.cu", "csrc/gemm.cuh", "csrc/gemm_tile.cuh", "csrc/posit32.cuh"]
-INST_SOURCE_DIGEST = "5a203b78e19bc143f412235179eae4c1e55abcb0a85c594a21c4e0e78f9bed8d"
+INST_SOURCE_DIGEST = "384f9cddec05f2c51b93f69e87d3c11167a7b5d604d3b9ea8ee2aa26bb469a04"
 
 
 def kernel_source_digest():
@@ -69,8 +71,8 @@ def inst_count_current():
 # m = n = 8192 - b, k = b (key b), from ncu dram__bytes_read.sum + dram__bytes_write.sum
 # of that launch.  Empty until measured; the benchmark then reports no traffic figure for
 # the shape rather than one scaled from another shape.
-TRAILING_TRAFFIC_BYTES = {16: 486810624, 32: 486020096, 64: 487125504, 128: 486207744, 256: 488396800}
-TRAILING_TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum, gemm_main_kernel<0,0>, "
+TRAILING_TRAFFIC_BYTES = {16: 483767040, 32: 482796544, 64: 483489024, 128: 484047104, 256: 482452992}
+TRAILING_TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum, gemm_main_kernel<0>, "
                            "one launch per shape (profiles/gemm_main_kernel_lu_trailing.md)")
 
 

@@ -1,5 +1,5 @@
 """The transposed triangular solves' warp chain on both sides of its groups (16 addends),
-runs (8), windows (512) and storage forms (patterns from 8941 rows), on values that stay in
+runs (8), windows (512) and storage forms (five bytes an addend from 8941 rows), on values that stay in
 one binade, wander across powers of two, change fraction width, go wide, cancel to zero or
 hold a NaR: Rpotrs 'L' and 'U' against the oracle bit for bit."""
 import numpy as np
