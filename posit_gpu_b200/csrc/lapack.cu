@@ -639,14 +639,11 @@ static cudaError_t launch_laswp_rhs(uint32_t *B, int ldb, int nrhs, int n, const
                                     cudaStream_t st)
 {
     if (n <= LASWP_COL_MAX) {
-        const size_t bytes = (size_t)n * 4;
-        if (bytes > 40 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(laswp_col_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)bytes);
-            if (e != cudaSuccess)
-                return e;
-        }
-        laswp_col_kernel<<<nrhs, LASWP_COL_THREADS, bytes, st>>>(B, ldb, n, ipiv, forward);
+        const cudaError_t e = cudaFuncSetAttribute(laswp_col_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   LASWP_COL_MAX * 4);
+        if (e != cudaSuccess)
+            return e;
+        laswp_col_kernel<<<nrhs, LASWP_COL_THREADS, (size_t)n * 4, st>>>(B, ldb, n, ipiv, forward);
     } else {
         laswp_kernel<<<(nrhs + 127) / 128, 128, 0, st>>>(B, ldb, nrhs, 1, n, ipiv, forward ? 1 : -1, nullptr);
     }
@@ -872,7 +869,9 @@ static cudaError_t launch_col(bool upper, bool unit, int nrhs, const uint32_t *A
             trsm_long_kernel<false><<<nrhs, 1024, 0, st>>>(A, lda, B, ldb, m, unit, info);
         return cudaGetLastError();
     }
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // Here and elsewhere the limit is set to the most the kernel can take, not to this launch's size:
+    // another thread's launch of the same kernel may come between this call and the launch.
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COL_SMEM_MAX);
     if (e != cudaSuccess)
         return e;
     cudaLaunchConfig_t cfg = {};
@@ -1515,18 +1514,16 @@ static cudaError_t launch_ltx(bool upper, bool unit, int n, int nrhs, const uint
                                 : trsm_ltx_kernel<ChainTerms64, LtxCol64, false>)
                        : (upper ? trsm_ltx_kernel<ChainTerms40, LtxColGlobal, true>
                                 : trsm_ltx_kernel<ChainTerms40, LtxColGlobal, false>);
-        if (bytes > 48 * 1024) {
-            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e != cudaSuccess)
-                return e;
-        }
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, LLT_SMEM_MAX);
+        if (e != cudaSuccess)
+            return e;
         fn<<<nrhs, LTX_THREADS, bytes, st>>>(A, lda, B, ldb, n, unit, info);
         return cudaGetLastError();
     }
     const size_t col = (size_t)n * 4;
     const bool staged = col <= (size_t)LLT_SMEM_MAX;
     if (staged && col > 48 * 1024) {
-        e = cudaFuncSetAttribute(trsm_llt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col);
+        e = cudaFuncSetAttribute(trsm_llt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LLT_SMEM_MAX);
         if (e != cudaSuccess)
             return e;
     }
