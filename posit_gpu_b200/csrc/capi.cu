@@ -122,6 +122,26 @@ int rgemm_device(bool nota, bool notb, int m, int n, int k, uint32_t alpha, cons
     return 0;
 }
 
+// Whether two host matrices' address ranges meet: then C is written only when A and B have been read.
+bool host_overlap(const uint32_t *X, int ldx, int rx, int cx, const uint32_t *Y, int ldy, int ry, int cy)
+{
+    const uintptr_t x = (uintptr_t)X, y = (uintptr_t)Y;
+    return x < y + ((size_t)(cy - 1) * ldy + ry) * 4 && y < x + ((size_t)(cx - 1) * ldx + rx) * 4;
+}
+
+// In how many stretches of columns a product of host matrices goes through.  A second stream and
+// its events cost about 140 us, and a stretch should still fill the GPU (100 tiles of 64x64).
+// From pageable memory, 1 / 2 / 4 stretches: 512^3 501 / 571 / 696 us, 1024^3 1846 / 1704 / 1751,
+// 2048^3 9119 / 8485 / 7556, 4096^3 57955 / 51088 / 47701 (8: 51719).
+int host_parts(int m, int n, int k)
+{
+    const double mads = (double)m * n * k;
+    int parts = mads < 0x1p30 ? 1 : (mads < 0x1p33 ? 2 : 4);
+    while (parts > 1 && (long long)((m + 63) / 64) * (n / parts / 64) < 100)
+        parts /= 2;
+    return parts;
+}
+
 } // namespace
 
 extern "C" {
@@ -176,34 +196,77 @@ int posit_rgemm(char transa, char transb, int m, int n, int k, uint32_t alpha, c
     // device copies of exactly the referenced submatrices, packed (ld = rows)
     const int ar = nota ? m : k, ac = nota ? k : m;
     const int br = notb ? k : n, bc = notb ? n : k;
-    uint32_t *dA = nullptr, *dB = nullptr, *dC = nullptr;
-    PG_TRY(cudaMallocAsync((void **)&dC, (size_t)m * n * 4, st));
+    // The columns of C go through in stretches of `w`: while one is computed the next one's operands
+    // come in and the last one's results go out, on a stream of their own.
+    const int parts = need_ab && !host_overlap(A, lda, ar, ac, C, ldc, m, n) && !host_overlap(B, ldb, br, bc, C, ldc, m, n)
+                          ? host_parts(m, n, k)
+                          : 1;
+    const int w = parts > 1 ? ((n + parts - 1) / parts + 63) / 64 * 64 : n;
+    const size_t na = need_ab ? (size_t)ar * ac : 0, nb = need_ab ? (size_t)br * bc : 0;
+    uint32_t *dev = nullptr;
+    PG_TRY(cudaMallocAsync((void **)&dev, (na + nb + (size_t)m * n) * 4, st));
+    uint32_t *dA = dev, *dB = dev + na, *dC = dev + na + nb;
+    cudaStream_t cp = st; // the copies' stream
+    cudaEvent_t in = nullptr, out[2] = {nullptr, nullptr};
+    cudaError_t e = cudaSuccess;
+    auto ok = [&](cudaError_t x) {
+        if (e == cudaSuccess)
+            e = x;
+        return e == cudaSuccess;
+    };
+    if (parts > 1 && ok(cudaEventCreateWithFlags(&in, cudaEventDisableTiming)) &&
+        ok(cudaEventCreateWithFlags(&out[0], cudaEventDisableTiming)) &&
+        ok(cudaEventCreateWithFlags(&out[1], cudaEventDisableTiming)) &&
+        ok(cudaStreamCreateWithFlags(&cp, cudaStreamNonBlocking)) && ok(cudaEventRecord(in, st)))
+        ok(cudaStreamWaitEvent(cp, in, 0)); // the allocation
+    auto upload = [&](uint32_t *d, const uint32_t *h, int ld, int rows, int cols) {
+        if (e == cudaSuccess)
+            ok(cudaMemcpy2DAsync(d, (size_t)rows * 4, h, (size_t)ld * 4, (size_t)rows * 4, cols, cudaMemcpyHostToDevice,
+                                 cp));
+    };
+    int rc = 0;
+    auto width = [&](int c0) { return n - c0 < w ? n - c0 : w; };
+    // the columns of C from c0 on: operands in, the product into the compute stream
+    auto start = [&](int c0) {
+        if (need_ab && notb)
+            upload(dB + (size_t)c0 * k, B + (size_t)c0 * ldb, ldb, k, width(c0));
+        if (beta != 0) // with beta == 0 the reference never reads C (Rgemm.cpp:143-147, 170-173, 197-198)
+            upload(dC + (size_t)c0 * m, C + (size_t)c0 * ldc, ldc, m, width(c0));
+        if (parts > 1 && e == cudaSuccess && ok(cudaEventRecord(in, cp)))
+            ok(cudaStreamWaitEvent(st, in, 0));
+        if (e == cudaSuccess)
+            rc = rgemm_device(nota, notb, m, width(c0), k, alpha, dA, ar, notb ? dB + (size_t)c0 * k : dB + c0, br, beta,
+                              dC + (size_t)c0 * m, m, nullptr, 0, st);
+        if (parts > 1 && e == cudaSuccess && rc == 0)
+            ok(cudaEventRecord(out[c0 / w & 1], st));
+    };
     if (need_ab) {
-        PG_TRY(cudaMallocAsync((void **)&dA, (size_t)ar * ac * 4, st));
-        PG_TRY(cudaMallocAsync((void **)&dB, (size_t)br * bc * 4, st));
-        PG_TRY(cudaMemcpy2DAsync(dA, (size_t)ar * 4, A, (size_t)lda * 4, (size_t)ar * 4, ac,
-                                 cudaMemcpyHostToDevice, st));
-        PG_TRY(cudaMemcpy2DAsync(dB, (size_t)br * 4, B, (size_t)ldb * 4, (size_t)br * 4, bc,
-                                 cudaMemcpyHostToDevice, st));
+        upload(dA, A, lda, ar, ac);
+        if (!notb)
+            upload(dB, B, ldb, br, bc);
     }
-    if (beta != 0) // with beta == 0 the reference never reads C (Rgemm.cpp:143-147, 170-173, 197-198)
-        PG_TRY(cudaMemcpy2DAsync(dC, (size_t)m * 4, C, (size_t)ldc * 4, (size_t)m * 4, n,
-                                 cudaMemcpyHostToDevice, st));
-    int rc = rgemm_device(nota, notb, m, n, k, alpha, dA, ar, dB, br, beta, dC, m, nullptr, 0, st);
-    if (rc == 0) {
-        cudaError_t e = cudaMemcpy2DAsync(C, (size_t)ldc * 4, dC, (size_t)m * 4, (size_t)m * 4, n,
-                                          cudaMemcpyDeviceToHost, st);
-        if (e != cudaSuccess)
-            rc = cuda_fail(e);
+    start(0);
+    for (int c0 = 0; c0 < n && rc == 0 && e == cudaSuccess; c0 += w) {
+        if (c0 + w < n)
+            start(c0 + w);
+        if (parts > 1 && e == cudaSuccess)
+            ok(cudaStreamWaitEvent(cp, out[c0 / w & 1], 0));
+        if (rc == 0 && e == cudaSuccess)
+            ok(cudaMemcpy2DAsync(C + (size_t)c0 * ldc, (size_t)ldc * 4, dC + (size_t)c0 * m, (size_t)m * 4,
+                                 (size_t)m * 4, width(c0), cudaMemcpyDeviceToHost, cp));
     }
-    if (dA)
-        cudaFreeAsync(dA, st);
-    if (dB)
-        cudaFreeAsync(dB, st);
-    cudaFreeAsync(dC, st);
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (rc == 0 && e != cudaSuccess)
-        rc = cuda_fail(e);
+    cudaError_t last = cp != st ? cudaStreamSynchronize(cp) : cudaSuccess;
+    cudaFreeAsync(dev, st);
+    const cudaError_t end = cudaStreamSynchronize(st);
+    if (last == cudaSuccess)
+        last = end;
+    if (cp != st)
+        cudaStreamDestroy(cp);
+    for (cudaEvent_t v : {in, out[0], out[1]})
+        if (v)
+            cudaEventDestroy(v);
+    if (rc == 0 && (e != cudaSuccess || last != cudaSuccess))
+        rc = cuda_fail(e != cudaSuccess ? e : last);
     if (rc == 0 && pg::read_device_error(true) != 0)
         rc = POSIT_E_DEVICE_FAULT;
     return rc;
