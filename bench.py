@@ -316,7 +316,7 @@ def ours(args):
                 "frac": achieved and round(achieved / peak, 4),
                 "traffic": (perf.MAIN_KERNEL_DRAM_BYTES_PER_MAD * mads
                             if perf.MAIN_KERNEL_DRAM_BYTES_PER_MAD and not args.trailing else None),
-                "kernel": "gemm_main_kernel<false,false>" if ta in "nN" else "gemm_main_kernel<true,false>",
+                "kernel": "gemm_main_kernel<0>",
                 "main_kernel_ms": round(main_avg_s * 1e3, 3),
                 "posit_gop_s_main_kernel": round(2 * mads / main_avg_s / 1e9, 2) if main_avg_s > 0 else None,
                 "warp_inst_per_mad": perf.WARP_INST_PER_MAD,
