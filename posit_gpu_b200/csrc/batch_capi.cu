@@ -165,7 +165,18 @@ extern "C" int posit_batch_gemm_plan_create(const posit_batch_gemm *probs, int n
         if (table[c] < 0 || table[c] >= pg::BATCH_TILE_CONFIGS)
             return POSIT_E_WORKSPACE;
     std::vector<pg::BatchGemmDesc> desc(nprob > 0 ? nprob : 1);
-    std::vector<pg::BatchTile> tiles;
+    std::vector<int> order; // the problems with any work
+    order.reserve(desc.size());
+    size_t ntiles = 0;
+    auto config = [&](const pg::BatchGemmDesc &d) { return table[size_bucket(d.m) * 3 + size_bucket(d.n)]; };
+    auto tile_rows = [&](const pg::BatchGemmDesc &d) {
+        const int b = pg::batch_tile_rows(config(d));
+        return (d.m + b - 1) / b;
+    };
+    auto tile_cols = [&](const pg::BatchGemmDesc &d) {
+        const int b = pg::batch_tile_cols(config(d));
+        return (d.n + b - 1) / b;
+    };
     for (int i = 0; i < nprob; ++i) {
         const posit_batch_gemm &q = probs[i];
         int info = gemm_args(q);
@@ -191,15 +202,19 @@ extern "C" int posit_batch_gemm_plan_create(const posit_batch_gemm *probs, int n
         // quick return (Rgemm.cpp:134-136): no work at all
         if (q.m == 0 || q.n == 0 || ((q.alpha == 0 || q.k == 0) && q.beta == 0x40000000u))
             continue;
-        const int cfg = table[size_bucket(q.m) * 3 + size_bucket(q.n)];
-        const int bm = pg::batch_tile_rows(cfg), bn = pg::batch_tile_cols(cfg);
-        for (int nt = 0; nt < (q.n + bn - 1) / bn; ++nt)
-            for (int mt = 0; mt < (q.m + bm - 1) / bm; ++mt)
+        order.push_back(i);
+        ntiles += (size_t)tile_rows(d) * tile_cols(d);
+    }
+    // longest k first (the problems are sorted, not their tiles: 32x32 tiles are many)
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return desc[a].k > desc[b].k; });
+    std::vector<pg::BatchTile> tiles;
+    tiles.reserve(ntiles);
+    for (int i : order) {
+        const int cfg = config(desc[i]), rows = tile_rows(desc[i]), cols = tile_cols(desc[i]);
+        for (int nt = 0; nt < cols; ++nt)
+            for (int mt = 0; mt < rows; ++mt)
                 tiles.push_back(pg::BatchTile{i, mt, nt, cfg});
     }
-    // longest k first
-    std::stable_sort(tiles.begin(), tiles.end(),
-                     [&](const pg::BatchTile &a, const pg::BatchTile &b) { return desc[a.prob].k > desc[b.prob].k; });
     posit_batch_plan *p = new (std::nothrow) posit_batch_plan();
     if (!p)
         return POSIT_E_NO_MEMORY;
