@@ -392,12 +392,18 @@ GemmRoute gemm_route(bool nota, bool notb, int m, int n, int k, const uint32_t *
         (spans_overlap(C, span(m, n, ldc), A, nota ? span(m, k, lda) : span(k, m, lda)) ||
          spans_overlap(C, span(m, n, ldc), B, notb ? span(k, n, ldb) : span(n, k, ldb))))
         return GEMM_STAGED;
-    const long long t44 = ceil_div(m, 64) * ceil_div(n, 64), t42 = ceil_div(m, 64) * ceil_div(n, 32);
+    const long long t44 = ceil_div(m, 64) * ceil_div(n, 64), t42 = ceil_div(m, 64) * ceil_div(n, 32),
+                    t22 = ceil_div(m, 32) * ceil_div(n, 32);
     // From 2^24 multiply-adds on 100 tiles the second launch is worth it: 1024 x 1024 x 24 39.9
     // against 44.4 us fused, 2048^2 x 32 121 / 125, 1000 x 1000 x 500 356 / 418, 700^3 272 / 301.
     if (t44 >= GEMM_STAGED_MIN_TILES && (double)m * n * k >= GEMM_STAGED_MIN_MADS)
         return GEMM_STAGED;
-    return t44 >= 2 * SM_COUNT ? GEMM_FUSED_64x64 : (t42 >= SM_COUNT ? GEMM_FUSED_64x32 : GEMM_FUSED_32x32);
+    // 64x32 tiles where there are so many that waves don't matter (1400^2 x 8 26.8 us against 28.9 in
+    // 32x32, 4000 x 1000 x 4 41.2 / 43.9, 1100^2 x 12 22.7 / 22.7) or they take one wave where 32x32
+    // tiles take two (4000 x 128 x 32 20.7 / 22.7); else 32x32 (640^2 x 32 17.5 against 20.7, 576^2
+    // x 512 191 / 219, 640 x 576 x 700 260 / 298).  64x64 tiles were slower throughout (1200^2 x 8 30.0).
+    const bool many = t42 >= 4 * SM_COUNT, one_wave = t42 <= 2 * SM_COUNT && t22 > 3 * SM_COUNT;
+    return many || one_wave ? GEMM_FUSED_64x32 : GEMM_FUSED_32x32;
 }
 
 template <class Kernel>
@@ -454,7 +460,6 @@ static cudaError_t gemm_launch_route(GemmRoute route, const TileArgs &P, void *w
     const bool prof = g_prof_on;
     cudaEvent_t e0 = prof && route != GEMM_STAGED ? prof_mark(stream) : nullptr;
     const cudaError_t e = route == GEMM_STAGED ? staged_launch<TRI>(P, workspace, stream, stop, prof ? &e0 : nullptr)
-                        : route == GEMM_FUSED_64x64 ? fused_launch<TRI, 4, 4>(P, stream, stop)
                         : route == GEMM_FUSED_64x32 ? fused_launch<TRI, 4, 2>(P, stream, stop)
                                                     : fused_launch<TRI, 2, 2>(P, stream, stop);
     if (prof) {

@@ -18,7 +18,7 @@ constexpr int MIN_CTAS_PER_SM = 2;
 constexpr int SM_COUNT = 148;
 
 // How a product is computed (gemm_route); the bits are the same.
-enum GemmRoute { GEMM_STAGED, GEMM_FUSED_64x64, GEMM_FUSED_64x32, GEMM_FUSED_32x32 };
+enum GemmRoute { GEMM_STAGED, GEMM_FUSED_64x32, GEMM_FUSED_32x32 };
 constexpr double GEMM_STAGED_MIN_MADS = 16777216.0; // 2^24 multiply-adds
 constexpr long long GEMM_STAGED_MIN_TILES = 100;
 

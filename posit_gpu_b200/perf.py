@@ -48,7 +48,7 @@ def fp64_pipe_peak_warp_inst_per_s(sm_mhz):
 # the benchmark recomputes the digest and, when it differs, marks the count stale and
 # reports no roofline fraction from it.
 KERNEL_SOURCES = ["csrc/gemm.cu", "csrc/gemm.cuh", "csrc/gemm_tile.cuh", "csrc/posit32.cuh"]
-INST_SOURCE_DIGEST = "384f9cddec05f2c51b93f69e87d3c11167a7b5d604d3b9ea8ee2aa26bb469a04"
+INST_SOURCE_DIGEST = "de3959670852b80076b1e212b2ff722ec4b29b16213019e852689cfc91f31402"
 
 
 def kernel_source_digest():

@@ -1,5 +1,5 @@
 """The GEMM's routes on both sides of every tile edge, against the oracle bit for bit.
-Separate operands take the fused route (32x32 tiles; 64x32 from 148 tiles, 64x64 from 296) but
+Separate operands take the fused route (32x32 tiles, or 64x32 where they are many) but
 for the one size beyond 2^24 multiply-adds, which is staged; so are A, B and C inside one matrix,
 whose address ranges meet (64x64 tiles of 32-row blocks, an odd count of blocks among them)."""
 import numpy as np
@@ -10,7 +10,7 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 SIZES = [(1, 1, 1), (31, 33, 15), (32, 32, 16), (33, 65, 17), (64, 64, 33), (97, 95, 48), (65, 2400, 20),
-         (1500, 640, 18), (1217, 1100, 19), (1153, 1089, 7)]
+         (1500, 640, 18), (1217, 1100, 19), (1153, 1089, 7), (4000, 100, 9)]
 
 
 def _values(rng, numel, kind):
