@@ -139,6 +139,9 @@ typedef struct posit_batch_plan posit_batch_plan;
 /* Uploads the descriptors (host array) and captures the launch; returns 0, 1/2 for bad
  * arguments / a bad descriptor, or POSIT_E_*. */
 int posit_batch_plan_create(const posit_batch_problem *probs, int nprob, posit_batch_plan **plan);
+/* How a plan of these problems runs on a GPU of `sms` SMs: route[i] = 0 for a CTA that has an
+ * SM for itself, 1 for one of two CTAs on an SM, 2 for a warp.  Host-only, no device needed. */
+int posit_batch_plan_routes(const posit_batch_problem *probs, int nprob, int sms, int *route);
 /* Many independent GEMMs (device pointers), each with the semantics and bits of
  * posit_rgemm_dev, in ONE persistent kernel fed by a device queue of output tiles
  * (longest k first), captured in a CUDA graph.  tile_table (9 ints, or NULL for the

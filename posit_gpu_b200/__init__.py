@@ -250,6 +250,8 @@ class _BatchProblem(_c.Structure):
 
 _lib.posit_batch_plan_create.argtypes = [_c.POINTER(_BatchProblem), _c.c_int, _c.POINTER(_VP)]
 _lib.posit_batch_plan_create.restype = _c.c_int
+_lib.posit_batch_plan_routes.argtypes = [_c.POINTER(_BatchProblem), _c.c_int, _c.c_int, _c.POINTER(_c.c_int)]
+_lib.posit_batch_plan_routes.restype = _c.c_int
 _lib.posit_batch_plan_launch.argtypes = [_VP, _VP]
 _lib.posit_batch_plan_launch.restype = _c.c_int
 _lib.posit_batch_plan_destroy.argtypes = [_VP]

@@ -438,22 +438,147 @@ __device__ __forceinline__ int factor_one(const BatchProblem &pr, unsigned char 
     return info;
 }
 
-// b_i - b_k*a_ik for the rows of one step of an axpy-form solve, all right-hand sides of the
-// group; the thread with row `next` then divides it (Rtrsm.cpp:127, 145; a zero is left
-// alone, as the reference skips it).
-constexpr int B_PRE = 2; // rows per thread whose coefficients are loaded a step ahead
+// ---------------------------------------------------------------------------
+// The right-hand sides
+// ---------------------------------------------------------------------------
+// The threads that solve one problem: a CTA, or a warp of one.
+template <int THREADS>
+struct Team {
+    static constexpr int T = THREADS;
+    __device__ __forceinline__ static int tid() { return THREADS == 32 ? threadIdx.x & 31 : threadIdx.x; }
+    __device__ __forceinline__ static void sync()
+    {
+        if (THREADS == 32)
+            __syncwarp();
+        else
+            __syncthreads();
+    }
+};
 
-// Rtrsm('L', LOWER ? 'L' : 'U', 'N') on the columns X (shared memory, [nrhs][n], FP64).
-template <class C, bool LOWER, bool UNIT>
-__device__ __forceinline__ void axpy_solve(const uint32_t *A, size_t lda, int n, double *X, int nrhs,
+// Right-hand sides between global memory (patterns) and X (shared memory, FP64, ldx apart).
+template <class TM, bool MANY>
+__device__ __forceinline__ void load_rhs(double *X, int ldx, const uint32_t *B, size_t ldb, int n, int cnt)
+{
+    if (!MANY) {
+        for (int r = 0; r < cnt; ++r)
+            for (int i = TM::tid(); i < n; i += TM::T)
+                X[r * ldx + i] = pd(B[r * ldb + i]);
+    } else {
+#pragma unroll 4
+        for (int e = TM::tid(); e < n * cnt; e += TM::T)
+            X[e / n * ldx + e % n] = pd(B[(size_t)(e / n) * ldb + e % n]);
+    }
+}
+template <class TM, bool MANY>
+__device__ __forceinline__ void store_rhs(const double *X, int ldx, uint32_t *B, size_t ldb, int n, int cnt)
+{
+    if (!MANY) {
+        for (int r = 0; r < cnt; ++r)
+            for (int i = TM::tid(); i < n; i += TM::T)
+                B[r * ldb + i] = p32_from_double_exact(X[r * ldx + i]);
+    } else {
+#pragma unroll 4
+        for (int e = TM::tid(); e < n * cnt; e += TM::T)
+            B[(size_t)(e / n) * ldb + e % n] = p32_from_double_exact(X[e / n * ldx + e % n]);
+    }
+}
+
+// Rlaswp, in order, a thread per right-hand side.
+template <class TM>
+__device__ __forceinline__ void swap_rhs(double *X, int ldx, const int *piv, int n, int cnt)
+{
+    for (int r = TM::tid(); r < cnt; r += TM::T) {
+        double *x = X + r * ldx;
+        for (int i = 0; i < n; ++i) {
+            const int p = piv[i];
+            const double t = x[i];
+            x[i] = x[p];
+            x[p] = t;
+        }
+    }
+}
+
+// Rtrsm('L', LOWER ? 'L' : 'U', 'N') on the columns X: b_i - b_k*a_ik for the rows of one step,
+// then (non-unit) the next row's division (Rtrsm.cpp:127, 145; a zero is left alone, as the
+// reference skips it).  A thread has row `row` of every RG-th right-hand side: few rows leave
+// threads over, which take other right-hand sides (a thread per row alone, whatever the
+// number of right-hand sides, took 4.0 ms for an LU of n = 33 with 300 of them; this takes 0.36).
+template <class TM, bool LOWER, bool UNIT>
+__device__ __forceinline__ void axpy_solve(const uint32_t *A, size_t lda, int n, double *X, int ldx, int nrhs,
                                            const unsigned char *tab)
+{
+    const int tid = TM::tid();
+    const int W = 2 * n <= TM::T ? n : TM::T, RG = TM::T / W;
+    const int row = tid % W, r0 = tid / W < RG ? tid / W : nrhs;
+    auto col_of = [&](int st) { return LOWER ? st : n - 1 - st; };
+    // a step's first coefficient and the next division's a_ii are loaded a step ahead
+    uint32_t cur = row < n ? A[row + (size_t)col_of(0) * lda] : 0u, dn = UNIT ? 0u : A[(size_t)col_of(0) * (lda + 1)];
+    for (int st = 0; st < n; ++st) {
+        const int k = col_of(st), kn = col_of(st + 1);
+        const bool more = st + 1 < n;
+        if (!UNIT) {
+            const double d = pd(dn), rc = 1.0 / d;
+            TM::sync(); // row k is up to date
+            for (int r = tid; r < nrhs; r += TM::T) {
+                double *x = X + r * ldx;
+                if (x[k] != 0.0)
+                    x[k] = f64_posit_div(x[k], d, rc);
+            }
+            dn = more ? A[(size_t)kn * (lda + 1)] : 0u;
+        }
+        TM::sync();
+        const uint32_t *ak = A + (size_t)k * lda;
+        const uint32_t nxt = more && row < n ? A[row + (size_t)kn * lda] : 0u;
+#pragma unroll 1
+        for (int i = row; i < n; i += W) {
+            if (LOWER ? i <= k : i >= k)
+                continue;
+            const double l = pd(i == row ? cur : ak[i]);
+            constexpr int U = 4;
+            int r = r0;
+#pragma unroll 1
+            for (; r + (U - 1) * RG < nrhs; r += U * RG) { // several at once, tested together
+                double y[U];
+                bool bad = false;
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    const double *x = X + (r + q * RG) * ldx;
+                    y[q] = step_one(x[i], -x[k], l, tab);
+                    bad |= y[q] != y[q];
+                }
+                if (bad)
+                    break; // the rest one by one
+#pragma unroll
+                for (int q = 0; q < U; ++q)
+                    X[(r + q * RG) * ldx + i] = y[q];
+            }
+#pragma unroll 1
+            for (; r < nrhs; r += RG) {
+                double *x = X + r * ldx;
+                const double xk = x[k];
+                if (xk != 0.0) // zero multipliers skipped (Rtrsm.cpp:125-126, 143-144)
+                    x[i] = mac_any(x[i], -xk, l, tab);
+            }
+        }
+        cur = nxt;
+    }
+    TM::sync();
+}
+
+constexpr int AXPY_FEW = 4;
+constexpr int B_PRE = 2; // rows per thread whose coefficients are loaded a step ahead
+// The same for up to AXPY_FEW right-hand sides by a CTA: a thread per row, no other barrier than
+// the step's; the thread with row `next` divides it when it has updated it.
+template <class C, bool LOWER, bool UNIT>
+__device__ __forceinline__ void axpy_few(const uint32_t *A, size_t lda, int n, double *X, int ldx, int nrhs,
+                                         const unsigned char *tab)
 {
     const int tid = threadIdx.x;
     auto col_of = [&](int st) { return LOWER ? st : n - 1 - st; };
     auto finish = [&](int i) {
         const double d = pd(A[i + (size_t)i * lda]), rc = 1.0 / d;
         for (int r = 0; r < nrhs; ++r) {
-            double *x = X + (size_t)r * n;
+            double *x = X + r * ldx;
             if (x[i] != 0.0)
                 x[i] = f64_posit_div(x[i], d, rc);
         }
@@ -477,7 +602,7 @@ __device__ __forceinline__ void axpy_solve(const uint32_t *A, size_t lda, int n,
             if (LOWER ? i > k : i < k) {
                 const double l = pd(a);
                 for (int r = 0; r < nrhs; ++r) {
-                    double *x = X + (size_t)r * n;
+                    double *x = X + r * ldx;
                     const double xk = x[k];
                     if (xk != 0.0) // zero multipliers skipped (Rtrsm.cpp:125-126, 143-144)
                         x[i] = mac_any(x[i], -xk, l, tab);
@@ -500,76 +625,138 @@ __device__ __forceinline__ void axpy_solve(const uint32_t *A, size_t lda, int n,
     }
 }
 
-// The right-hand sides: Rgetrs('N') or Rpotrs('L').
-template <class C, bool LU>
+// Rtrsm('L', 'L', 'T') (Rtrsm.cpp:175-186) on one column x by one thread: t = b_i,
+// t = t - a_ki*b_k for k = i+1 .. n-1 in order, b_i = t / a_ii.  `coef(k, i)` is a_ki in FP64.
+// Eight steps are tested together, the next eight's coefficients loaded meanwhile.
+template <class Coef>
+__device__ __forceinline__ void thread_llt(double *x, int n, Coef coef, const unsigned char *tab)
+{
+    constexpr int U = 8;
+#pragma unroll 1
+    for (int i = n - 1; i >= 0; --i) {
+        double t = x[i], a[U], an[U];
+        const double d = coef(i, i), rc = 1.0 / d;
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            an[q] = coef(min(i + 1 + q, n - 1), i);
+#pragma unroll 1
+        for (int k = i + 1; k < n; k += U) {
+#pragma unroll
+            for (int q = 0; q < U; ++q)
+                a[q] = an[q];
+            if (k + U < n) {
+#pragma unroll
+                for (int q = 0; q < U; ++q)
+                    an[q] = coef(min(k + U + q, n - 1), i);
+            }
+            const double t0 = t;
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const double r = step_one(t, -x[min(k + q, n - 1)], a[q], tab);
+                t = k + q < n ? r : t;
+            }
+            if (t != t) {
+                t = t0;
+#pragma unroll 1
+                for (int q = k; q < min(k + U, n); ++q)
+                    t = mac_any(t, -x[q], coef(q, i), tab);
+            }
+        }
+        x[i] = f64_posit_div(t, d, rc);
+    }
+}
+
+// Whether the L^T solve of `nrhs` columns goes by a thread each (thread_llt, up to `threads` at a
+// time) instead of a warp each (`warps` at a time) or, `block`, the CTA for one after the other.
+// In ns, measured: a thread's chain 70 n^2 and a little (n = 64 290 us, 128 1150), a warp's solve
+// 1900 n + 7.5 n^2 (64 150, 200 770), a CTA's 1400 n + 4.5 n^2.  n = 64: 16 columns 440 us by warps and
+// 487 by threads, 100 columns 1851 and 562.
+__device__ __forceinline__ bool llt_by_thread(int n, int nrhs, int threads, int warps, bool block)
+{
+    const long long by_thread = (long long)((nrhs + threads - 1) / threads) * n * 80;
+    const long long other = block ? nrhs * (1400 + n * 9 / 2)
+                                  : (long long)((nrhs + warps - 1) / warps) * (1900 + n * 15 / 2);
+    return by_thread < other;
+}
+
+// The right-hand sides: Rgetrs('N') or Rpotrs('L').  MANY: any number of them, else a few
+// (batch_many_rhs).
+template <class C, bool LU, bool MANY>
 __device__ __forceinline__ void solve_one(const BatchProblem &pr, unsigned char *smem, BatchShared &s)
 {
+    using TM = Team<C::T>;
     const int n = pr.n, tid = threadIdx.x;
+    const size_t lda = (size_t)pr.lda, ldb = (size_t)pr.ldb;
     const unsigned char *tab = smem;
     unsigned char *area = smem + STEP_TAB_BYTES + C::U_BYTES;
     double *X = reinterpret_cast<double *>(area);
-    const int group = max(1, (int)((C::AREA_BYTES - 4 * (size_t)n) / (8 * (size_t)n)));
+    const int ldx = MANY ? n | 1 : n; // odd: a thread per column meets no bank conflicts
+    const int group = max(1, (int)((C::AREA_BYTES - 4 * (size_t)n) / (8 * (size_t)ldx)));
+    // L^T backward.  Few right-hand sides: one after the other, a warp adding and the others
+    // forming terms; more: a warp for each, as many at a time as fit; short columns or many
+    // of them: a thread for each.
+    const size_t one = 2 * ChainTerms64::bytes(n) + (size_t)n * 8;
+    const size_t per = ChainTerms64::bytes(n) + (((size_t)n * 8 + 15) & ~(size_t)15);
+    const bool by_block = pr.nrhs <= 2 && one <= (size_t)C::AREA_BYTES;
+    const int warps = min(C::T / 32, (int)(C::AREA_BYTES / per));
+    const bool by_thread = MANY && !LU && llt_by_thread(n, pr.nrhs, min(group, C::T), warps, by_block);
     for (int r0 = 0; r0 < pr.nrhs; r0 += group) {
         const int cnt = min(group, pr.nrhs - r0);
-        uint32_t *B = pr.B + (size_t)r0 * pr.ldb;
-        for (int r = 0; r < cnt; ++r)
-            for (int i = tid; i < n; i += C::T)
-                X[(size_t)r * n + i] = pd(B[(size_t)r * pr.ldb + i]);
-        if (LU) { // Rlaswp, in order, a thread per column
-            int *piv = reinterpret_cast<int *>(X + (size_t)cnt * n);
+        uint32_t *B = pr.B + r0 * ldb;
+        load_rhs<TM, MANY>(X, ldx, B, ldb, n, cnt);
+        if (LU) {
+            int *piv = reinterpret_cast<int *>(X + (size_t)cnt * ldx);
             for (int i = tid; i < n; i += C::T)
                 piv[i] = pr.ipiv[i] - 1;
             __syncthreads();
-            for (int r = tid; r < cnt; r += C::T) {
-                double *x = X + (size_t)r * n;
-                for (int i = 0; i < n; ++i) {
-                    const int p = piv[i];
-                    const double t = x[i];
-                    x[i] = x[p];
-                    x[p] = t;
-                }
-            }
+            swap_rhs<TM>(X, ldx, piv, n, cnt);
         }
         __syncthreads();
-        axpy_solve<C, true, LU>(pr.A, (size_t)pr.lda, n, X, cnt, tab);
-        if (LU)
-            axpy_solve<C, false, false>(pr.A, (size_t)pr.lda, n, X, cnt, tab);
-        for (int r = 0; r < cnt; ++r)
-            for (int i = tid; i < n; i += C::T)
-                B[(size_t)r * pr.ldb + i] = p32_from_double_exact(X[(size_t)r * n + i]);
+        if (!MANY || cnt <= AXPY_FEW) {
+            axpy_few<C, true, LU>(pr.A, lda, n, X, ldx, cnt, tab);
+            if (LU)
+                axpy_few<C, false, false>(pr.A, lda, n, X, ldx, cnt, tab);
+        } else {
+            axpy_solve<TM, true, LU>(pr.A, lda, n, X, ldx, cnt, tab);
+            if (LU)
+                axpy_solve<TM, false, false>(pr.A, lda, n, X, ldx, cnt, tab);
+        }
+        if (by_thread) {
+            const uint32_t *A = pr.A;
+            for (int r = tid; r < cnt; r += C::T)
+                thread_llt(X + r * ldx, n, [=](int k, int i) { return pd(A[k + i * lda]); }, tab);
+            __syncthreads();
+        }
+        store_rhs<TM, MANY>(X, ldx, B, ldb, n, cnt);
         __syncthreads();
     }
-    if (LU)
+    if (LU || by_thread)
         return;
-    // L^T backward.  Few right-hand sides: one after the other, a warp adding and the others
-    // forming terms; more: a warp for each, as many at a time as fit.
-    const size_t one = 2 * ChainTerms64::bytes(n) + (size_t)n * 8;
-    if (pr.nrhs <= 2 && one <= (size_t)C::AREA_BYTES) {
+    if (by_block) {
         LtxCol64 x;
         x.b = reinterpret_cast<double *>(area + 2 * ChainTerms64::bytes(n));
         for (int r = 0; r < pr.nrhs; ++r) {
-            uint32_t *b = pr.B + (size_t)r * pr.ldb;
+            uint32_t *b = pr.B + r * ldb;
             for (int i = tid; i < n; i += C::T)
                 x.set(i, pd(b[i]));
-            block_ltx_solve<C::T, false, ChainTerms64>(pr.A, (size_t)pr.lda, x, n, false, area, s.ltx);
+            block_ltx_solve<C::T, false, ChainTerms64>(pr.A, lda, x, n, false, area, s.ltx);
             for (int i = tid; i < n; i += C::T)
                 b[i] = p32_from_double_exact(x.get(i));
             __syncthreads();
         }
         return;
     }
-    const size_t per = ChainTerms64::bytes(n) + (((size_t)n * 8 + 15) & ~(size_t)15);
-    const int warps = min(C::T / 32, (int)(C::AREA_BYTES / per)), warp = tid >> 5, lane = tid & 31;
+    const int warp = tid >> 5, lane = tid & 31;
     if (warp < warps) {
         ChainTerms64 q;
         q.q = reinterpret_cast<double *>(area + warp * per);
         double *x = reinterpret_cast<double *>(area + warp * per + ChainTerms64::bytes(n));
         for (int r = warp; r < pr.nrhs; r += warps) {
-            uint32_t *b = pr.B + (size_t)r * pr.ldb;
+            uint32_t *b = pr.B + r * ldb;
             for (int i = lane; i < n; i += 32)
                 x[i] = pd(b[i]);
             __syncwarp();
-            warp_llt_solve(pr.A, (size_t)pr.lda, x, n, q);
+            warp_llt_solve(pr.A, lda, x, n, q);
             for (int i = lane; i < n; i += 32)
                 b[i] = p32_from_double_exact(x[i]);
             __syncwarp();
@@ -582,16 +769,17 @@ __device__ __forceinline__ void solve_one(const BatchProblem &pr, unsigned char 
 // ---------------------------------------------------------------------------
 // A CTA's barriers cost such a problem more than its arithmetic; eight of them run side by
 // side in a CTA instead.
-constexpr int SMALL_N = 32;
+constexpr int SMALL_N = BATCH_WARP_N;
 constexpr int SMALL_LD = SMALL_N + 1;
 struct SmallArea {
-    double a[SMALL_N * SMALL_LD]; // a_ic at [c * SMALL_LD + i]
+    double a[SMALL_N * SMALL_LD + SMALL_N]; // a_ic at [c * SMALL_LD + i]; then, many right-hand sides
     double x[SMALL_N];
-    double terms[36]; // ChainTerms64 of 32
     int piv[SMALL_N];
 };
-static_assert(ChainTerms64::GROUP_DOUBLES * (SMALL_N / 16) == 36, "");
 static_assert(sizeof(SmallArea) * (SmallCfg::T / 32) <= SmallCfg::U_BYTES + SmallCfg::AREA_BYTES, "a problem per warp");
+// From this many right-hand sides on they go through side by side.  n = 24, three and four of them:
+// LU 85 us one by one and 97 side by side, 94 / 84; Cholesky 144 / 133, 174 / 127.
+constexpr int SMALL_MANY_LU = 4, SMALL_MANY_CHOL = 3;
 
 template <bool LU>
 __device__ __forceinline__ int small_factor(SmallArea &w, int n, const unsigned char *tab)
@@ -659,7 +847,7 @@ __device__ __forceinline__ int small_factor(SmallArea &w, int n, const unsigned 
     return info;
 }
 
-template <bool LU>
+template <bool LU, bool MANY>
 __device__ __forceinline__ void run_small(const BatchProblem &pr, SmallArea &w, const unsigned char *tab)
 {
     constexpr unsigned FULL = 0xFFFFFFFFu;
@@ -685,6 +873,31 @@ __device__ __forceinline__ void run_small(const BatchProblem &pr, SmallArea &w, 
             w.piv[lane] = pr.ipiv[lane] - 1;
     }
     __syncwarp();
+    if (MANY && pr.nrhs >= (LU ? SMALL_MANY_LU : SMALL_MANY_CHOL)) {
+        using TM = Team<32>;
+        const int ldx = n | 1, group = (int)(sizeof(w.a) / sizeof(double)) / ldx;
+        const uint32_t *A = pr.A; // the factor, from global memory: X takes its place
+        for (int r0 = 0; r0 < pr.nrhs; r0 += group) {
+            const int cnt = min(group, pr.nrhs - r0);
+            uint32_t *B = pr.B + (size_t)r0 * pr.ldb;
+            load_rhs<TM, true>(w.a, ldx, B, (size_t)pr.ldb, n, cnt);
+            __syncwarp();
+            if (LU) {
+                swap_rhs<TM>(w.a, ldx, w.piv, n, cnt);
+                __syncwarp();
+            }
+            axpy_solve<TM, true, LU>(A, lda, n, w.a, ldx, cnt, tab);
+            if (LU)
+                axpy_solve<TM, false, false>(A, lda, n, w.a, ldx, cnt, tab);
+            else
+                for (int r = lane; r < cnt; r += 32)
+                    thread_llt(w.a + r * ldx, n, [=](int k, int i) { return pd(A[k + i * lda]); }, tab);
+            __syncwarp();
+            store_rhs<TM, true>(w.a, ldx, B, (size_t)pr.ldb, n, cnt);
+            __syncwarp();
+        }
+        return;
+    }
     double d = 1.0;
     if (lane < n)
         d = w.a[lane * SMALL_LD + lane];
@@ -716,9 +929,10 @@ __device__ __forceinline__ void run_small(const BatchProblem &pr, SmallArea &w, 
         } else {
             w.x[lane] = x;
             __syncwarp();
-            ChainTerms64 q;
-            q.q = w.terms;
-            warp_llt_solve(pr.A, lda, w.x, n, q);
+            const double *a = w.a;
+            if (lane == 0)
+                thread_llt(w.x, n, [=](int k, int i) { return a[i * SMALL_LD + k]; }, tab);
+            __syncwarp();
             x = w.x[lane];
             __syncwarp();
         }
@@ -727,7 +941,7 @@ __device__ __forceinline__ void run_small(const BatchProblem &pr, SmallArea &w, 
     }
 }
 
-template <class C, bool LU>
+template <class C, bool LU, bool MANY>
 __device__ __forceinline__ void run_one(const BatchProblem &pr, unsigned char *smem, BatchShared &s)
 {
     int info = 0;
@@ -738,16 +952,17 @@ __device__ __forceinline__ void run_one(const BatchProblem &pr, unsigned char *s
         __syncthreads();
     }
     if (pr.n > 0 && pr.nrhs > 0 && (LU || info == 0))
-        solve_one<C, LU>(pr, smem, s);
+        solve_one<C, LU, MANY>(pr, smem, s);
 }
 
 } // namespace
 
-// The problems [first, last) of the list, from the queue `next` (which counts from 0).
-template <class C>
+// The problems [first, last) of the list, from the queue `next` (which counts from 0); from
+// warp_from on a warp takes each.
+template <class C, bool MANY>
 __global__ void __launch_bounds__(C::T, 512 / C::T) batch_factor_kernel(const BatchProblem *__restrict__ probs, int first,
                                                                         int last, const int *__restrict__ order,
-                                                                        int *__restrict__ next)
+                                                                        int warp_from, int *__restrict__ next)
 {
     extern __shared__ __align__(128) unsigned char smem_batch[];
     __shared__ BatchShared s;
@@ -762,7 +977,7 @@ __global__ void __launch_bounds__(C::T, 512 / C::T) batch_factor_kernel(const Ba
         if (item >= last)
             return;
         const BatchProblem pr = probs[order ? order[item] : item];
-        if (C::T == SmallCfg::T && order && pr.n <= SMALL_N) { // sorted: so are all that follow
+        if (C::T == SmallCfg::T && item >= warp_from) {
             SmallArea &w = reinterpret_cast<SmallArea *>(smem_batch + STEP_TAB_BYTES)[threadIdx.x >> 5];
             const bool lead = (threadIdx.x & 31) == 0;
             auto take = [&]() { return __shfl_sync(0xFFFFFFFFu, lead ? first + atomicAdd(next, 1) : 0, 0); };
@@ -770,9 +985,9 @@ __global__ void __launch_bounds__(C::T, 512 / C::T) batch_factor_kernel(const Ba
                 const BatchProblem ps = probs[order[mine]];
                 if (ps.n > 0) {
                     if ((ps.kind & 1) == BATCH_LU)
-                        run_small<true>(ps, w, smem_batch);
+                        run_small<true, MANY>(ps, w, smem_batch);
                     else
-                        run_small<false>(ps, w, smem_batch);
+                        run_small<false, MANY>(ps, w, smem_batch);
                     __syncwarp();
                 } else if (lead && !(ps.kind & BATCH_SOLVE_ONLY)) {
                     *ps.info = 0;
@@ -781,34 +996,37 @@ __global__ void __launch_bounds__(C::T, 512 / C::T) batch_factor_kernel(const Ba
             return;
         }
         if ((pr.kind & 1) == BATCH_LU)
-            run_one<C, true>(pr, smem_batch, s);
+            run_one<C, true, MANY>(pr, smem_batch, s);
         else
-            run_one<C, false>(pr, smem_batch, s);
+            run_one<C, false, MANY>(pr, smem_batch, s);
         __syncthreads();
     }
 }
 
-template <class C>
-static cudaError_t launch_cfg(const BatchProblem *probs, int first, int last, const int *order, int *next, int ctas,
-                              cudaStream_t st)
+template <class C, bool MANY>
+static cudaError_t launch_cfg(const BatchProblem *probs, int first, int last, const int *order, int warp_from, int *next,
+                              int ctas, cudaStream_t st)
 {
-    cudaError_t e = cudaFuncSetAttribute(batch_factor_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(batch_factor_kernel<C, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(next, 0, sizeof(int), st);
     if (e != cudaSuccess)
         return e;
     const int count = last - first;
-    batch_factor_kernel<C><<<count < ctas ? count : ctas, C::T, C::SMEM, st>>>(probs, first, last, order, next);
+    batch_factor_kernel<C, MANY><<<count < ctas ? count : ctas, C::T, C::SMEM, st>>>(probs, first, last, order, warp_from, next);
     return cudaGetLastError();
 }
 
-cudaError_t batch_factor_launch(bool large, const BatchProblem *probs, int first, int last, const int *order, int *next,
-                                int sms, cudaStream_t st)
+cudaError_t batch_factor_launch(bool large, bool many, const BatchProblem *probs, int first, int last, const int *order,
+                                int warp_from, int *next, int sms, cudaStream_t st)
 {
     if (last <= first)
         return cudaSuccess;
-    return large ? launch_cfg<LargeCfg>(probs, first, last, order, next, sms, st)
-                 : launch_cfg<SmallCfg>(probs, first, last, order, next, 2 * sms, st);
+    if (large)
+        return many ? launch_cfg<LargeCfg, true>(probs, first, last, order, warp_from, next, sms, st)
+                    : launch_cfg<LargeCfg, false>(probs, first, last, order, warp_from, next, sms, st);
+    return many ? launch_cfg<SmallCfg, true>(probs, first, last, order, warp_from, next, 2 * sms, st)
+                : launch_cfg<SmallCfg, false>(probs, first, last, order, warp_from, next, 2 * sms, st);
 }
 
 } // namespace pg

@@ -9,6 +9,17 @@ constexpr int BATCH_LU = 0;
 constexpr int BATCH_CHOL = 1;
 constexpr int BATCH_MAX_N = 4096; // largest n a batched problem may have
 constexpr int BATCH_LARGE_N = 224;  // a problem of more rows takes an SM for itself
+constexpr int BATCH_WARP_N = 32;    // a problem of up to this many rows may be a warp's
+// From this many right-hand sides on a warp is the slower place for such a problem, unless there
+// are so many of them that CTAs take more than three turns.  One problem of n = 32 with 300 right-hand
+// sides: 1520 us by a warp, 462 by a CTA; 2000 of them: 2571 us by warps, about 3400 by CTAs.
+constexpr int BATCH_WARP_RHS = 16;
+constexpr int BATCH_CTA_TURNS = 3;
+// Whether a problem needs the kernels that spread right-hand sides over the threads (up to 4 pay
+// a thread per row, up to 2 a warp's turns).  Launches without one take kernels without that
+// code: with it in, the compiler spills more in the factorization, and an LU of n = 512 takes
+// 9.1 ms instead of 8.2.
+inline bool batch_many_rhs(int n, int nrhs) { return nrhs > (n > BATCH_WARP_N ? 4 : 2); }
 
 // One problem: A (n x n, column-major, lda) is factored in place, B (n x nrhs, ldb)
 // overwritten with the solution; ipiv (LU) receives n 1-based pivots, info the
@@ -26,9 +37,10 @@ struct BatchProblem {
 
 // Runs problems probs[order[i]] (order null: probs[i]), first <= i < last, on persistent CTAs;
 // `order` sorts by decreasing n.  `large`: one CTA per SM (problems of more than
-// BATCH_LARGE_N rows), else two smaller ones.  `next` is a device counter the launch zeroes
-// first.  A null order may be in any order, of any sizes.
-cudaError_t batch_factor_launch(bool large, const BatchProblem *probs, int first, int last, const int *order, int *next,
-                                int sms, cudaStream_t st);
+// BATCH_LARGE_N rows), else two smaller ones; those from warp_from on (of up to BATCH_WARP_N
+// rows) go to a warp each.  `many`: there is one of batch_many_rhs.  `next` is a device counter
+// the launch zeroes first.  A null order may be in any order, of any sizes, with warp_from = last.
+cudaError_t batch_factor_launch(bool large, bool many, const BatchProblem *probs, int first, int last, const int *order,
+                                int warp_from, int *next, int sms, cudaStream_t st);
 
 } // namespace pg

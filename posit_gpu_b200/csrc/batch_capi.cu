@@ -36,6 +36,37 @@ static void plan_free(posit_batch_plan *p)
     delete p;
 }
 
+// The order in which a plan takes its problems: the largest first (work grows like n^3), those
+// that go to a warp each (batch.cuh) last.  [0, nlarge) are the large ones, [warp_from, nprob)
+// the warps'.
+static void batch_order(const posit_batch_problem *probs, int nprob, int sms, std::vector<int> &order, int &nlarge,
+                        int &warp_from)
+{
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return probs[a].n > probs[b].n; });
+    nlarge = 0;
+    while (nlarge < nprob && probs[order[nlarge]].n > pg::BATCH_LARGE_N)
+        ++nlarge;
+    auto many_rhs = [&](int i) { return probs[i].n <= pg::BATCH_WARP_N && probs[i].nrhs >= pg::BATCH_WARP_RHS; };
+    const bool crowd = std::count_if(order.begin(), order.end(), many_rhs) > (long)pg::BATCH_CTA_TURNS * 2 * sms;
+    auto by_cta = [&](int i) { return probs[i].n > pg::BATCH_WARP_N || (many_rhs(i) && !crowd); };
+    warp_from = (int)(std::stable_partition(order.begin(), order.end(), by_cta) - order.begin());
+}
+
+// How a plan of these problems runs on a GPU of `sms` SMs: route[i] = 0: a CTA that has an SM for
+// itself, 1: one of two CTAs on an SM, 2: a warp.
+extern "C" int posit_batch_plan_routes(const posit_batch_problem *probs, int nprob, int sms, int *route)
+{
+    if (!probs || nprob < 0 || !route)
+        return 1;
+    std::vector<int> order(nprob);
+    int nlarge = 0, warp_from = 0;
+    batch_order(probs, nprob, sms, order, nlarge, warp_from);
+    for (int i = 0; i < nprob; ++i)
+        route[order[i]] = i < nlarge ? 0 : (i < warp_from ? 1 : 2);
+    return 0;
+}
+
 extern "C" int posit_batch_plan_create(const posit_batch_problem *probs, int nprob, posit_batch_plan **out)
 {
     if (!probs || nprob < 0 || !out)
@@ -54,13 +85,11 @@ extern "C" int posit_batch_plan_create(const posit_batch_problem *probs, int npr
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     p->ctas = sms;
-    // largest problems first (work grows like n^3)
     std::vector<int> order(nprob);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return probs[a].n > probs[b].n; });
-    int nlarge = 0;
-    while (nlarge < nprob && probs[order[nlarge]].n > pg::BATCH_LARGE_N)
-        ++nlarge;
+    int nlarge = 0, warp_from = 0;
+    batch_order(probs, nprob, sms, order, nlarge, warp_from);
+    const bool many = std::any_of(probs, probs + nprob,
+                                  [](const posit_batch_problem &q) { return pg::batch_many_rhs(q.n, q.nrhs); });
     cudaError_t e = cudaMalloc((void **)&p->d_probs, sizeof(pg::BatchProblem) * (nprob > 0 ? nprob : 1));
     if (e == cudaSuccess)
         e = cudaMalloc(&p->d_order, sizeof(int) * (nprob > 0 ? nprob : 1));
@@ -91,9 +120,10 @@ extern "C" int posit_batch_plan_create(const posit_batch_problem *probs, int npr
             if (le == cudaSuccess)
                 le = cudaStreamWaitEvent(side, fork, 0);
             if (le == cudaSuccess)
-                le = pg::batch_factor_launch(true, d, 0, nlarge, o, p->d_next, p->ctas, cs);
+                le = pg::batch_factor_launch(true, many, d, 0, nlarge, o, nlarge, p->d_next, p->ctas, cs);
             if (le == cudaSuccess)
-                le = pg::batch_factor_launch(false, d, nlarge, nprob, o, p->d_next + 1, p->ctas, side);
+                le = pg::batch_factor_launch(false, many, d, nlarge, nprob, o, warp_from, p->d_next + 1, p->ctas,
+                                             side);
             if (le == cudaSuccess)
                 le = cudaEventRecord(join, side);
             if (le == cudaSuccess)
