@@ -102,6 +102,9 @@ size_t posit_rgemm_workspace_size(char transa, char transb, int m, int n, int k)
 /* The panel width nb <= 0 selects for an n x n LU (lu = 1) or lower Cholesky (lu = 0);
  * host-only, no device needed. */
 int posit_tuned_panel_width(int lu, int n);
+/* How many CTAs (a thread-block cluster) solve one of nrhs right-hand sides of n rows together
+ * in the axpy-form solves of Rgetrs 'N' and Rpotrs; host-only, no device needed. */
+int posit_solve_cluster_ctas(int n, int nrhs);
 
 /* Rgetrf (libRpack/Rgetrf.cpp:32-137; mplapack_posit.h:48), Rgetrf_opencl (mplapack_posit.h:49) */
 int posit_rgetrf_dev(int m, int n, uint32_t *A, int lda, int *ipiv, int nb, int *info, void *stream);

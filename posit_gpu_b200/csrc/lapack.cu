@@ -849,12 +849,37 @@ __global__ void __launch_bounds__(1024) trsm_long_kernel(const uint32_t *__restr
     }
 }
 
-// One cluster per right-hand side: a CTA per 16 blocks (512 rows), up to 8.
+// CTAs of a right-hand side's cluster: up to one per 16 blocks (512 rows) and 8, but not so many
+// that the right-hand sides take more turns for it.  A cluster's time goes as 1 + m / (1800 ctas): its
+// chain of rows, and the updates its CTAs share.  Rgetrs, n = 4096: one right-hand side 3.1 ms with 8
+// CTAs, 4.1 with 4, 8.0 with 1; 1024 of them 204 ms with 8, 123 with 4, 55 with 1 (107 in the
+// form before this one, a CTA each); n = 2048, 1024 of them: 47 ms with 4, 18 with 1.
+int solve_cluster_ctas(int m, int nrhs)
+{
+    // clusters on the GPU at a time by size, one CTA per SM (a cluster lies within one GPC)
+    static const int at_once[COL_MAX_CTAS + 1] = {0, 148, 74, 44, 32, 20, 20, 15, 15};
+    const int nb = (m + COL_BLK - 1) / COL_BLK;
+    const int most = std::max(1, std::min(COL_MAX_CTAS, (nb + COL_WARPS - 1) / COL_WARPS));
+    int best = most;
+    double best_cost = 0.0;
+    for (int c = most; c >= 1; --c) {
+        if (c < most && col_smem_bytes(nb, c, std::min(COL_WARPS, (nb + c - 1) / c)) > COL_SMEM_MAX)
+            break; // long columns: fewer CTAs would hold fewer warps
+        const double cost = (double)((nrhs + at_once[c] - 1) / at_once[c]) * (1.0 + m / (1800.0 * c));
+        if (c == most || cost < best_cost) {
+            best = c;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+// One cluster per right-hand side.
 static cudaError_t launch_col(bool upper, bool unit, int nrhs, const uint32_t *A, size_t lda, uint32_t *B, size_t ldb,
                               int m, const int *info, cudaStream_t st)
 {
     const int nb = (m + COL_BLK - 1) / COL_BLK;
-    const int ncta = std::min(COL_MAX_CTAS, (nb + COL_WARPS - 1) / COL_WARPS);
+    const int ncta = solve_cluster_ctas(m, nrhs);
     auto *fn = upper ? (unit ? trsm_block_kernel<true, true> : trsm_block_kernel<true, false>)
                      : (unit ? trsm_block_kernel<false, true> : trsm_block_kernel<false, false>);
     // no more warps than a CTA has blocks (nor, for the longest columns, than fit)

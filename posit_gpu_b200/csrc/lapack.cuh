@@ -19,6 +19,8 @@ size_t rpotrf_workspace_bytes(int n, int nb);
 cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb, int *info, void *ws,
                           cudaStream_t st, int max_ctas = 0);
 cudaError_t rpotrf_lower_launch(int n, uint32_t *A, int lda, int nb, int *info, void *ws, cudaStream_t st);
+// CTAs that solve one of nrhs right-hand sides of m rows together (axpy-form solves).
+int solve_cluster_ctas(int m, int nrhs);
 cudaError_t rgetrs_launch(int n, int nrhs, const uint32_t *A, int lda, const int *ipiv, uint32_t *B, int ldb,
                           cudaStream_t st);
 cudaError_t rpotrs_lower_launch(int n, int nrhs, const uint32_t *A, int lda, uint32_t *B, int ldb,
