@@ -76,6 +76,10 @@ int posit_rgemm_dev_noalloc(char transa, char transb, int m, int n, int k, uint3
 
 /* Bytes of device workspace posit_rgemm_dev needs for this shape (0 when none). */
 size_t posit_rgemm_workspace_size(char transa, char transb, int m, int n, int k);
+/* How an m x n x k product on matrices that do not overlap is computed: 0 staged (operands
+ * converted into the workspace first), 1 and 2 in one launch by tiles of 64x32 and 32x32;
+ * -1 for no product.  The bits are the same.  Host-only, no device needed. */
+int posit_rgemm_route(int m, int n, int k);
 
 /* ---- Device-resident factorizations and solves ------------------------------------
  * Bit-identical to the reference's CPU Rgetrf / Rgetrs / Rpotrf / Rpotrs (at any block

@@ -164,6 +164,13 @@ size_t posit_rgemm_workspace_size(char transa, char transb, int m, int n, int k)
     return pg::gemm_workspace_bytes(m, n, k);
 }
 
+int posit_rgemm_route(int m, int n, int k)
+{
+    if (m <= 0 || n <= 0 || k <= 0)
+        return -1;
+    return (int)pg::gemm_route(true, true, m, n, k, nullptr, m, nullptr, k, nullptr, m, true);
+}
+
 int posit_rgemm_dev(char transa, char transb, int m, int n, int k, uint32_t alpha, const uint32_t *A,
                     int lda, const uint32_t *B, int ldb, uint32_t beta, uint32_t *C, int ldc, void *workspace,
                     size_t workspace_bytes, void *stream)

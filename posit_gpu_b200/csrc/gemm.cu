@@ -10,19 +10,20 @@
 // operand prescale (alpha*B for NN/NT), the accumulator's start value and the
 // epilogue.  Two routes, the same k-step (gemm_tile.cuh) and the same bits:
 //
-//  * staged (large products, see gemm_route): a pre-pass converts op(A) and op(B) (times alpha for NN/NT,
+//  * staged (see gemm_route): a pre-pass converts op(A) and op(B) (times alpha for NN/NT,
 //    rounded exactly as the reference rounds alpha*b_lj) ONCE per element to FP64 (posit32
 //    values are exact there) into a workspace of 32 x 16 blocks, [block][k-tile][l][32],
 //    plus a NaR flag per row and column; transposition is absorbed here.  The main kernel,
 //    one CTA of 256 threads per 64x64 tile of C, 2 CTAs per SM, brings each k tile's four
 //    4 KB blocks into shared memory by the bulk-copy (TMA) engine (cp.async.bulk + mbarrier
 //    transaction counts, 3 stages, every wait bounded);
-//  * fused (small products): one launch, no workspace; a CTA reads the patterns of its own
+//  * fused (small and skinny products): one launch, no workspace; a CTA reads the patterns of its own
 //    operand blocks and converts them itself (gemm_tile.cuh, fused_tile).
 #include "gemm.cuh"
 #include "gemm_tile.cuh"
 #include "posit32.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <vector>
@@ -392,18 +393,32 @@ GemmRoute gemm_route(bool nota, bool notb, int m, int n, int k, const uint32_t *
         (spans_overlap(C, span(m, n, ldc), A, nota ? span(m, k, lda) : span(k, m, lda)) ||
          spans_overlap(C, span(m, n, ldc), B, notb ? span(k, n, ldb) : span(n, k, ldb))))
         return GEMM_STAGED;
-    const long long t44 = ceil_div(m, 64) * ceil_div(n, 64), t42 = ceil_div(m, 64) * ceil_div(n, 32),
-                    t22 = ceil_div(m, 32) * ceil_div(n, 32);
-    // From 2^24 multiply-adds on 100 tiles the second launch is worth it: 1024 x 1024 x 24 39.9
-    // against 44.4 us fused, 2048^2 x 32 121 / 125, 1000 x 1000 x 500 356 / 418, 700^3 272 / 301.
-    if (t44 >= GEMM_STAGED_MIN_TILES && (double)m * n * k >= GEMM_STAGED_MIN_MADS)
+    // A call's time on each route: launches (and the conversion pre-pass), then the tiles of the
+    // fullest SM, one after the other as far as the FP64 issue slots go; an SM with one or two tiles
+    // does not hide their latencies and takes a little longer for each.  Fitted to 895 shapes (k to
+    // 8192; m = n to 8128; n = 1 to 512 by m to 100,000 and the reverse), each timed on all three
+    // routes: the route it names is 0.4 % slower than the best on average, at most 8 %.  Edge
+    // tiles count as whole ones, which is what they cost: 12800 x 32 x 512 staged 397 us, 64x32 226,
+    // 32x32 197; 16384 x 1 x 1024 staged 780, 64x32 433; 3200 x 129 x 512 371 / 226 / 257; 1371 x 400
+    // x 32 47 / 26 / 29.  Full tiles in numbers are staged: 1024^2 x 300 228 / 258 / 257, 2500^2
+    // x 300 1117 / 1297 / 1474.
+    struct Cost {
+        double call, per_k, per_tile; // us
+        double one, two, more;        // an SM's tiles, in tiles: one, two, or t + more
+        double of(long long tiles, int k) const
+        {
+            const long long t = ceil_div(tiles, SM_COUNT);
+            return call + (t == 1 ? one : t == 2 ? two : (double)t + more) * (per_k * k + per_tile);
+        }
+    };
+    static const Cost staged = {20.4, 0.3172, 3.83, 1.17, 2.12, 0.25}, f64x32 = {10.4, 0.1834, 1.73, 1.50, 2.22, 0.30},
+                      f32x32 = {10.1, 0.1076, 0.96, 1.57, 2.43, 0.31};
+    if (ceil_div(n, 32) > 65535) // columns of 32-wide tiles: more than a grid has in y
         return GEMM_STAGED;
-    // 64x32 tiles where there are so many that waves don't matter (1400^2 x 8 26.8 us against 28.9 in
-    // 32x32, 4000 x 1000 x 4 41.2 / 43.9, 1100^2 x 12 22.7 / 22.7) or they take one wave where 32x32
-    // tiles take two (4000 x 128 x 32 20.7 / 22.7); else 32x32 (640^2 x 32 17.5 against 20.7, 576^2
-    // x 512 191 / 219, 640 x 576 x 700 260 / 298).  64x64 tiles were slower throughout (1200^2 x 8 30.0).
-    const bool many = t42 >= 4 * SM_COUNT, one_wave = t42 <= 2 * SM_COUNT && t22 > 3 * SM_COUNT;
-    return many || one_wave ? GEMM_FUSED_64x32 : GEMM_FUSED_32x32;
+    const double cs = staged.of(ceil_div(m, 64) * ceil_div(n, 64), k),
+                 c42 = f64x32.of(ceil_div(m, 64) * ceil_div(n, 32), k),
+                 c22 = f32x32.of(ceil_div(m, 32) * ceil_div(n, 32), k);
+    return cs < std::min(c42, c22) ? GEMM_STAGED : (c42 < c22 ? GEMM_FUSED_64x32 : GEMM_FUSED_32x32);
 }
 
 template <class Kernel>

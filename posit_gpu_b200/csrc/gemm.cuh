@@ -19,8 +19,6 @@ constexpr int SM_COUNT = 148;
 
 // How a product is computed (gemm_route); the bits are the same.
 enum GemmRoute { GEMM_STAGED, GEMM_FUSED_64x32, GEMM_FUSED_32x32 };
-constexpr double GEMM_STAGED_MIN_MADS = 16777216.0; // 2^24 multiply-adds
-constexpr long long GEMM_STAGED_MIN_TILES = 100;
 
 // Error flags a kernel can raise (read back with posit_get_device_error).
 constexpr int DEV_ERR_WAIT_TIMEOUT = 1;
