@@ -210,9 +210,17 @@ int posit_rgemm(char transa, char transb, int m, int n, int k, uint32_t alpha, c
                           : 1;
     const int w = parts > 1 ? ((n + parts - 1) / parts + 63) / 64 * 64 : n;
     const size_t na = need_ab ? (size_t)ar * ac : 0, nb = need_ab ? (size_t)br * bc : 0;
-    uint32_t *dev = nullptr;
-    PG_TRY(cudaMallocAsync((void **)&dev, (na + nb + (size_t)m * n) * 4, st));
-    uint32_t *dA = dev, *dB = dev + na, *dC = dev + na + nb;
+    // One allocation for all, the workspace too (if the first or the last stretch is staged): once a
+    // stretch has gone out into C, nothing may be short any more.
+    auto staged = [&](int cols) {
+        return pg::gemm_route(nota, notb, m, cols, k, nullptr, ar, nullptr, br, nullptr, m, true) == pg::GEMM_STAGED;
+    };
+    const bool any_staged = need_ab && (staged(w) || staged(n - (n - 1) / w * w));
+    const size_t ws_bytes = any_staged ? (pg::gemm_workspace_bytes(m, w, k) + 255) / 256 * 256 : 0;
+    unsigned char *dev = nullptr;
+    PG_TRY(cudaMallocAsync((void **)&dev, ws_bytes + (na + nb + (size_t)m * n) * 4, st));
+    uint32_t *dA = reinterpret_cast<uint32_t *>(dev + ws_bytes), *dB = dA + na, *dC = dB + nb;
+    void *ws = ws_bytes ? dev : nullptr;
     cudaStream_t cp = st; // the copies' stream
     cudaEvent_t in = nullptr, out[2] = {nullptr, nullptr};
     cudaError_t e = cudaSuccess;
@@ -243,7 +251,7 @@ int posit_rgemm(char transa, char transb, int m, int n, int k, uint32_t alpha, c
             ok(cudaStreamWaitEvent(st, in, 0));
         if (e == cudaSuccess)
             rc = rgemm_device(nota, notb, m, width(c0), k, alpha, dA, ar, notb ? dB + (size_t)c0 * k : dB + c0, br, beta,
-                              dC + (size_t)c0 * m, m, nullptr, 0, st);
+                              dC + (size_t)c0 * m, m, ws, ws_bytes, st);
         if (parts > 1 && e == cudaSuccess && rc == 0)
             ok(cudaEventRecord(out[c0 / w & 1], st));
     };
