@@ -219,7 +219,8 @@ typedef struct {
     int cache_off;        /* 1: never keep factors */
     int batch_lanes;      /* lanes reserved for batched units; 0 = 4 */
     int order_window_ms;  /* > 0: requests submitted within one window of this many ms are
-                             admitted largest work first, windows in arrival order; 0 = arrival order */
+                             admitted largest work first, windows in arrival order (an idle server
+                             waits until none has come for 0.5 ms before it admits); 0 = arrival order */
     int priority_n;       /* blocked requests with n >= this run on lanes of the device's greatest
                              stream priority (a quarter of the blocked lanes), so the longest
                              requests get SMs first; 0 = POSIT_SERVER_PRIORITY_N, < 0 = none */

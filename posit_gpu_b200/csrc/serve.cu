@@ -522,6 +522,36 @@ void order_pending(posit_server *s)
     });
 }
 
+// With an order window, a server that has nothing else to do lets the burst a request belongs to
+// come in before it admits: until no request has come for BURST_QUIET_MS, BURST_MOST_MS (or the
+// window) at most.  Otherwise the first request of a burst, of whatever size, goes ahead of all:
+// always where the server was idle, and where the request before it ends between two submissions.
+constexpr double BURST_QUIET_MS = 0.5, BURST_MOST_MS = 5.0;
+void gather_burst(posit_server *s)
+{
+    if (s->order_window_ms <= 0.0 || s->inflight > 0)
+        return;
+    const Clock::time_point start = Clock::now();
+    const double most = std::min(BURST_MOST_MS, s->order_window_ms);
+    while (!s->pending.empty()) {
+        Clock::time_point newest = s->pending.front()->t_submit;
+        for (const Req &r : s->pending)
+            newest = std::max(newest, r->t_submit);
+        const Clock::time_point now = Clock::now();
+        const double left = std::min(BURST_QUIET_MS - ms_between(newest, now), most - ms_between(start, now));
+        if (left <= 0.0)
+            return;
+        std::unique_lock<std::mutex> lk(s->mu);
+        s->cv_work.wait_for(lk, std::chrono::duration<double, std::milli>(left),
+                            [&] { return s->stop || !s->incoming.empty(); });
+        if (s->stop)
+            return; // the loop sees to it
+        for (auto &r : s->incoming)
+            s->pending.push_back(r);
+        s->incoming.clear();
+    }
+}
+
 // One admission pass over the queue, in admission order (loop thread).
 void admit(posit_server *s, std::vector<Req> &done, std::vector<Unit *> &units)
 {
@@ -690,6 +720,7 @@ void loop_main(posit_server *s)
             }
             s->pending.clear();
         } else {
+            gather_burst(s);
             admit(s, done, units);
         }
         lk.lock();
