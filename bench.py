@@ -236,6 +236,44 @@ def whole_job_rate(world, work_per_step, steps, ms_max):
 # ---------------------------------------------------------------------------
 # our arm
 # ---------------------------------------------------------------------------
+# by posit_rgemm_route
+GEMM_KERNELS = ("gemm_main_kernel<0>", "gemm_fused_kernel<0, 4, 2>", "gemm_fused_kernel<0, 2, 2>")
+
+
+def gemm_roofline(route, m, n, k, kernel_s, sm_mhz, trailing=0):
+    """Roofline of the timed GEMM kernel: instruction issue (FP64 pipe the busiest pipe).  The
+    instruction and traffic figures are the staged route's main kernel's: a product on another
+    route (posit_rgemm_route) has its kernel's name and time here and no figure from those."""
+    from posit_gpu_b200 import perf
+    mads = float(m) * n * k
+    staged = route == 0
+    peak = perf.issue_peak_warp_inst_per_s(sm_mhz)
+    achieved = fp64_frac = None
+    current = perf.inst_count_current()
+    if staged and perf.WARP_INST_PER_MAD and kernel_s > 0 and current:
+        achieved = perf.WARP_INST_PER_MAD * mads / kernel_s
+        fp64_frac = perf.FP64_WARP_INST_PER_MAD * mads / kernel_s / perf.fp64_pipe_peak_warp_inst_per_s(sm_mhz)
+    roofline = {"bound": "issue", "achieved": achieved and round(achieved / 1e12, 4),
+                "peak": round(peak / 1e12, 4), "unit": "T warp-inst/s",
+                "frac": achieved and round(achieved / peak, 4),
+                "traffic": (perf.MAIN_KERNEL_DRAM_BYTES_PER_MAD * mads
+                            if staged and perf.MAIN_KERNEL_DRAM_BYTES_PER_MAD and not trailing else None),
+                "kernel": GEMM_KERNELS[route],
+                "main_kernel_ms": round(kernel_s * 1e3, 3),
+                "posit_gop_s_main_kernel": round(2 * mads / kernel_s / 1e9, 2) if kernel_s > 0 else None,
+                "warp_inst_per_mad": perf.WARP_INST_PER_MAD if staged else None,
+                "fp64_pipe_frac": fp64_frac and round(fp64_frac, 4),
+                "peak_basis": f"148 SMs x 4 SMSP x 1 warp-inst/clk at {sm_mhz:.0f} MHz (sampled median); "
+                              "MEASURED_PEAKS.json has no issue or FP64 figure",
+                "inst_source": perf.INST_SOURCE if staged else None,
+                "inst_source_stale": not current,
+                "kernel_source_sha256": perf.kernel_source_digest()}
+    if trailing:  # measured per shape, never scaled from the cube
+        roofline["traffic"] = perf.trailing_traffic(k) if staged else None
+        roofline["traffic_source"] = perf.TRAILING_TRAFFIC_SOURCE if roofline["traffic"] else "not measured"
+    return roofline
+
+
 def ours(args):
     import numpy as np
     import torch
@@ -300,37 +338,9 @@ def ours(args):
     ops_per_step = 2.0 * m * n * k
     value = whole_job_rate(world, ops_per_step, args.steps, ms_max) / 1e9
 
-    # roofline of the main kernel: instruction issue (FP64 pipe the busiest pipe)
-    mads = float(m) * n * k
-    main_avg_s = main_ms / 1e3 / max(main_launches, 1) if main_launches else 0.0
     sm_mhz = clocks.get("sm_mhz") or perf.SM_MAX_MHZ
-    peak = perf.issue_peak_warp_inst_per_s(sm_mhz)
-    achieved = None
-    current = perf.inst_count_current()
-    if perf.WARP_INST_PER_MAD and main_avg_s > 0 and current:
-        achieved = perf.WARP_INST_PER_MAD * mads / main_avg_s
-    fp64_frac = (perf.FP64_WARP_INST_PER_MAD * mads / main_avg_s / perf.fp64_pipe_peak_warp_inst_per_s(sm_mhz)
-                 if main_avg_s > 0 else None)
-    roofline = {"bound": "issue", "achieved": achieved and round(achieved / 1e12, 4),
-                "peak": round(peak / 1e12, 4), "unit": "T warp-inst/s",
-                "frac": achieved and round(achieved / peak, 4),
-                "traffic": (perf.MAIN_KERNEL_DRAM_BYTES_PER_MAD * mads
-                            if perf.MAIN_KERNEL_DRAM_BYTES_PER_MAD and not args.trailing else None),
-                "kernel": "gemm_main_kernel<0>",
-                "main_kernel_ms": round(main_avg_s * 1e3, 3),
-                "posit_gop_s_main_kernel": round(2 * mads / main_avg_s / 1e9, 2) if main_avg_s > 0 else None,
-                "warp_inst_per_mad": perf.WARP_INST_PER_MAD,
-                "fp64_pipe_frac": fp64_frac and round(fp64_frac, 4),
-                "peak_basis": f"148 SMs x 4 SMSP x 1 warp-inst/clk at {sm_mhz:.0f} MHz (sampled median); "
-                              "MEASURED_PEAKS.json has no issue or FP64 figure",
-                "inst_source": perf.INST_SOURCE,
-                "inst_source_stale": not current,
-                "kernel_source_sha256": perf.kernel_source_digest()}
-    if not current:
-        roofline["fp64_pipe_frac"] = None
-    if args.trailing:  # measured per shape, never scaled from the cube
-        roofline["traffic"] = perf.trailing_traffic(k)
-        roofline["traffic_source"] = perf.TRAILING_TRAFFIC_SOURCE if roofline["traffic"] else "not measured"
+    roofline = gemm_roofline(pg._lib.posit_rgemm_route(m, n, k), m, n, k,
+                             main_ms / 1e3 / max(main_launches, 1) if main_launches else 0.0, sm_mhz, args.trailing)
 
     if args.trailing:
         # short k: HBM reported beside the issue roofline (algorithmic bytes 4*(mk + kn + 2mn))

@@ -273,10 +273,11 @@ int posit_to_double_dev(const uint32_t *x, double *out, size_t n, void *stream);
 /* Reads (and with clear != 0 resets) the device-side error flags raised by kernels. */
 int posit_device_error(int clear);
 
-/* Instrumentation (no reference counterpart).  When enabled, CUDA events are recorded
- * around every GEMM main-kernel launch on its own stream; posit_profile_read waits for
- * them and returns the summed main-kernel time, the number of main-kernel launches and
- * the number of all kernels this library launched since the last reset. */
+/* Instrumentation (no reference counterpart).  When enabled, CUDA events are recorded on its
+ * own stream around the kernel that multiplies of every GEMM launch -- the main kernel behind the
+ * staged route's conversion, or the fused one (posit_rgemm_route); posit_profile_read waits for
+ * them and returns their summed time, their number and the number of all GEMM, scaling and
+ * conversion kernels launched since the last reset. */
 void posit_profile_enable(int on);
 int posit_profile_read(double *main_kernel_ms, long long *main_launches, long long *all_launches, int reset);
 

@@ -67,7 +67,7 @@ int read_device_error(bool clear);
 // Device address of the kernels' error flag (for stream-ordered copies of it).
 cudaError_t device_error_address(int **p);
 
-// Optional instrumentation: CUDA events around each main-kernel launch, recorded on
+// Optional instrumentation: CUDA events around each multiplying kernel (main or fused), recorded on
 // the launch stream, plus a count of this library's kernel launches.
 void profile_enable(bool on);
 int profile_read(double *main_ms, long long *main_launches, long long *all_launches, bool reset);
