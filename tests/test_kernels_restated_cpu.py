@@ -85,6 +85,29 @@ def test_quotient_on_ties_and_near_ties(hk):
         _div(hk, _neighbours(t, by), ua)
 
 
+def test_quotient_next_to_half_way(hk):
+    """Quotients 2^-51 to 2^-56 of their size away from half way between two posits: the FP64 value
+    of most is half way itself, and only the integer quotient knows the side.  t = (a h -+ 1) / 2^28 with the 29-bit odd
+    h half way and a its inverse modulo 2^28 (or less that)."""
+    rng = np.random.default_rng(6)
+    h = (rng.integers(2**27, 2**28, 40_000, dtype=np.uint64) * np.uint64(2) + np.uint64(1))
+    inv = h.copy()  # 3 bits right; doubled by each step
+    for _ in range(5):
+        inv = inv * (np.uint64(2) - h * inv)
+    m = np.uint64(2**28)
+    total = 0
+    for a, r in ((inv % m, 1), ((m - inv % m) % m, -1)):
+        ok = (a < 2**27) & (a > 2**23)  # t of at most 28 bits; 1 / (a h) below 2^-50
+        A, H = a[ok], h[ok]
+        t = (A.astype(object) * H.astype(object) - r)
+        assert all(v % 2**28 == 0 for v in t)
+        t = np.array([v >> 28 for v in t], np.float64)
+        ut, ua = (oracle.from_double(x / 2.0 ** np.floor(np.log2(x))) for x in (t, A.astype(np.float64)))
+        assert _div(hk, ut, ua) == ut.size
+        total += ut.size
+    assert total > 20_000
+
+
 def test_quotient_everywhere_else(hk):
     rng = np.random.default_rng(2)
     n = 500_000
@@ -123,9 +146,23 @@ def test_root(hk):
     tie = oracle.from_double((z + np.ldexp(1.0, e - fb - 1)) ** 2)
     for by in (-1, 0, 1):
         check(_neighbours(tie, by))
-    # exact roots
-    near = check(oracle.from_double(z * z))
-    assert near >= 0
+    check(oracle.from_double(z * z))  # exact ones
+    # as for the quotient: a = (h^2 - c) / 2^s with a small c, h odd and half way; square roots of c
+    # modulo 2^s lifted from the four modulo 8
+    total = 0
+    for s in (29, 30):
+        for c in range(-31, 33, 8):
+            roots = [1, 3, 5, 7]
+            for bit in range(3, s):
+                roots = [x for r in roots for x in (r, r + 2**bit) if (x * x - c) % 2 ** (bit + 1) == 0]
+            a = [(r * r - c) >> s for r in roots if 2**28 < r < 2**29]
+            a = sorted({v for v in a if 0 < v < 2**28})
+            if a:
+                x = np.array(a, np.float64)
+                # an even power of two away from the root's own scale
+                check(oracle.from_double(x * 2.0 ** (-28 if s == 30 else -27)))
+                total += check(oracle.from_double(x * 2.0 ** (-28 + s % 2)))
+    assert total >= 16, total
     check(np.array([1, 2, 3, 0x7FFFFFFF, 0x7FFFFFFE, 0x40000000, 0x40000001, 0x3FFFFFFF], np.uint32))
 
 
