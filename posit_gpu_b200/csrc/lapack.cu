@@ -271,8 +271,8 @@ __device__ __forceinline__ int cand_best_lane(const PivotCand &c)
     return __ffs(__ballot_sync(FULL, c.hi == hi && c.lo == lo && c.row == row)) - 1;
 }
 
-// rw[c*T] += -u[c] * l for the columns [c0, jb) of one row, PANEL_U at a time; up to
-// PANEL_U - 1 columns past jb are read and written too (u is zero there).
+// The columns of a row are updated PANEL_U at a time; up to PANEL_U - 1 columns past jb are read
+// and written too (u is zero there).
 constexpr int PANEL_U = 8;
 __host__ __device__ constexpr int panel_cols(int jb) { return jb + PANEL_U - 1; } // columns a row takes in shared memory
 inline size_t lu_panel_smem(int R, int T, int jb, int ncta)
@@ -280,7 +280,7 @@ inline size_t lu_panel_smem(int R, int T, int jb, int ncta)
     return STEP_TAB_BYTES + ((size_t)R * T + 3 * (size_t)ncta) * panel_cols(jb) * sizeof(double);
 }
 
-// The update of one row's columns [c0, jb).
+// rw[c*T] += -u[c] * l for the columns [c0, jb) of one row.
 __device__ __forceinline__ void panel_row_update(double *rw, int T, const double *u, double l, int c0, int jb,
                                                  const unsigned char *tab)
 {
@@ -307,9 +307,6 @@ __device__ __forceinline__ void panel_row_update(double *rw, int T, const double
     }
 }
 
-// MAXT: the most threads a CTA of this instance has, MAXR: the most slots of a thread.  One CTA per SM is said to the compiler
-// so that it spends registers on overlapping a row's columns (62 instead of 40: 355 cycles for
-// 8 columns of a warp instead of 511).
 // One row of jb columns from the matrix into shared memory, zeros behind it; eight loads in
 // flight.
 __device__ __forceinline__ void panel_load_row(double *rw, int T, const uint32_t *p, size_t lda, int jb)
@@ -328,6 +325,9 @@ __device__ __forceinline__ void panel_load_row(double *rw, int T, const uint32_t
     }
 }
 
+// MAXT: the most threads a CTA of this instance has, MAXR: the most slots of a thread.  One CTA
+// per SM is said to the compiler so that it spends registers on overlapping a row's columns (62
+// instead of 40: 355 cycles for 8 columns of a warp instead of 511).
 template <int MAXT, int MAXR>
 __global__ void __launch_bounds__(MAXT, 1) lu_panel_cluster_kernel(uint32_t *__restrict__ P, size_t lda, int M, int jb,
                                                                    int R, int row0, int *__restrict__ ipiv,
@@ -1269,15 +1269,18 @@ size_t rgetrf_workspace_bytes(int m, int n, int nb)
 // The LU panel's form: the cluster panel held in shared memory when its rows fit (ncta CTAs,
 // one per PANEL1_ROWS_PER_CTA rows up to 8, T threads each -- the CTA's rows rounded up to
 // whole warps, at most 1024 -- R slots per thread), else the two-launch form (ncta = 0).
+// The tables, the padding columns and the pushed rows leave room for 8192 rows of 16 columns, 6144 of 24,
+// 4864 of 32, 2560 of 64, 1280 of 128, fewer than the cluster panel without them took (8192 of 24, 6144
+// of 32).  The rows in between lost nothing by it: 6144 x 32 takes 0.47 ms in two launches a column
+// and took 0.83 in that cluster, LU n = 6000 86 ms and 153.
 struct PanelForm {
     int ncta, R, T; // CTAs (0: the panel does not fit), slots per thread, threads per CTA
 };
-static PanelForm panel_form(int M, int jb, int max_ctas)
+static PanelForm panel_form(int M, int jb)
 {
     if (jb > PANEL1_MAX_JB)
         return {0, 0, 0};
-    const int cap = max_ctas > 0 ? std::min(max_ctas, PANEL1_MAX_CTAS) : PANEL1_MAX_CTAS;
-    const int ncta = std::max(1, std::min(cap, (M + PANEL1_ROWS_PER_CTA - 1) / PANEL1_ROWS_PER_CTA));
+    const int ncta = std::max(1, std::min(PANEL1_MAX_CTAS, (M + PANEL1_ROWS_PER_CTA - 1) / PANEL1_ROWS_PER_CTA));
     const int rpc = (M + ncta - 1) / ncta; // rows per CTA
     const int T = std::min(PANEL1_THREADS, (rpc + 31) / 32 * 32), R = (rpc + T - 1) / T;
     if (lu_panel_smem(R, T, jb, ncta) > PANEL1_SMEM || R > PANEL1_MAX_R)
@@ -1316,7 +1319,7 @@ static dim3 panel_grid(int M, int jb, int k)
 // Rgetrf.cpp:95-132 with the device kernels above.  `ws` holds the pivot record, the
 // scratch column and the trailing GEMM's workspace.
 cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb, int *info, void *ws,
-                          cudaStream_t st, int max_ctas)
+                          cudaStream_t st)
 {
     const int mn = imin(m, n);
     if (nb < 1)
@@ -1330,7 +1333,7 @@ cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb,
         const int M = m - j;
         uint32_t *P = A + j + (size_t)j * L;
         uint32_t *lc = lcol + j; // indexed by panel-local row
-        const PanelForm pf = panel_form(M, jb, max_ctas);
+        const PanelForm pf = panel_form(M, jb);
         if (pf.ncta > 0) {
             cudaError_t e = launch_panel_cluster(pf.R > 1      ? lu_panel_cluster_kernel<PANEL1_THREADS, PANEL1_MAX_R>
                                                  : pf.T <= 128 ? lu_panel_cluster_kernel<128, 1>

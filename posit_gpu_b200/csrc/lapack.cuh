@@ -13,11 +13,8 @@ size_t rpotrf_workspace_bytes(int n, int nb);
 
 // All pointers are device pointers; ipiv is 1-based as in the reference; *info must be
 // zero on entry (it receives the first zero pivot / the first non-positive diagonal).
-// max_ctas caps the thread-block cluster of an LU panel held in shared memory (0: up to 8); a
-// caller that runs many factorizations at once uses smaller clusters, which the GPU can
-// place beside other work.  The bits do not depend on it.
 cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb, int *info, void *ws,
-                          cudaStream_t st, int max_ctas = 0);
+                          cudaStream_t st);
 cudaError_t rpotrf_lower_launch(int n, uint32_t *A, int lda, int nb, int *info, void *ws, cudaStream_t st);
 // CTAs that solve one of nrhs right-hand sides of m rows together (axpy-form solves).
 int solve_cluster_ctas(int m, int nrhs);

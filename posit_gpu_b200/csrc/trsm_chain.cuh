@@ -7,14 +7,13 @@
 // chain of m(m-1)/2 dependent multiply-subtracts with two roundings each.  Three forms:
 //   * llt_chain: one thread runs a right-hand side's whole chain with the accumulator
 //     held in the decoded integer form (very long columns);
-//   * chain_add_run / chain_add_run_reg: one thread's chain of additions in FP64, the
-//     products computed elsewhere (chain_add_run is the sequence the tests hold the others
-//     to);
 //   * warp_chain (end of this file): a warp sums a row's additions with the running value
 //     biased onto its binade's grid, one FP64 addition per step, and where the value is calm
 //     as a parallel prefix of step maps (lapack.cu's transposed-solve kernel and the
-//     batched kernels).  The scan form it grew from, one map per addend, stays written out
-//     for the host.
+//     batched kernels);
+//   * the forms it grew from, for the host: chain_add_run and chain_add_run_reg (one thread's
+//     chain, its products computed elsewhere) and the scan with one map per addend (SegFn).
+//     No kernel runs them; the CPU tests do.
 //
 // For the one-thread chains latency is everything.  Only the addition depends on the previous step: loads,
 // decoding and the product of step k+1 can overlap the addition of step k, but not across
@@ -151,8 +150,8 @@ PG_HD double llt_term(uint32_t l, uint32_t bk, uint32_t *nar)
 }
 
 // t + q_0 + q_1 + ... + q_{count-1}, every addition rounded (p32_add), in that order; t
-// and the q are posit32 values in FP64.  (The kernels use the scan form and
-// chain_add_run_reg below; this plain form is the sequence the tests hold them to.)
+// and the q are posit32 values in FP64.  (The kernels use warp_chain below; this plain form is a
+// sequence the tests hold chains to.)
 // Blocks of CHAIN_BLOCK steps without a branch, the flags tested once per block, a
 // flagged block replayed exactly from its start.
 PG_HD double chain_add_run(double t, const double *q, int count)
@@ -343,16 +342,10 @@ PG_HD double f64_posit_add_split(double t, double q, double C, int32_t run, uint
 
 // t + q_0 + ... + q_{count-1} as chain_add_run, with the fixed-width step: blocks of
 // CHAIN_BLOCK steps without a branch, a flagged block redone step by step exactly.
-// Terms read from FP64 values or from posit32 patterns (converted on load).
 struct TermsF64 {
     const double *q;
     PG_HD_MEMBER double operator[](int i) const { return q[i]; }
     PG_HD_MEMBER TermsF64 operator+(int i) const { return TermsF64{q + i}; }
-};
-struct TermsP32 {
-    const uint32_t *q;
-    PG_HD_MEMBER double operator[](int i) const { return p32_to_double(q[i]); }
-    PG_HD_MEMBER TermsP32 operator+(int i) const { return TermsP32{q + i}; }
 };
 
 template <class Q>

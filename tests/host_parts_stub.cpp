@@ -144,7 +144,7 @@ size_t rpotrf_workspace_bytes(int, int) { return 256; }
 size_t rpotrf_upper_workspace_bytes(int, int) { return 256; }
 int tuned_panel_width(bool, int) { return 32; }
 int solve_cluster_ctas(int, int) { return 1; }
-cudaError_t rgetrf_launch(int, int, uint32_t *, int, int *, int, int *, void *, cudaStream_t, int) { return cudaSuccess; }
+cudaError_t rgetrf_launch(int, int, uint32_t *, int, int *, int, int *, void *, cudaStream_t) { return cudaSuccess; }
 cudaError_t rpotrf_lower_launch(int, uint32_t *, int, int, int *, void *, cudaStream_t) { return cudaSuccess; }
 cudaError_t rpotrf_upper_launch(int, uint32_t *, int, int, int *, void *, cudaStream_t) { return cudaSuccess; }
 cudaError_t rgetrs_launch(int, int, const uint32_t *, int, const int *, uint32_t *, int, cudaStream_t) { return cudaSuccess; }
