@@ -11,11 +11,12 @@
 // block size bit for bit (the zero-multiplier skips of Rtrsm/Rsyrk add zero and change
 // nothing unless a NaR is present), and the device code may block the work its own way:
 //
-//   panel (nb columns)   one launch: LU on a thread-block cluster holding the panel in shared
-//                        memory, Cholesky on independent CTAs; LU panels too tall or wide
-//                        for shared memory take two launches per column, ordered by the
-//                        kernel boundary alone (the pivot step of one CTA, then the scaling
-//                        and the rank-1 update over all rows in parallel);
+//   panel (nb columns)   one launch: LU on a thread-block cluster holding up to 32 columns in
+//                        shared memory (wider or taller blocks by inner panels), Cholesky
+//                        on independent CTAs; LU panels of more rows than fit take two
+//                        launches per column, ordered by the kernel boundary alone (the
+//                        pivot step of one CTA, then the scaling and the rank-1 update over
+//                        all rows in parallel);
 //   U block row          Rtrsm("L","L","N","U"), a warp or a CTA per column;
 //   row interchanges     Rlaswp on the columns outside the panel;
 //   trailing update      the posit32 GEMM of gemm.cu (NN for LU; NT restricted to the
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(PANEL_ROWS) lu_update_kernel(uint32_t *__restr
 // LU n = 1024: 5.3 -> 3.4 ms, 4096: 51.6 -> 32.7.
 // ---------------------------------------------------------------------------
 constexpr int PANEL1_THREADS = 1024; // most threads per CTA
-constexpr int PANEL1_MAX_JB = 512;
+constexpr int PANEL1_MAX_JB = 32;        // wider blocks go by inner panels (panel_width)
 constexpr int PANEL1_MAX_CTAS = 8;
 constexpr int PANEL1_MAX_R = 4;          // slots per thread (the LU panel keeps their row numbers in registers)
 constexpr int PANEL1_ROWS_PER_CTA = 128; // the rows one CTA takes before another joins
@@ -494,11 +495,14 @@ __global__ void __launch_bounds__(MAXT, 1) lu_panel_cluster_kernel(uint32_t *__r
 // column, lane i holding row j+i and (for an interchange with a row below the block) that
 // row's value, loaded together; the interchanges run in order as exchanges between lanes,
 // the solve as jb steps of one multiply-add per lane with the step's b_k from its lane.
+// For an inner panel of a wider block (rgetrf_launch), A is the block's corner, at row and column
+// `off` of the matrix, n its width, and `skip` false: a panel's own updates skip no multiplier.
 constexpr int ROWS_JB_MAX = 32;
 constexpr int ROWS_THREADS = 256; // 8 columns per block
 
 __global__ void __launch_bounds__(ROWS_THREADS) lu_rows_kernel(uint32_t *__restrict__ A, size_t lda, int n, int j,
-                                                               int jb, const int *__restrict__ ipiv)
+                                                               int jb, const int *__restrict__ ipiv, int off,
+                                                               bool skip)
 {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     __shared__ double s_L[ROWS_JB_MAX * ROWS_JB_MAX]; // l_ik at [i * ROWS_JB_MAX + k], FP64
@@ -510,7 +514,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) lu_rows_kernel(uint32_t *__restr
         s_L[i * ROWS_JB_MAX + k] = p32_to_double(A[(j + i) + (size_t)(j + k) * lda]);
     }
     for (int i = tid; i < jb; i += ROWS_THREADS)
-        s_t[i] = ipiv[j + i] - 1;
+        s_t[i] = ipiv[j + i] - 1 - off;
     __syncthreads();
     for (int i = tid; i < jb; i += ROWS_THREADS) {
         int a = -1;
@@ -557,7 +561,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) lu_rows_kernel(uint32_t *__restr
         double x = row ? p32_to_double(v) : 0.0;
         for (int k = 0; k < jb; ++k) {
             const double bk = __shfl_sync(FULL, x, k);
-            if (bk != 0.0 && lane > k && row)
+            if ((bk != 0.0 || !skip) && lane > k && row)
                 x = f64_posit_mac_checked(x, -bk, s_L[lane * ROWS_JB_MAX + k]);
         }
         v = p32_from_double(x);
@@ -1256,23 +1260,9 @@ int tuned_panel_width(bool lu, int n)
     return nb;
 }
 
-size_t rgetrf_workspace_bytes(int m, int n, int nb)
-{
-    int mn = imin(m, n);
-    if (nb < 1)
-        nb = 1;
-    int jb = imin(nb, mn);
-    size_t g = mn > jb ? gemm_workspace_bytes(m - jb > 0 ? m - jb : 1, n - jb > 0 ? n - jb : 1, jb) : 0;
-    return panel_ws_bytes(m) + g;
-}
-
 // The LU panel's form: the cluster panel held in shared memory when its rows fit (ncta CTAs,
 // one per PANEL1_ROWS_PER_CTA rows up to 8, T threads each -- the CTA's rows rounded up to
 // whole warps, at most 1024 -- R slots per thread), else the two-launch form (ncta = 0).
-// The tables, the padding columns and the pushed rows leave room for 8192 rows of 16 columns, 6144 of 24,
-// 4864 of 32, 2560 of 64, 1280 of 128, fewer than the cluster panel without them took (8192 of 24, 6144
-// of 32).  The rows in between lost nothing by it: 6144 x 32 takes 0.47 ms in two launches a column
-// and took 0.83 in that cluster, LU n = 6000 86 ms and 153.
 struct PanelForm {
     int ncta, R, T; // CTAs (0: the panel does not fit), slots per thread, threads per CTA
 };
@@ -1286,6 +1276,37 @@ static PanelForm panel_form(int M, int jb)
     if (lu_panel_smem(R, T, jb, ncta) > PANEL1_SMEM || R > PANEL1_MAX_R)
         return {0, 0, 0};
     return {ncta, R, T};
+}
+
+// The columns of a block of jb that one panel launch takes: all, if they are at most 32 and fit in a
+// cluster (tables, padding columns and pushed rows beside them leave room for 4864 rows of 32
+// columns, 6144 of 24, 8192 of 16, 13,300 of 8); else inner panels of 32, 24 or 16, the widest that fits, the
+// block's columns updated between them; else all, in two launches per column.  A block's update of
+// the rest of the matrix stays one of jb columns.
+// Two launches per column cost 14 us a column, and one launch for all columns of a wide block gains
+// less with each: 6144 x 32 0.47 ms in two launches a column (0.83 in the cluster of all 32 that fitted
+// without the padding) and 0.15 by inner panels, 3072 x 64 0.82 (0.71) and 0.20, 1536 x 128 1.58 (1.46)
+// and 0.39; LU n = 8192 197 -> 161 ms, n = 1024 with the caller's nb = 256 14.1 -> 4.5, with nb = 128 (one
+// launch a panel) 5.5 -> 4.6.
+static int panel_width(int M, int jb)
+{
+    if (panel_form(M, jb).ncta == 0)
+        for (int w : {32, 24, 16})
+            if (w < jb && panel_form(M, w).ncta > 0)
+                return w;
+    return jb;
+}
+
+size_t rgetrf_workspace_bytes(int m, int n, int nb)
+{
+    int mn = imin(m, n);
+    if (nb < 1)
+        nb = 1;
+    int jb = imin(nb, mn);
+    size_t g = mn > jb ? gemm_workspace_bytes(m - jb > 0 ? m - jb : 1, n - jb > 0 ? n - jb : 1, jb) : 0;
+    if (jb > 16) // inner panels
+        g = std::max(g, gemm_workspace_bytes(m, jb, PANEL1_MAX_JB));
+    return panel_ws_bytes(m) + g;
 }
 
 template <class... Args>
@@ -1333,27 +1354,42 @@ cudaError_t rgetrf_launch(int m, int n, uint32_t *A, int lda, int *ipiv, int nb,
         const int M = m - j;
         uint32_t *P = A + j + (size_t)j * L;
         uint32_t *lc = lcol + j; // indexed by panel-local row
-        const PanelForm pf = panel_form(M, jb);
-        if (pf.ncta > 0) {
-            cudaError_t e = launch_panel_cluster(pf.R > 1      ? lu_panel_cluster_kernel<PANEL1_THREADS, PANEL1_MAX_R>
-                                                 : pf.T <= 128 ? lu_panel_cluster_kernel<128, 1>
-                                                 : pf.T <= 512 ? lu_panel_cluster_kernel<512, 1>
-                                                               : lu_panel_cluster_kernel<PANEL1_THREADS, 1>,
-                                                 pf, lu_panel_smem(pf.R, pf.T, jb, pf.ncta),
-                                                 st, P, L, M, jb, pf.R, j, ipiv, info);
-            if (e != cudaSuccess)
-                return e;
-        } else {
-            lu_pivot_kernel<<<1, 1024, 0, st>>>(P, L, M, jb, 0, j, ipiv, info, pinfo, lc, -1);
-            for (int k = 0; k < jb; ++k) {
-                lu_update_kernel<<<panel_grid(M, jb, k), PANEL_ROWS, 0, st>>>(P, L, M, jb, k, info, pinfo, lc);
-                lu_pivot_kernel<<<1, 1024, 0, st>>>(P, L, M, jb, k + 1, j, ipiv, info, pinfo, lc, k);
+        const int w = panel_width(M, jb);
+        for (int q = 0; q < jb; q += w) { // the block's inner panels (one, where w == jb)
+            const int wj = imin(w, jb - q), rest = jb - q - wj;
+            uint32_t *Pq = P + q + (size_t)q * L;
+            const PanelForm pf = panel_form(M - q, wj);
+            if (pf.ncta > 0) {
+                cudaError_t e = launch_panel_cluster(pf.R > 1      ? lu_panel_cluster_kernel<PANEL1_THREADS, PANEL1_MAX_R>
+                                                     : pf.T <= 128 ? lu_panel_cluster_kernel<128, 1>
+                                                     : pf.T <= 512 ? lu_panel_cluster_kernel<512, 1>
+                                                                   : lu_panel_cluster_kernel<PANEL1_THREADS, 1>,
+                                                     pf, lu_panel_smem(pf.R, pf.T, wj, pf.ncta), st, Pq, L, M - q, wj,
+                                                     pf.R, j + q, ipiv, info);
+                if (e != cudaSuccess)
+                    return e;
+            } else { // (never an inner panel)
+                lu_pivot_kernel<<<1, 1024, 0, st>>>(P, L, M, jb, 0, j, ipiv, info, pinfo, lc, -1);
+                for (int k = 0; k < jb; ++k) {
+                    lu_update_kernel<<<panel_grid(M, jb, k), PANEL_ROWS, 0, st>>>(P, L, M, jb, k, info, pinfo, lc);
+                    lu_pivot_kernel<<<1, 1024, 0, st>>>(P, L, M, jb, k + 1, j, ipiv, info, pinfo, lc, k);
+                }
+            }
+            if (wj == jb)
+                break;
+            lu_rows_kernel<<<(jb - wj + ROWS_THREADS / 32 - 1) / (ROWS_THREADS / 32), ROWS_THREADS, 0, st>>>(
+                P, L, jb, q, wj, ipiv + j, j, false);
+            if (rest > 0 && M - q > wj) {
+                cudaError_t e = gemm_launch(true, true, M - q - wj, rest, wj, 0xC0000000u /* -1 */, Pq + wj, lda,
+                                            Pq + (size_t)wj * L, lda, P32_ONE, Pq + wj + (size_t)wj * L, lda, gws, st, true);
+                if (e != cudaSuccess)
+                    return e;
             }
         }
         if (jb <= ROWS_JB_MAX) {
             if (n > jb)
                 lu_rows_kernel<<<(n - jb + ROWS_THREADS / 32 - 1) / (ROWS_THREADS / 32), ROWS_THREADS, 0, st>>>(
-                    A, L, n, j, jb, ipiv);
+                    A, L, n, j, jb, ipiv, 0, true);
         } else {
             if (j > 0)
                 laswp_kernel<<<(j + 127) / 128, 128, 0, st>>>(A, L, j, j + 1, j + jb, ipiv, 1, info);
