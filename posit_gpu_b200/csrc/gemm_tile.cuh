@@ -19,8 +19,8 @@
 //     sum's 4-byte ones (half the bank cycles, one move for the zero low word): 3950 against
 //     3700 (both 8-byte: shared-memory bandwidth) and 3850 Gop/s (both 4-byte);
 //   * 4x4 outputs per thread and an unrolled k loop (4x2: 3800).
-// ncu on the main kernel (4096 x 4096 x 1024 NN): 13.75 instructions per multiply-add (before:
-// 22.4), 6.03 of them FP64, issue 71 % and the second FP64 slots 31 %: full.  8192^3 NN,
+// ncu on the main kernel (4096^3 NN): 14.02 instructions per multiply-add (before: 22.4), 6.03 of
+// them FP64, issue 71.7 % and the second FP64 slots 31 %: full.  8192^3 NN,
 // the whole call: 470 -> 289 ms.  Wide-range data (10^U(-20,20), 2048^3, nearly every sum
 // outside the fast window): 206 -> 20 ms, with g_outside_table (61 ms with the integer
 // rounding on every such step).

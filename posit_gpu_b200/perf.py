@@ -48,7 +48,7 @@ def fp64_pipe_peak_warp_inst_per_s(sm_mhz):
 # the benchmark recomputes the digest and, when it differs, marks the count stale and
 # reports no roofline fraction from it.
 KERNEL_SOURCES = ["csrc/gemm.cu", "csrc/gemm.cuh", "csrc/gemm_tile.cuh", "csrc/posit32.cuh"]
-INST_SOURCE_DIGEST = "de3959670852b80076b1e212b2ff722ec4b29b16213019e852689cfc91f31402"
+INST_SOURCE_DIGEST = "54aed4f387b4609bc67e2a97ff14d8745f33f5a74caa3839ff5ec8225e792bcf"
 
 
 def kernel_source_digest():
