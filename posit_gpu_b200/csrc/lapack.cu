@@ -1280,7 +1280,7 @@ static PanelForm panel_form(int M, int jb)
 
 // The columns of a block of jb that one panel launch takes: all, if they are at most 32 and fit in a
 // cluster (tables, padding columns and pushed rows beside them leave room for 4864 rows of 32
-// columns, 6144 of 24, 8192 of 16, 13,300 of 8); else inner panels of 32, 24 or 16, the widest that fits, the
+// columns, 6144 of 24, 8192 of 16); else inner panels of 32, 24 or 16, the widest that fits, the
 // block's columns updated between them; else all, in two launches per column.  A block's update of
 // the rest of the matrix stays one of jb columns.
 // Two launches per column cost 14 us a column, and one launch for all columns of a wide block gains
