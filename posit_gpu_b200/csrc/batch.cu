@@ -18,6 +18,7 @@
 #include "posit32.cuh"
 #include "trsm_chain.cuh"
 
+#include <algorithm>
 #include <limits.h>
 
 namespace pg {
@@ -679,8 +680,8 @@ __device__ __forceinline__ bool llt_by_thread(int n, int nrhs, int threads, int 
     return by_thread < other;
 }
 
-// The right-hand sides: Rgetrs('N') or Rpotrs('L').  MANY: any number of them, else a few
-// (batch_many_rhs).
+// The right-hand sides: Rgetrs('N') or Rpotrs('L').  MANY: many of them, spread over the
+// threads (batch_spread_pays).
 template <class C, bool LU, bool MANY>
 __device__ __forceinline__ void solve_one(const BatchProblem &pr, unsigned char *smem, BatchShared &s)
 {
@@ -1017,15 +1018,40 @@ static cudaError_t launch_cfg(const BatchProblem *probs, int first, int last, co
     return cudaGetLastError();
 }
 
-cudaError_t batch_factor_launch(bool large, bool many, const BatchProblem *probs, int first, int last, const int *order,
+// The kernels without the code that spreads right-hand sides solve any number of them too, a thread
+// per row (a warp's one by one), and factor faster: with that code in, the compiler spills more, and an
+// LU of n = 512 takes 9.1 ms instead of 8.2 (two CTAs an SM: n = 200 1.75 instead of 1.70). So it is
+// a matter of the launch's longest problem, or of all of them over its CTAs.  Times in us, fitted to
+// problems of 33 to 512 rows and 1 to 300 right-hand sides.
+bool batch_spread_pays(bool large, const BatchProblem *probs, int first, int last, const int *order, int sms)
+{
+    double longest[2] = {0.0, 0.0}, sum[2] = {0.0, 0.0};
+    bool many = false;
+    for (int i = first; i < last; ++i) {
+        const BatchProblem &q = probs[order ? order[i] : i];
+        const double n = q.n, rhs = q.nrhs, f = (q.kind & BATCH_SOLVE_ONLY) ? 0.0 : (large ? 0.030 : 0.039) * n * n;
+        const bool spread = q.nrhs > (q.n > BATCH_WARP_N ? AXPY_FEW : 2);
+        many |= spread;
+        const double each = q.n <= BATCH_WARP_N && (q.kind & 1) == BATCH_CHOL ? 1.5 : 0.41; // a right-hand side, us a row
+        const double t[2] = {f + each * n * rhs, f * (large ? 1.10 : 1.03) + (spread ? 0.12 : each) * n * rhs};
+        for (int w = 0; w < 2; ++w) {
+            longest[w] = std::max(longest[w], t[w]);
+            sum[w] += t[w];
+        }
+    }
+    const double ctas = large ? sms : 2.0 * sms;
+    return many && std::max(longest[1], sum[1] / ctas) < std::max(longest[0], sum[0] / ctas);
+}
+
+cudaError_t batch_factor_launch(bool large, bool spread, const BatchProblem *probs, int first, int last, const int *order,
                                 int warp_from, int *next, int sms, cudaStream_t st)
 {
     if (last <= first)
         return cudaSuccess;
     if (large)
-        return many ? launch_cfg<LargeCfg, true>(probs, first, last, order, warp_from, next, sms, st)
+        return spread ? launch_cfg<LargeCfg, true>(probs, first, last, order, warp_from, next, sms, st)
                     : launch_cfg<LargeCfg, false>(probs, first, last, order, warp_from, next, sms, st);
-    return many ? launch_cfg<SmallCfg, true>(probs, first, last, order, warp_from, next, 2 * sms, st)
+    return spread ? launch_cfg<SmallCfg, true>(probs, first, last, order, warp_from, next, 2 * sms, st)
                 : launch_cfg<SmallCfg, false>(probs, first, last, order, warp_from, next, 2 * sms, st);
 }
 

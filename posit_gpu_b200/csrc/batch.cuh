@@ -15,12 +15,6 @@ constexpr int BATCH_WARP_N = 32;    // a problem of up to this many rows may be 
 // sides: 1520 us by a warp, 462 by a CTA; 2000 of them: 2571 us by warps, about 3400 by CTAs.
 constexpr int BATCH_WARP_RHS = 16;
 constexpr int BATCH_CTA_TURNS = 3;
-// Whether a problem needs the kernels that spread right-hand sides over the threads (up to 4 pay
-// a thread per row, up to 2 a warp's turns).  Launches without one take kernels without that
-// code: with it in, the compiler spills more in the factorization, and an LU of n = 512 takes
-// 9.1 ms instead of 8.2.
-inline bool batch_many_rhs(int n, int nrhs) { return nrhs > (n > BATCH_WARP_N ? 4 : 2); }
-
 // One problem: A (n x n, column-major, lda) is factored in place, B (n x nrhs, ldb)
 // overwritten with the solution; ipiv (LU) receives n 1-based pivots, info the
 // reference's info.  All pointers are device pointers.
@@ -38,9 +32,13 @@ struct BatchProblem {
 // Runs problems probs[order[i]] (order null: probs[i]), first <= i < last, on persistent CTAs;
 // `order` sorts by decreasing n.  `large`: one CTA per SM (problems of more than
 // BATCH_LARGE_N rows), else two smaller ones; those from warp_from on (of up to BATCH_WARP_N
-// rows) go to a warp each.  `many`: there is one of batch_many_rhs.  `next` is a device counter
-// the launch zeroes first.  A null order may be in any order, of any sizes, with warp_from = last.
-cudaError_t batch_factor_launch(bool large, bool many, const BatchProblem *probs, int first, int last, const int *order,
+// rows) go to a warp each.  `spread`: by the kernels that spread right-hand sides over the threads
+// (batch_spread_pays; the bits are the same).  `next` is a device counter the launch zeroes first.  A null order may be in any order, of any sizes, with warp_from = last.
+cudaError_t batch_factor_launch(bool large, bool spread, const BatchProblem *probs, int first, int last, const int *order,
                                 int warp_from, int *next, int sms, cudaStream_t st);
+
+// Whether such a launch of the host array's problems probs[order[i]] (order null: probs[i]), first <=
+// i < last, is shorter with the kernels that spread right-hand sides over the threads.
+bool batch_spread_pays(bool large, const BatchProblem *probs, int first, int last, const int *order, int sms);
 
 } // namespace pg

@@ -88,8 +88,9 @@ extern "C" int posit_batch_plan_create(const posit_batch_problem *probs, int npr
     std::vector<int> order(nprob);
     int nlarge = 0, warp_from = 0;
     batch_order(probs, nprob, sms, order, nlarge, warp_from);
-    const bool many = std::any_of(probs, probs + nprob,
-                                  [](const posit_batch_problem &q) { return pg::batch_many_rhs(q.n, q.nrhs); });
+    const auto *host = reinterpret_cast<const pg::BatchProblem *>(probs);
+    const bool spread_large = pg::batch_spread_pays(true, host, 0, nlarge, order.data(), sms),
+               spread = pg::batch_spread_pays(false, host, nlarge, nprob, order.data(), sms);
     cudaError_t e = cudaMalloc((void **)&p->d_probs, sizeof(pg::BatchProblem) * (nprob > 0 ? nprob : 1));
     if (e == cudaSuccess)
         e = cudaMalloc(&p->d_order, sizeof(int) * (nprob > 0 ? nprob : 1));
@@ -120,10 +121,10 @@ extern "C" int posit_batch_plan_create(const posit_batch_problem *probs, int npr
             if (le == cudaSuccess)
                 le = cudaStreamWaitEvent(side, fork, 0);
             if (le == cudaSuccess)
-                le = pg::batch_factor_launch(true, many, d, 0, nlarge, o, nlarge, p->d_next, p->ctas, cs);
+                le = pg::batch_factor_launch(true, spread_large, d, 0, nlarge, o, nlarge, p->d_next, p->ctas, cs);
             if (le == cudaSuccess)
-                le = pg::batch_factor_launch(false, many, d, nlarge, nprob, o, warp_from, p->d_next + 1, p->ctas,
-                                             side);
+                le = pg::batch_factor_launch(false, spread, d, nlarge, nprob, o, warp_from, p->d_next + 1,
+                                             p->ctas, side);
             if (le == cudaSuccess)
                 le = cudaEventRecord(join, side);
             if (le == cudaSuccess)

@@ -333,11 +333,9 @@ int launch_batched(posit_server *s, Unit *u)
     Lane &L = *u->lane;
     cudaStream_t st = L.st;
     const int np = (int)u->reqs.size();
-    bool many = false;
     for (int i = 0; i < np; ++i) {
         Request &r = *u->reqs[i];
         Factor *f = r.f;
-        many |= pg::batch_many_rhs(r.q.n, r.q.nrhs);
         if (!r.hit)
             SV_TRY(upload_matrix(s, f, r.q.A, st));
         SV_TRY(upload_rhs(s, r, st));
@@ -358,8 +356,8 @@ int launch_batched(posit_server *s, Unit *u)
     int *d_next = reinterpret_cast<int *>(static_cast<unsigned char *>(dd) + desc_bytes);
     cudaError_t e = cudaMemcpyAsync(dd, L.h_desc, sizeof(pg::BatchProblem) * np, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
-        e = pg::batch_factor_launch(false, many, static_cast<pg::BatchProblem *>(dd), 0, np, nullptr, np, d_next,
-                                    s->sms, st);
+        e = pg::batch_factor_launch(false, pg::batch_spread_pays(false, L.h_desc, 0, np, nullptr, s->sms),
+                                    static_cast<pg::BatchProblem *>(dd), 0, np, nullptr, np, d_next, s->sms, st);
     cudaFreeAsync(dd, st);
     if (e != cudaSuccess)
         return fail_code(e);

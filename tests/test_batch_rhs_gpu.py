@@ -109,3 +109,14 @@ def test_many_problems_with_many_right_hand_sides(cuda_ok, what):
     rng = np.random.default_rng(9)
     sizes = [(1, 20), (3, 16), (4, 31), (7, 33), (13, 90), (16, 16), (17, 40), (31, 36), (32, 33), (32, 16)]
     _run(pg, rng, [(q & 1, *sizes[q // 2 % len(sizes)]) for q in range(1000)], what)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["uniform", "special"])
+def test_few_many_right_hand_sides_beside_longer_problems(cuda_ok, what):
+    """Where a few problems with many right-hand sides do not bound the launch, it takes the kernels
+    with a thread per row; they solve any number all the same."""
+    import posit_gpu_b200 as pg
+    rng = np.random.default_rng(12)
+    _run(pg, rng, [(0, 620, 1), (0, 300, 8), (1, 240, 6), (0, 200, 1), (0, 40, 7), (1, 36, 9), (1, 12, 5), (0, 7, 9)],
+         what)
